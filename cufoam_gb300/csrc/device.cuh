@@ -746,33 +746,42 @@ __device__ __forceinline__ void sell_long_rows(int n, int s, const int32_t *__re
     }
 }
 
-// f(row, sum_t val[t] g(col[t])) for every row, one warp per slice; the
-// entries are taken B at a time (all B loads and gathers issued before the
+// sum_t val[t] g(col[t]) of this lane's row of slice s (sell_slice), and
+// f(row, sum) for every row, one warp per slice (sell_rows); the entries are taken B at a time (all B loads and gathers issued before the
 // first FMA), the row's last r < B entries as an exact batch: a guarded slot
 // of a full batch would still issue its FMA (measured: 9 DFMA per 7-entry
 // row).  The slice length is warp-uniform, so the branches never diverge.
 // Matrices with rows longer than kLongRow (has_long) sum those rows with
 // the whole warp (sell_long_rows), as the CSR passes do.  cs: the columns
 // (SellCols32 or SellCodes8).
+template <class V, int B, class C, class G>
+__device__ __forceinline__ V sell_slice(int n, int s, const int32_t *__restrict__ off, const C &cs,
+                                        const V *__restrict__ val, const int32_t *__restrict__ ro, bool has_long,
+                                        uint64_t pol, G g)
+{
+    const int lane = threadIdx.x & 31;
+    const int b = __ldg(off + s);
+    const int len = (__ldg(off + s + 1) - b) >> 5;
+    const int rb = sell_row_base(s * 32 + lane, n);
+    const V *vp = val + (int64_t)b + lane;
+    V acc = V(0);
+    int t0 = 0;
+    for (; t0 + B <= len; t0 += B) sell_batch<V, B>(cs, b, lane, len, t0, rb, vp + 32 * t0, pol, g, acc);
+    sell_tail<V, B>(len - t0, cs, b, lane, len, t0, rb, vp + 32 * t0, pol, g, acc);
+    if (has_long) sell_long_rows(n, s, ro, cs, b, len, val + b, g, acc);
+    return acc;
+}
+
 template <class V, int B, class C, class G, class F>
 __device__ __forceinline__ void sell_rows(int n, int n_slices, const int32_t *__restrict__ off, const C &cs,
                                           const V *__restrict__ val, const int32_t *__restrict__ ro,
                                           bool has_long, G g, F f)
 {
     const uint64_t pol = l2_evict_first_policy();
-    const int lane = threadIdx.x & 31;
     const int nw = gridDim.x * kWarps;
     for (int s = blockIdx.x * kWarps + (threadIdx.x >> 5); s < n_slices; s += nw) {
-        const int b = __ldg(off + s);
-        const int len = (__ldg(off + s + 1) - b) >> 5;
-        const int row = s * 32 + lane;
-        const int rb = sell_row_base(row, n);
-        const V *vp = val + (int64_t)b + lane;
-        V acc = V(0);
-        int t0 = 0;
-        for (; t0 + B <= len; t0 += B) sell_batch<V, B>(cs, b, lane, len, t0, rb, vp + 32 * t0, pol, g, acc);
-        sell_tail<V, B>(len - t0, cs, b, lane, len, t0, rb, vp + 32 * t0, pol, g, acc);
-        if (has_long) sell_long_rows(n, s, ro, cs, b, len, val + b, g, acc);
+        const V acc = sell_slice<V, B>(n, s, off, cs, val, ro, has_long, pol, g);
+        const int row = s * 32 + (threadIdx.x & 31);
         if (row < n) f(row, acc);
     }
 }

@@ -193,6 +193,8 @@ struct Context {
     // system, see GridCap); the reference order keeps the reference's grid
     int grid_cap = 0;
     int small_cg_ok = -1;      // 16-CTA clusters schedulable (-1: not asked yet)
+    int coop_ok = -1;          // cooperative launches supported (-1: not asked yet)
+    DeviceBuffer persist;      // grid-persistent solves: block partials, barrier counter
 
     // scratch of the matrix builds (grow-only: a conversion after the first
     // allocates nothing) and the matrix of one-shot ldu2csr conversions
@@ -321,6 +323,12 @@ SmallSolveResult solve_cg_single_cluster(Matrix *m, const cf_controls &c, const 
 SmallSolveResult solve_small_single_cluster(Matrix *m, int solver, const cf_controls &c, const double *b,
                                             double *x, double *r, double *d, double *y);
 bool small_cg_ok(Context *ctx);
+
+// a whole FP64 solve in the fast order as one cooperative launch (persist.cu)
+const void *persist_kernel_for(Context *ctx, int solver, int format);
+void launch_persist(Context *ctx, const void *kernel, int solver, const SolveArgs &A, const DevState &S, int l1,
+                    DevState *out);
+void persist_reset(Context *ctx);
 
 struct Batch;
 Batch *batch_create(Context *ctx, int n_systems, const cf_ldu_view *views);

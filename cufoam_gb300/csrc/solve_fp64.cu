@@ -750,7 +750,9 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     const int fmt = solve_format(A);
     const Kernels kk = ref ? body_kernels(solver, sell) : fast_body_kernels(solver, fmt);
     SolveArgs *d_args = ctx->args.as<SolveArgs>();
-    if (use_graph && !mixed) {
+    // the fast order over the SELL-32 copy: one cooperative launch
+    const void *persist = (use_graph && !ref && !mixed) ? persist_kernel_for(ctx, solver, fmt) : nullptr;
+    if (use_graph && !mixed && !persist) {
         try {
             ge = loop_graph(ctx, kk, solver, CF_PREC_FP64, cap, ref, d_args, fmt);
         } catch (const Error &) {
@@ -758,9 +760,19 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
             use_graph = false;
         }
     }
-    A.use_cond = (use_graph && !mixed) ? 1 : 0;
-    A.cond = (use_graph && !mixed) ? ge->cond : 0;
+    A.use_cond = ge ? 1 : 0;
+    A.cond = ge ? ge->cond : 0;
     *ctx->h_abort = 0;
+    const int l1 = (c.norm_type == CF_NORM_OPENFOAM_L1) ? 1 : 0;
+    const auto wall0 = std::chrono::steady_clock::now();
+    double kms[3] = {0.0, 0.0, 0.0};
+    int klaunch[3] = {0, 0, 0};
+    MixedResult mres;
+    if (persist) {
+        CF_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
+        launch_persist(ctx, persist, solver, A, S, l1, ctx->h_state);
+        CF_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
+    } else {
     CF_CUDA(cudaMemcpyAsync(d_args, &A, sizeof(SolveArgs), cudaMemcpyHostToDevice, ctx->stream));
     CF_CUDA(cudaMemcpyAsync(A.st, &S, sizeof(DevState), cudaMemcpyHostToDevice, ctx->stream));
 
@@ -770,8 +782,7 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     {
         launch(ctx, ctx->stream, (const void *)k_nf_sum,
                launch_cfg(ctx, (const void *)k_nf_sum, false, cap, ref), args1);
-        int l1 = (c.norm_type == CF_NORM_OPENFOAM_L1) ? 1 : 0;
-        void *a2[] = {&d_args, &l1};
+        void *a2[] = {&d_args, (void *)&l1};
         launch(ctx, ctx->stream, (const void *)k_nf_dist,
                launch_cfg(ctx, (const void *)k_nf_dist, !sell, cap, ref), a2);
     }
@@ -801,10 +812,6 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     }
     // ---- iterations: device-driven while loop, or host-driven chunks ----
     CF_CUDA(cudaEventRecord(ctx->ev_mid, ctx->stream));
-    auto wall0 = std::chrono::steady_clock::now();
-    double kms[3] = {0.0, 0.0, 0.0};
-    int klaunch[3] = {0, 0, 0};
-    MixedResult mres;
     if (mixed) {
         mres = run_mixed(ctx, m, solver, c, d_args, cap, use_graph);
     } else if (use_graph) {
@@ -878,6 +885,7 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     }
     CF_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
     CF_CUDA(cudaMemcpyAsync(ctx->h_state, A.st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
+    }
     if (c.time_limit_s > 0 && use_graph) {
         while (cudaEventQuery(ctx->ev_stop) == cudaErrorNotReady) {
             const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - wall0).count();
@@ -887,6 +895,7 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     }
     CF_CUDA(cudaStreamSynchronize(ctx->stream));
     const DevState R = *ctx->h_state;
+    if (persist && R.flags) persist_reset(ctx);
     if (c.memory == CF_MEM_HOST) {
         download(ctx, x_io, x, sizeof(double) * n, CF_MEM_HOST);
     }
