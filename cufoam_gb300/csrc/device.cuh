@@ -100,6 +100,211 @@ __device__ __forceinline__ void block_sum_fast(T (&v)[NV], T *sm)
     }
 }
 
+// ---------------------------------------------------------------------------
+// The bits of a sequential FP64 sum of up to 1,280 values, formed by a block
+// of 256 threads (the reference order sums the 1,216 block partials of a
+// reduction one after the other).
+//
+// While the running sum s stays inside one binade, it is a multiple of one
+// unit u, and s + v rounds to s + u RN(v / u) whatever s is, unless v / u
+// lies exactly between two integers: over such a stretch the sum is an
+// integer sum.  Where the binade changes is known beforehand, from the exact
+// prefix sums P (64-bit fixed point, 51 bits for the largest value): s
+// differs from P by less than kSeqBand units of it, the truncation of 1,280
+// values plus 1,280 roundings of the largest possible s.  So
+//   * a value whose prefixes before and after lie in the same binade, at
+//     least kSeqBand from its ends, and that is not a tie, contributes
+//     q = RN(v / u) (a value 0 contributes 0);
+//   * every other value is an event: s takes the integers since the last
+//     event -- an addition to its bits, the exponent does not change -- and
+//     then the value itself by an FP64 addition.
+// Sums of like terms have about 15 events, sums with cancellation 20 to 70.
+// More than kSeqEvents, or values that fixed point cannot hold (non-finite,
+// exponents near the ends), are added one by one.
+//
+// Why: a dependent FP64 addition takes 80 cycles on GB300 (its sub-partition
+// holds the FP64 unit for 64 whatever the active lanes): 1,216 of them in one
+// thread took 47 us; an event costs about as much as one addition.  Per step
+// at 113k / 893k / 2.1M rows: BiCG 169 / 252 / 378 -> 57 / 159 / 271 us, CG in
+// the reference order 116 / 168 / 233 -> 41 / 97 / 170 us.  (Working through
+// the values a binade at a time -- one warp, a round of integer prefix sums
+// per change of binade, about 1 us each -- was slower than the thread's
+// additions for BiCG's signed sums: 405 us per step at 2.1M rows.)
+// ---------------------------------------------------------------------------
+constexpr int kSeqPer = 5;                      // consecutive values per thread
+constexpr int kSeqMax = kSeqPer * kBlock;
+constexpr int kSeqEvents = 256;
+constexpr long long kSeqBand = 1ll << 20;
+
+struct SeqScratch {
+    uint32_t wmax[kWarps];
+    uint32_t wor[kWarps];
+    long long wsum[kWarps];
+    uint32_t wcnt[kWarps];
+    long long qtot;
+    int32_t events;        // -1: add one by one
+};
+
+// inclusive scan over the block of one 64-bit value per thread
+__device__ __forceinline__ long long seq_block_scan(long long v, long long *wsum)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long t = __shfl_up_sync(kFull, v, o);
+        if (lane >= o) v += t;
+    }
+    if (lane == 31) wsum[warp] = v;
+    __syncthreads();
+    long long off = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w)
+        if (w < warp) off += wsum[w];
+    return v + off;
+}
+
+// All 256 threads: the events of part[0 .. G) into rec (value j at rec[j],
+// the integers before it at rec[kSeqEvents + j]) and sc.
+static __device__ __noinline__ void seq_prepare(const double *part, int G, double *rec, SeqScratch *sc)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k0 = threadIdx.x * kSeqPer;
+    double v[kSeqPer];
+    uint32_t emax = 0, any = 0;
+#pragma unroll
+    for (int u = 0; u < kSeqPer; ++u) v[u] = k0 + u < G ? ld_cg(part + k0 + u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < kSeqPer; ++u) {
+        emax = max(emax, ((uint32_t)__double2hiint(v[u]) >> 20) & 0x7ffu);
+        any |= v[u] != 0.0;
+    }
+    emax = __reduce_max_sync(kFull, emax);
+    any = __reduce_or_sync(kFull, any);
+    if (lane == 0) {
+        sc->wmax[warp] = emax;
+        sc->wor[warp] = any;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        emax = max(emax, sc->wmax[w]);
+        any |= sc->wor[w];
+    }
+    if (!any || emax < 128u || emax > 1900u || G > kSeqMax) {   // (uniform)
+        if (threadIdx.x == 0) {
+            sc->events = any ? -1 : 0;
+            sc->qtot = 0;
+        }
+        __syncthreads();
+        return;
+    }
+    // exact prefixes in units of 2^(emax - 1073)
+    long long f[kSeqPer], fsum = 0;
+#pragma unroll
+    for (int u = 0; u < kSeqPer; ++u) {
+        const long long b = __double_as_longlong(v[u]);
+        const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
+        const uint32_t sh = emax - e + 2;
+        const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
+        const long long q = sh < 64u ? (long long)(m >> sh) : 0ll;
+        f[u] = b < 0 ? -q : q;
+        fsum += f[u];
+    }
+    long long P = seq_block_scan(fsum, sc->wsum) - fsum;
+    long long q[kSeqPer], qsum = 0;
+    uint32_t ev = 0;
+#pragma unroll
+    for (int u = 0; u < kSeqPer; ++u) {
+        const long long Pb = P, Pa = P + f[u];
+        P = Pa;
+        const unsigned long long ab = Pb < 0 ? -Pb : Pb, aa = Pa < 0 ? -Pa : Pa;
+        const int pos = 63 - __clzll((long long)ab);            // -1 for 0
+        const long long b = __double_as_longlong(v[u]);
+        const int e = (int)((uint32_t)(b >> 52) & 0x7ffu);
+        const int d = pos + (int)emax - 50 - e;                 // log2 of the sum's unit over the value's
+        const unsigned long long lo = (1ull << (pos & 63)) + kSeqBand, hi = (2ull << (pos & 63)) - kSeqBand;
+        const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | (1ull << 52);
+        bool event = pos < 22 || ab < lo || ab > hi || aa < lo || aa > hi || (Pa ^ Pb) < 0 || d < -1;
+        unsigned long long r = 0;
+        if (d < 0) {
+            r = m << 1;
+        } else if (d < 54) {
+            r = m >> d;
+            const unsigned long long rest = m & ((1ull << d) - 1);
+            const unsigned long long half = d ? 1ull << (d - 1) : 0ull;
+            if (d && rest == half) event = true;
+            if (rest > half) ++r;
+        }
+        if (v[u] == 0.0) {
+            event = false;
+            r = 0;
+        }
+        q[u] = event ? 0ll : (b < 0 ? -(long long)r : (long long)r);
+        qsum += q[u];
+        ev |= (event ? 1u : 0u) << u;
+    }
+    uint32_t cnt = __popc(ev);
+    uint32_t pre = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, pre, o);
+        if (lane >= o) pre += t;
+    }
+    if (lane == 31) sc->wcnt[warp] = pre;
+    __syncthreads();   // wsum of the first scan is consumed, wcnt visible
+    long long Q = seq_block_scan(qsum, sc->wsum);
+    uint32_t at = pre - cnt, all = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        if (w < warp) at += sc->wcnt[w];
+        all += sc->wcnt[w];
+    }
+    if (threadIdx.x == kBlock - 1) {
+        sc->qtot = Q;
+        sc->events = all <= kSeqEvents ? (int32_t)all : -1;
+    }
+    Q -= qsum;
+#pragma unroll
+    for (int u = 0; u < kSeqPer; ++u) {
+        if ((ev >> u) & 1u) {
+            if (at < kSeqEvents) {
+                rec[at] = v[u];
+                rec[kSeqEvents + at] = __longlong_as_double(Q);
+            }
+            ++at;
+        }
+        Q += q[u];
+    }
+    __syncthreads();
+}
+
+// One warp: the sum itself.
+static __device__ __noinline__ double seq_finish(const double *part, int G, const double *rec, const SeqScratch *sc)
+{
+    double s = 0.0;
+    const int n = sc->events;
+    if (n < 0) {
+        const int lane = threadIdx.x & 31;
+        for (int b = 0; b < G; b += 32) {
+            const double t = b + lane < G ? ld_cg(part + b + lane) : 0.0;
+            const int m = min(32, G - b);
+            for (int l = 0; l < m; ++l) s += __shfl_sync(kFull, t, l);
+        }
+        return s;
+    }
+    long long Qp = 0;
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+        const double v = rec[j];
+        const long long Q = __double_as_longlong(rec[kSeqEvents + j]), dq = Q - Qp;
+        const long long b = __double_as_longlong(s);
+        Qp = Q;
+        s = __longlong_as_double(b + (b < 0 ? -dq : dq)) + v;
+    }
+    const long long b = __double_as_longlong(s), dq = sc->qtot - Qp;
+    return __longlong_as_double(b + (b < 0 ? -dq : dq));
+}
+
 // Single-pass grid reduction.  Every block publishes its NV partials; the
 // block that arrives last sums them in a fixed order (sequentially in block
 // order for the reference order, else a strided sum + block tree), so the
@@ -110,7 +315,8 @@ template <int NV, class T>
 __device__ __forceinline__ bool grid_reduce(T (&acc)[NV], T *partials, int stride,
                                             uint32_t *counter, bool ref_order, T (&out)[NV])
 {
-    __shared__ T sm[NV * kBlock];
+    // (the reference order's sequential sums use it for their events)
+    __shared__ T sm[NV * (sizeof(T) == 8 ? 2 * kSeqEvents : kBlock)];
     __shared__ bool s_last;
     pdl_trigger();
 #if CF_FAST_BLOCK_SUM
@@ -130,38 +336,23 @@ __device__ __forceinline__ bool grid_reduce(T (&acc)[NV], T *partials, int strid
     __threadfence();
     const int G = gridDim.x;
     if (ref_order) {
-        // the partials in block order, one sequential sum per value; the
-        // whole block stages them through shared memory a chunk at a time
-        // so that thread 0 adds from shared memory instead of waiting on
-        // one L2 load per partial
-        T run[NV];
-#pragma unroll
-        for (int i = 0; i < NV; ++i) run[i] = T(0);
-        for (int b0 = 0; b0 < G; b0 += kBlock) {
-            const int m = min(kBlock, G - b0);
-            __syncthreads(); // the previous chunk (or the block sum) is consumed
-            if (threadIdx.x < m)
-#pragma unroll
-                for (int i = 0; i < NV; ++i) sm[i * kBlock + threadIdx.x] = ld_cg(partials + i * stride + b0 + threadIdx.x);
+        // the partials in block order, one sequential sum per value: the
+        // block prepares each value's events, warp i adds up value i
+        if constexpr (sizeof(T) == 8) {
+            __shared__ SeqScratch sc[NV];
+            __syncthreads(); // the block sum's use of sm is over
+#pragma unroll 1
+            for (int i = 0; i < NV; ++i) seq_prepare(partials + i * stride, G, sm + i * 2 * kSeqEvents, &sc[i]);
+            const int warp = threadIdx.x >> 5;
+            double run = 0.0;
+            if (warp < NV) run = seq_finish(partials + warp * stride, G, sm + warp * 2 * kSeqEvents, &sc[warp]);
             __syncthreads();
-            if (threadIdx.x == 0) {
-                if (m == kBlock) {
-                    // a full chunk: a fixed trip count lets the shared
-                    // loads run ahead of the dependent additions
-#pragma unroll 32
-                    for (int b = 0; b < kBlock; ++b)
+            if (warp < NV && (threadIdx.x & 31) == 0) sm[warp] = run;
+            __syncthreads();
+            if (threadIdx.x == 0)
 #pragma unroll
-                        for (int i = 0; i < NV; ++i) run[i] += sm[i * kBlock + b];
-                } else {
-                    for (int b = 0; b < m; ++b)
-#pragma unroll
-                        for (int i = 0; i < NV; ++i) run[i] += sm[i * kBlock + b];
-                }
-            }
+                for (int i = 0; i < NV; ++i) out[i] = sm[i];
         }
-        if (threadIdx.x == 0)
-#pragma unroll
-            for (int i = 0; i < NV; ++i) out[i] = run[i];
     } else {
         // thread t adds partials t, t + 256, ... in that order; for grids of
         // up to 5 * 256 blocks (the fast grid is at most 8 blocks per SM,
