@@ -666,6 +666,14 @@ __device__ __forceinline__ uint64_t l2_evict_first_policy()
     return p;
 }
 
+// ... and for a matrix that fits in L2 beside the vectors
+__device__ __forceinline__ uint64_t l2_evict_normal_policy()
+{
+    uint64_t p;
+    asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+
 __device__ __forceinline__ double ld_stream(const double *p, uint64_t pol)
 {
     double v;
@@ -937,22 +945,20 @@ __device__ __forceinline__ void sell_long_rows(int n, int s, const int32_t *__re
     }
 }
 
-// sum_t val[t] g(col[t]) of this lane's row of slice s (sell_slice), and
-// f(row, sum) for every row, one warp per slice (sell_rows); the entries are taken B at a time (all B loads and gathers issued before the
-// first FMA), the row's last r < B entries as an exact batch: a guarded slot
+// sum_t val[t] g(col[t]) of this lane's row of slice s, at element b with len
+// slots (sell_slice_at), and f(row, sum) for every row, one warp per slice
+// (sell_rows); the entries are taken B at a time (all B loads and gathers
+// issued before the first FMA), the row's last r < B entries as an exact batch: a guarded slot
 // of a full batch would still issue its FMA (measured: 9 DFMA per 7-entry
 // row).  The slice length is warp-uniform, so the branches never diverge.
 // Matrices with rows longer than kLongRow (has_long) sum those rows with
 // the whole warp (sell_long_rows), as the CSR passes do.  cs: the columns
 // (SellCols32 or SellCodes8).
 template <class V, int B, class C, class G>
-__device__ __forceinline__ V sell_slice(int n, int s, const int32_t *__restrict__ off, const C &cs,
-                                        const V *__restrict__ val, const int32_t *__restrict__ ro, bool has_long,
-                                        uint64_t pol, G g)
+__device__ __forceinline__ V sell_slice_at(int n, int s, int b, int len, const C &cs, const V *__restrict__ val,
+                                           const int32_t *__restrict__ ro, bool has_long, uint64_t pol, G g)
 {
     const int lane = threadIdx.x & 31;
-    const int b = __ldg(off + s);
-    const int len = (__ldg(off + s + 1) - b) >> 5;
     const int rb = sell_row_base(s * 32 + lane, n);
     const V *vp = val + (int64_t)b + lane;
     V acc = V(0);
@@ -971,7 +977,9 @@ __device__ __forceinline__ void sell_rows(int n, int n_slices, const int32_t *__
     const uint64_t pol = l2_evict_first_policy();
     const int nw = gridDim.x * kWarps;
     for (int s = blockIdx.x * kWarps + (threadIdx.x >> 5); s < n_slices; s += nw) {
-        const V acc = sell_slice<V, B>(n, s, off, cs, val, ro, has_long, pol, g);
+        const int b = __ldg(off + s);
+        const int len = (__ldg(off + s + 1) - b) >> 5;
+        const V acc = sell_slice_at<V, B>(n, s, b, len, cs, val, ro, has_long, pol, g);
         const int row = s * 32 + (threadIdx.x & 31);
         if (row < n) f(row, acc);
     }

@@ -194,6 +194,7 @@ struct Context {
     int grid_cap = 0;
     int small_cg_ok = -1;      // 16-CTA clusters schedulable (-1: not asked yet)
     int coop_ok = -1;          // cooperative launches supported (-1: not asked yet)
+    int cluster16_ok = 0;      // a 16-block cluster of k_persist fits (asked with coop_ok)
     DeviceBuffer persist;      // grid-persistent solves: block partials, barrier counter
 
     // scratch of the matrix builds (grow-only: a conversion after the first
@@ -255,6 +256,7 @@ struct Matrix {
     int sell = -1;             // -1 not decided, 0 CSR kernels, 1 SELL-32
     int32_t n_slices = 0;
     int64_t sell_nnz = 0;      // stored entries including padding
+    int32_t sell_max_len = 0;  // slots per row of the longest slice
     DeviceBuffer s_off, s_col, s_val, s_valT, s_val32, s_valT32;
     // one-byte column codes of the SELL-32 slots and the table of offsets
     // col - row they index (n_codes distinct offsets; 0: 32-bit columns only)
@@ -324,9 +326,9 @@ SmallSolveResult solve_small_single_cluster(Matrix *m, int solver, const cf_cont
                                             double *x, double *r, double *d, double *y);
 bool small_cg_ok(Context *ctx);
 
-// a whole FP64 solve in the fast order as one cooperative launch (persist.cu)
-const void *persist_kernel_for(Context *ctx, int solver, int format);
-void launch_persist(Context *ctx, const void *kernel, int solver, const SolveArgs &A, const DevState &S, int l1,
+// a whole FP64 solve in the fast order as one launch (persist.cu)
+bool persist_usable(Context *ctx, int solver, int format);
+void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1, int max_len,
                     DevState *out);
 void persist_reset(Context *ctx);
 

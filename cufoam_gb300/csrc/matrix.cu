@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv_sell_ref(int n, int n_slices, c
 // SELL-32 copy (layout described in device.cuh)
 // ---------------------------------------------------------------------------
 // slot s: 32 x the longest row of slice s (slot n_slices = 0); the stored
-// total accumulates in 64 bits
+// total accumulates in 64 bits in total[0], the longest row in total[1]
 __global__ void k_sell_len(int n, int n_slices, const int32_t *__restrict__ ro, int32_t *slen,
                            unsigned long long *total)
 {
@@ -313,6 +313,8 @@ __global__ void k_sell_len(int n, int n_slices, const int32_t *__restrict__ ro, 
             const int r1 = min(n, 32 * s + 32);
             for (int r = 32 * s; r < r1; ++r) mx = max(mx, __ldg(ro + r + 1) - __ldg(ro + r));
             atomicAdd(total, 32ull * (unsigned long long)mx);
+            if ((unsigned long long)mx > *(volatile unsigned long long *)(total + 1))
+                atomicMax(total + 1, (unsigned long long)mx);
         }
         slen[s] = 32 * mx;
     }
@@ -1116,8 +1118,8 @@ bool matrix_ensure_sell(Matrix *m, bool transpose, bool fp32)
             m->s_off.ensure(sizeof(int32_t) * ((size_t)ns + 1));
             DeviceBuffer slen, tmp, tot;
             slen.ensure(sizeof(int32_t) * ((size_t)ns + 1));
-            tot.ensure(sizeof(unsigned long long));
-            CF_CUDA(cudaMemsetAsync(tot.ptr, 0, sizeof(unsigned long long), ctx->stream));
+            tot.ensure(2 * sizeof(unsigned long long));
+            CF_CUDA(cudaMemsetAsync(tot.ptr, 0, 2 * sizeof(unsigned long long), ctx->stream));
             k_sell_len<<<grid_for(ctx, (int64_t)ns + 1), kBlock, 0, ctx->stream>>>(
                 m->n, ns, m->ro.as<int32_t>(), slen.as<int32_t>(), tot.as<unsigned long long>());
             CF_CHECK_LAUNCH();
@@ -1125,13 +1127,14 @@ bool matrix_ensure_sell(Matrix *m, bool transpose, bool fp32)
             const bool want_codes = req == CF_FORMAT_AUTO || req == CF_FORMAT_SELL_C8;
             const bool want_d16 = req == CF_FORMAT_AUTO || req == CF_FORMAT_SELL_D16;
             if (want_codes || want_d16) queue_offsets(m);
-            unsigned long long total = 0;
+            unsigned long long sizes[2] = {0, 0};
             std::vector<int32_t> hk(want_codes || want_d16 ? kCodeHash + 2 : 0);
-            CF_CUDA(cudaMemcpyAsync(&total, tot.ptr, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
+            CF_CUDA(cudaMemcpyAsync(sizes, tot.ptr, sizeof(sizes), cudaMemcpyDeviceToHost, ctx->stream));
             if (want_codes || want_d16)
                 CF_CUDA(cudaMemcpyAsync(hk.data(), ctx->scratch_codes.ptr, sizeof(int32_t) * (kCodeHash + 2),
                                         cudaMemcpyDeviceToHost, ctx->stream));
             CF_CUDA(cudaStreamSynchronize(ctx->stream));
+            const unsigned long long total = sizes[0];
             const bool fits = total < (unsigned long long)INT32_MAX - 64;
             const bool good = fits && (double)total <= 1.2 * (double)m->nnz + 32.0 * 8 &&
                               m->nnz <= 32 * (int64_t)m->n;
@@ -1141,6 +1144,7 @@ bool matrix_ensure_sell(Matrix *m, bool transpose, bool fp32)
                 exclusive_scan(ctx, ns + 1, slen.as<int32_t>(), m->s_off.as<int32_t>(), tmp);
                 m->n_slices = ns;
                 m->sell_nnz = (int64_t)total;
+                m->sell_max_len = (int32_t)sizes[1];
                 m->s_col.ensure(sizeof(int32_t) * ((size_t)total + 32));
                 k_sell_fill<double, double><<<grid_for(ctx, 32 * (int64_t)ns), kBlock, 0, ctx->stream>>>(
                     m->n, ns, m->ro.as<int32_t>(), m->col.as<int32_t>(), nullptr, m->s_off.as<int32_t>(),

@@ -16,6 +16,7 @@ namespace cf {
 // passes of the multi-kernel loop have (four blocks of 256), and a quarter
 // of their arrivals at the grid barrier.  Measured on GB300 (152 SMs): 1.2
 // us per barrier with 152 arrivals, 2.1 us with 608.
+// (fewer warps where a block has fewer slices)
 constexpr int kPBlock = 1024;
 constexpr int kPWarps = kPBlock / 32;
 constexpr int kPMaxNV = 4;
@@ -133,32 +134,65 @@ __device__ __forceinline__ void red_release(uint32_t *p)
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
 }
 
-struct PersistShared {
+constexpr int kPClusterMax = 16;       // blocks of a cluster
+
+// SLOTS: room for the warp sums of every block of a cluster, by parity
+// (1 where the sums go through global memory)
+template <int SLOTS> struct PersistShared {
     double w[kPMaxNV][kPWarps];
-    double tot[kPMaxNV];
-    int32_t fail;          // the barrier gave up
-    int32_t stop;          // block 0 asked for an early end
+    double slot[2][kPMaxNV][SLOTS];
+    int32_t slot_stop[2];
+    int32_t fail;              // the grid barrier gave up
+    int32_t stop;              // block 0 asked for an early end
 };
 
-// The grid-wide state of one block: every thread holds a copy.
-struct PersistSync {
+// the block's sums of v in s (valid in warp 0)
+template <int NV>
+__device__ __forceinline__ void block_sum_fixed(const double (&v)[NV], PersistShared<1> *sh, double (&s)[NV])
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const double t[1] = {v[i]};
+        const double x = warp_sum_fixed<1>(t);
+        if (lane == 0) sh->w[i][warp] = x;
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const double t[1] = {lane < nw ? sh->w[i][lane] : 0.0};
+            s[i] = warp_sum_fixed<1>(t);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The two scopes a solve runs in.  Both offer
+//   barrier()  all blocks' writes before it are visible after it;
+//   sum(v, abort_flag, post)  sums over all blocks; thread 0 of every block
+//              runs post(totals) (the step logic, the same bits everywhere)
+//              before any thread goes on.  Also a barrier.  `abort_flag`,
+//              read by block 0, arrives in sh->stop.
+// and return false when a wait gave up (grid only).
+// ---------------------------------------------------------------------------
+struct GridSync {
+    using Shared = PersistShared<1>;
     PersistGrid g;
-    PersistShared *sh;
+    Shared *sh;
     uint32_t epoch;        // barriers passed
     uint32_t red;          // sums done
 
-    __device__ __forceinline__ void init(const PersistGrid &g_, PersistShared *sh_)
+    __device__ __forceinline__ GridSync(const PersistGrid &g_, Shared *sh_) : g(g_), sh(sh_), epoch(0), red(0)
     {
-        g = g_;
-        sh = sh_;
-        epoch = 0;
-        red = 0;
         if (threadIdx.x == 0) {
             sh->fail = 0;
             sh->stop = 0;
         }
         __syncthreads();
     }
+    __device__ __forceinline__ int rank() const { return blockIdx.x; }
+    __device__ __forceinline__ int blocks() const { return gridDim.x; }
 
     // thread 0: arrive (releasing the block's writes) and wait for all blocks
     __device__ __forceinline__ void arrive_wait()
@@ -173,7 +207,6 @@ struct PersistSync {
             }
     }
 
-    // all of the grid's writes before it are visible after it; false: gave up
     __device__ __forceinline__ bool barrier()
     {
         __syncthreads();
@@ -183,50 +216,36 @@ struct PersistSync {
         return !sh->fail;
     }
 
-    // Sums over the grid: totals in sh->tot for every thread, after
-    // `post(tot)` ran in thread 0 (the step logic: the same in every block).
-    // Also a grid barrier.  `abort_flag` (block 0 reads it) ends the solve.
     template <int NV, class Post>
     __device__ __forceinline__ bool sum(const double (&v)[NV], const volatile int32_t *abort_flag, Post post)
     {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int lane = threadIdx.x & 31;
         const int G = gridDim.x;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const double t[1] = {v[i]};
-            const double s = warp_sum_fixed<1>(t);
-            if (lane == 0) sh->w[i][warp] = s;
-        }
-        __syncthreads();
-        if (warp == 0) {
+        double s[NV];
+        block_sum_fixed(v, sh, s);
+        if (threadIdx.x < 32) {
             double *part = g.part + (size_t)(red & 1) * kPMaxNV * kPMaxGrid;
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                const double t[1] = {sh->w[i][lane]};
-                const double s = warp_sum_fixed<1>(t);
-                if (lane == 0) part[i * kPMaxGrid + blockIdx.x] = s;
-            }
             if (lane == 0) {
+#pragma unroll
+                for (int i = 0; i < NV; ++i) part[i * kPMaxGrid + blockIdx.x] = s[i];
                 if (blockIdx.x == 0) g.stop[red & 1] = abort_flag ? *abort_flag : 0;
                 arrive_wait();
             }
             __syncwarp();
             constexpr int kPer = kPMaxGrid / 32;
-            double s[NV];
+            double t[NV][kPer];
 #pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                double t[kPer];
+            for (int i = 0; i < NV; ++i)
 #pragma unroll
                 for (int u = 0; u < kPer; ++u) {
                     const int b = lane + 32 * u;
-                    t[u] = b < G ? ld_cg(part + i * kPMaxGrid + b) : 0.0;
+                    t[i][u] = b < G ? ld_cg(part + i * kPMaxGrid + b) : 0.0;
                 }
-                s[i] = warp_sum_fixed<kPer>(t);
-            }
-            if (lane == 0) {
-                sh->stop = ld_cg(g.stop + (red & 1));
+            const int32_t stop = abort_flag ? ld_cg(g.stop + (red & 1)) : 0;
 #pragma unroll
-                for (int i = 0; i < NV; ++i) sh->tot[i] = s[i];
+            for (int i = 0; i < NV; ++i) s[i] = warp_sum_fixed<kPer>(t[i]);
+            if (lane == 0) {
+                sh->stop = stop;
                 post(s);
             }
         }
@@ -246,5 +265,103 @@ struct PersistSync {
         }
     }
 };
+
+// one thread-block cluster: the hardware barrier, sums through distributed
+// shared memory
+struct ClusterSync {
+    using Shared = PersistShared<kPClusterMax * kPWarps>;
+    Shared *sh;
+    uint32_t red;
+    uint32_t me, n;
+
+    __device__ __forceinline__ ClusterSync(const PersistGrid &, Shared *sh_) : sh(sh_), red(0)
+    {
+        asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(me));
+        asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+        if (threadIdx.x == 0) {
+            sh->fail = 0;
+            sh->stop = 0;
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ int rank() const { return (int)me; }
+    __device__ __forceinline__ int blocks() const { return (int)n; }
+    __device__ __forceinline__ bool barrier()
+    {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return true;
+    }
+    template <class T>
+    __device__ __forceinline__ uint32_t remote(const T *p, uint32_t rank) const
+    {
+        uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+        return r;
+    }
+    template <int K> static __device__ __forceinline__ double sum_slots(const double *w, int m)
+    {
+        const int lane = threadIdx.x & 31;
+        double t[K];
+#pragma unroll
+        for (int u = 0; u < K; ++u) t[u] = lane + 32 * u < m ? w[lane + 32 * u] : 0.0;
+        return warp_sum_fixed<K>(t);
+    }
+    // Every warp stores its sum into every block's shared memory; after the
+    // cluster barrier warp 0 of each block adds up what it has (no second
+    // stage, no remote loads).
+    template <int NV, class Post>
+    __device__ __forceinline__ bool sum(const double (&v)[NV], const volatile int32_t *abort_flag, Post post)
+    {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        const int par = red & 1;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const double t[1] = {v[i]};
+            const double x = warp_sum_fixed<1>(t);
+            if (lane < (int)n)
+                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote(&sh->slot[par][i][me * nw + warp],
+                                                                              (uint32_t)lane)),
+                             "d"(x)
+                             : "memory");
+        }
+        if (abort_flag && me == 0 && warp == 0 && lane < (int)n) {
+            const int32_t stop = *abort_flag;
+            asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(remote(&sh->slot_stop[par], (uint32_t)lane)),
+                         "r"(stop)
+                         : "memory");
+        }
+        barrier();
+        if (threadIdx.x < 32) {
+            const int m = (int)n * nw;
+            double s[NV];
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                const double *w = sh->slot[par][i];
+                s[i] = m <= 128 ? sum_slots<4>(w, m) : m <= 256 ? sum_slots<8>(w, m) : sum_slots<16>(w, m);
+            }
+            if (lane == 0) {
+                sh->stop = abort_flag ? sh->slot_stop[par] : 0;
+                post(s);
+            }
+        }
+        ++red;
+        __syncthreads();
+        return true;
+    }
+    // no block leaves while a peer may still read its shared memory
+    __device__ __forceinline__ void leave() { barrier(); }
+};
+
+// a / b with the correctly rounded reciprocal rb = 1 / b at hand: the
+// rounding of a division (Markstein: one residual step from a correctly
+// rounded reciprocal), three dependent FP64 operations instead of about ten
+__device__ __forceinline__ double div_by_reciprocal(double a, double b, double rb)
+{
+    const uint32_t ea = ((uint32_t)__double2hiint(a) >> 20) & 0x7ffu, eb = ((uint32_t)__double2hiint(b) >> 20) & 0x7ffu;
+    if (ea - 200u > 1600u || eb - 200u > 1600u) return a / b;   // zero, near the range's ends, or not finite
+    const double q = __dmul_rn(a, rb);
+    return __fma_rn(__fma_rn(-q, b, a), rb, q);
+}
 
 } // namespace cf

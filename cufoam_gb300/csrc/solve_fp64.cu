@@ -522,11 +522,10 @@ static Kernels body_kernels(int solver, bool sell)
 
 static size_t vec_bytes(int n) { return sizeof(double) * ((size_t)n + 8); }
 
-// Systems up to this many rows solve CG (fast order, FP64, no history) in one
-// cluster-persistent launch instead of the multi-kernel loop: at 64^2 8.7 us
-// per step against 16.7; from ~14k rows on (24^3: 17.4 against 17-20 us)
-// the loop's full-GPU passes are as fast, and at 40^3 the single cluster is
-// 2.5x slower.
+// CSR systems (rows too uneven for SELL-32) up to this many rows solve in one
+// cluster-persistent launch (batched.cu) instead of the multi-kernel loop: CG
+// at 64^2 7.0 us per step against 16.7; from ~14k rows on the loop's
+// full-GPU passes are as fast.
 #ifndef CF_SMALL_CG_ROWS
 #define CF_SMALL_CG_ROWS 8192
 #endif
@@ -636,13 +635,14 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     const bool hist_time = want_hist && c.history_time != 0;
     if (hist_time) ctx->hist_t.ensure(sizeof(unsigned long long) * (size_t)hist_cap);
 
-    // ---- a small system: one cluster-persistent launch -----------------
+    // ---- a small system in CSR: one cluster-persistent launch ----------
+    // (over SELL-32 the solve below is one launch at every size)
     // (kernel boundaries, not bytes, set a small system's step time; CG runs
     // in the batched kernel, Jacobi, Richardson and the MR family in
     // k_small_solve, the whole solve behind hardware cluster barriers)
     const bool small_kind = solver == CF_CG || solver == CF_JACOBI || solver == CF_RICHARDSON ||
                             solver == CF_MR || solver == CF_MRJACOBI || solver == CF_MRS || solver == CF_JMR;
-    if (small_kind && !ref && !mixed && !tr && n <= kSmallCgRows && !want_hist &&
+    if (!sell && small_kind && !ref && !mixed && !tr && n <= kSmallCgRows && !want_hist &&
         c.time_limit_s <= 0 && c.profile_kernels == 0 && c.rel_tol == 0 && c.min_iter <= 0 &&
         c.norm_type == CF_NORM_REFERENCE_L2 && !c.absolute_tolerance && c.use_graph != 0 && small_cg_ok(ctx)) {
         const SmallSolveResult R =
@@ -750,8 +750,8 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     const int fmt = solve_format(A);
     const Kernels kk = ref ? body_kernels(solver, sell) : fast_body_kernels(solver, fmt);
     SolveArgs *d_args = ctx->args.as<SolveArgs>();
-    // the fast order over the SELL-32 copy: one cooperative launch
-    const void *persist = (use_graph && !ref && !mixed) ? persist_kernel_for(ctx, solver, fmt) : nullptr;
+    // the fast order over the SELL-32 copy: one launch
+    const bool persist = use_graph && !ref && !mixed && persist_usable(ctx, solver, fmt);
     if (use_graph && !mixed && !persist) {
         try {
             ge = loop_graph(ctx, kk, solver, CF_PREC_FP64, cap, ref, d_args, fmt);
@@ -770,7 +770,7 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     MixedResult mres;
     if (persist) {
         CF_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
-        launch_persist(ctx, persist, solver, A, S, l1, ctx->h_state);
+        launch_persist(ctx, solver, fmt, A, S, l1, m->sell_max_len, ctx->h_state);
         CF_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
     } else {
     CF_CUDA(cudaMemcpyAsync(d_args, &A, sizeof(SolveArgs), cudaMemcpyHostToDevice, ctx->stream));
