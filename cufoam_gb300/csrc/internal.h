@@ -327,9 +327,13 @@ SmallSolveResult solve_small_single_cluster(Matrix *m, int solver, const cf_cont
 bool small_cg_ok(Context *ctx);
 
 // a whole FP64 solve in the fast order as one launch (persist.cu)
-bool persist_usable(Context *ctx, int solver, int format);
+bool persist_usable(Context *ctx, int solver, int format, bool mixed);
 void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1, int max_len,
                     DevState *out);
+// ... and a whole mixed-precision solve (persist_mixed.cu); the total of FP32
+// steps in out_in->k
+void launch_persist_mixed(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1,
+                          int max_len, const cf_controls &c, DevState *out, DevState *out_in);
 void persist_reset(Context *ctx);
 
 struct Batch;
@@ -362,6 +366,7 @@ struct MixedResult {
     int status = CF_OK;
 };
 bool mixed_supported(int solver);
+double mixed_inner_tolerance(const cf_controls &c, int solver);
 void mixed_prepare(Context *ctx, Matrix *m, int solver, SolveArgs &A);
 MixedResult run_mixed(Context *ctx, Matrix *m, int solver, const cf_controls &c, SolveArgs *d_args,
                       int cap, bool use_graph);

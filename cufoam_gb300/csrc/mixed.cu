@@ -443,6 +443,14 @@ bool mixed_supported(int solver)
     return solver == CF_CG || solver == CF_BICG || solver == CF_MR || mr_scaled_solver(solver);
 }
 
+// default inner tolerance per solver, the fastest measured on GB300: CG at
+// 128^3 27.5 ms with 1e-6 against 32.4 ms with 1e-4 (fewer restarts of the
+// Krylov space); BiCG and MR on C3 within 3% for 1e-4 .. 1e-6
+double mixed_inner_tolerance(const cf_controls &c, int solver)
+{
+    return (c.mixed_inner_rtol > 0 && c.mixed_inner_rtol < 1) ? c.mixed_inner_rtol : (solver == CF_CG ? 1e-6 : 1e-4);
+}
+
 void mixed_prepare(Context *ctx, Matrix *m, int solver, SolveArgs &A)
 {
     require(mixed_supported(solver), CF_UNSUPPORTED,
@@ -528,11 +536,7 @@ MixedResult run_mixed(Context *ctx, Matrix *m, int solver, const cf_controls &c,
     CF_CUDA(cudaStreamSynchronize(ctx->stream));
     const int64_t max_total = c.max_iter <= 0 ? INT_MAX : c.max_iter;
     const int max_outer = c.mixed_max_outer > 0 ? c.mixed_max_outer : 50;
-    // default inner tolerance per solver, the fastest measured on GB300: CG
-    // at 128^3 27.5 ms with 1e-6 against 32.4 ms with 1e-4 (fewer restarts of
-    // the Krylov space); BiCG and MR on C3 within 3% for 1e-4 .. 1e-6
-    const double eta = (c.mixed_inner_rtol > 0 && c.mixed_inner_rtol < 1) ? c.mixed_inner_rtol
-                                                                          : (solver == CF_CG ? 1e-6 : 1e-4);
+    const double eta = mixed_inner_tolerance(c, solver);
     // every inner sweep runs to the inner tolerance unless capped
     int inner_cap = c.mixed_inner_max > 0 ? c.mixed_inner_max : INT_MAX;
     // x and r before each correction, to undo a sweep that made things worse

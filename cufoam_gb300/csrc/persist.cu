@@ -139,40 +139,6 @@ template <> struct PersistCols<kSellD> {
     static __device__ __forceinline__ SellDelta16 make(const SolveArgs &A) { return SellDelta16{A.s_d16}; }
 };
 
-// sell_slice over slots in shared memory (cp, vp: this lane's first slot):
-// the same chain in the same order
-template <int M, class G>
-__device__ __forceinline__ void local_batch(const int32_t *cp, const double *vp, G g, double &acc)
-{
-    double v[M], x[M];
-#pragma unroll
-    for (int u = 0; u < M; ++u) x[u] = g(cp[32 * u]);
-#pragma unroll
-    for (int u = 0; u < M; ++u) v[u] = vp[32 * u];
-#pragma unroll
-    for (int u = 0; u < M; ++u) acc = fma_t(v[u], x[u], acc);
-}
-template <int B, class G>
-__device__ __forceinline__ void local_tail(int r, const int32_t *cp, const double *vp, G g, double &acc)
-{
-    if constexpr (B > 1) {
-        if (r == B - 1) {
-            local_batch<B - 1>(cp, vp, g, acc);
-            return;
-        }
-        local_tail<B - 1>(r, cp, vp, g, acc);
-    }
-}
-template <class G>
-__device__ __forceinline__ double local_slice(const int32_t *cp, const double *vp, int len, G g)
-{
-    double acc = 0.0;
-    int t0 = 0;
-    for (; t0 + kSellBatch <= len; t0 += kSellBatch) local_batch<kSellBatch>(cp + 32 * t0, vp + 32 * t0, g, acc);
-    local_tail<kSellBatch>(len - t0, cp + 32 * t0, vp + 32 * t0, g, acc);
-    return acc;
-}
-
 // LOCALM: this block's slots of the matrix and its vectors stay in shared
 // memory for the whole solve, and only the gathered vector crosses blocks.
 // SYNC: the grid, or one cluster.
@@ -248,7 +214,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
         const int o = off[s - s_lo], len = (off[s - s_lo + 1] - o) >> 5;
         if constexpr (LOCALM) {
             const int l = o - off[0] + lane;
-            return local_slice(lcol + l, lval + l, len, g);
+            return local_slice<double, kSellBatch>(lcol + l, lval + l, len, g);
         } else {
             return sell_slice_at<double, kSellBatch>(n, s, o, len, cols, val, A.ro, has_long, pol, g);
         }
@@ -258,7 +224,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
         const int o = off[s - s_lo], len = (off[s - s_lo + 1] - o) >> 5;
         if constexpr (LOCALM && !Tr::kScaledMatrix) {
             const int l = o - off[0] + lane;
-            return local_slice(lcol + l, lval + l, len, g);
+            return local_slice<double, kSellBatch>(lcol + l, lval + l, len, g);
         } else {
             return sell_slice_at<double, kSellBatch>(n, s, o, len, cols, A.s_val, A.ro, has_long, pol, g);
         }
@@ -570,8 +536,6 @@ out:
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-enum { kScopeGrid = 0, kScopeGridLocal = 1, kScopeCluster = 2 };
-
 template <int SOLVER>
 static const void *persist_pick(int scope, int format)
 {
@@ -601,9 +565,10 @@ static const void *persist_kernel(int solver, int scope, int format)
 // multi-kernel loop at every size, see the top of the file); CSR matrices
 // (their staging buffers), BiCG's fast order and devices without cooperative
 // launches or with more SMs than the partial sums are sized for run the loop.
-bool persist_usable(Context *ctx, int solver, int format)
+bool persist_usable(Context *ctx, int solver, int format, bool mixed)
 {
-    if (format == kCsr || !persist_kernel(solver, kScopeGrid, format) || ctx->sm_count > kPMaxGrid) return false;
+    if (format == kCsr || ctx->sm_count > kPMaxGrid) return false;
+    if (!mixed && !persist_kernel(solver, kScopeGrid, format)) return false;
     if (ctx->coop_ok < 0) {
         int coop = 0;
         if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) != cudaSuccess) {
@@ -633,21 +598,45 @@ bool persist_usable(Context *ctx, int solver, int format)
     return ctx->coop_ok == 1;
 }
 
-// Dynamic shared memory of a block: at most this much in all, and at most
-// CF_PERSIST_VEC_BYTES for vectors alone when the matrix streams from L2 or
-// HBM (the rest of the SM's 256 KB is the L1 of the gathers).
-#ifndef CF_PERSIST_LOCAL_BYTES
-#define CF_PERSIST_LOCAL_BYTES (200 * 1024)
-#endif
-#ifndef CF_PERSIST_VEC_BYTES
-#define CF_PERSIST_VEC_BYTES (144 * 1024)
-#endif
-// Systems up to this many rows run in one cluster of up to 16 blocks: CG step
-// 5.4 us against 8.1 on the grid at 4,096 rows, 6.7 against 8.1 at 8,100, 8.6
-// against 8.3 at 12,100.
-#ifndef CF_PERSIST_CLUSTER_ROWS
-#define CF_PERSIST_CLUSTER_ROWS 10240
-#endif
+PersistGrid persist_grid(Context *ctx)
+{
+    const size_t part = sizeof(double) * 2 * kPMaxNV * kPMaxGrid;
+    if (ctx->persist.bytes == 0) {
+        ctx->persist.ensure(part + 64);
+        CF_CUDA(cudaMemsetAsync(ctx->persist.ptr, 0, part + 64, ctx->stream));
+    }
+    PersistGrid g;
+    g.part = ctx->persist.as<double>();
+    g.count = reinterpret_cast<uint32_t *>(static_cast<char *>(ctx->persist.ptr) + part);
+    g.stop = reinterpret_cast<int32_t *>(g.count + 4);
+    return g;
+}
+
+void launch_persist_kernel(Context *ctx, const void *kernel, bool cluster, int grid, int slices_per_block,
+                           size_t smem, void **args)
+{
+    if (smem > 8 * 1024)   // (with the static part above the default limit of 48 KB)
+        CF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int warps = std::max(4, std::min(kPWarps, (slices_per_block + 3) / 4 * 4));
+    if (!cluster) {
+        CF_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(32 * warps), args, smem, ctx->stream));
+        return;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = grid;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.blockDim = dim3(32 * warps);
+    cfg.gridDim = dim3(grid);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (grid > 8) CF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    CF_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
+}
 
 // `max_len`: slots per row of the longest slice.
 void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1, int max_len,
@@ -655,14 +644,7 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
 {
     PersistArgs P;
     std::memset(&P, 0, sizeof(P));
-    const size_t part = sizeof(double) * 2 * kPMaxNV * kPMaxGrid;
-    if (ctx->persist.bytes == 0) {
-        ctx->persist.ensure(part + 64);
-        CF_CUDA(cudaMemsetAsync(ctx->persist.ptr, 0, part + 64, ctx->stream));
-    }
-    P.g.part = ctx->persist.as<double>();
-    P.g.count = reinterpret_cast<uint32_t *>(static_cast<char *>(ctx->persist.ptr) + part);
-    P.g.stop = reinterpret_cast<int32_t *>(P.g.count + 4);
+    P.g = persist_grid(ctx);
     P.out = out;
     P.tolerance = S.tolerance;
     P.rel_tol = S.rel_tol;
@@ -682,7 +664,6 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
                        solver == CF_JMR;
     const bool own = solver == CF_CG || solver == CF_PCG || solver == CF_MRJACOBI || solver == CF_MRS;
     const int ns = A.n_slices;
-    auto round_up = [](int v, int m) { return (v + m - 1) / m * m; };
     // everything a block of `slices` slices keeps in shared memory, in doubles
     auto plan_all = [&](int slices) {
         PersistPlan p;
@@ -747,29 +728,9 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
     const double slots = (double)ns * 32.0 * max_len * 12.0, vectors = 40.0 * A.n;
     P.keep = slots + vectors < 0.95 * (double)ctx->l2_bytes ? 1 : 0;
     const void *kernel = persist_kernel(solver, scope, format);
-    if (smem > 8 * 1024)   // (with the static part above the default limit of 48 KB)
-        CF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int warps = std::max(4, std::min(kPWarps, round_up((ns + grid - 1) / grid, 4)));
     SolveArgs a = A;
     void *args[] = {&a, &P};
-    if (scope != kScopeCluster) {
-        CF_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(32 * warps), args, smem, ctx->stream));
-        return;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = grid;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(32 * warps);
-    cfg.gridDim = dim3(grid);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (grid > 8) CF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CF_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
+    launch_persist_kernel(ctx, kernel, scope == kScopeCluster, grid, (ns + grid - 1) / grid, smem, args);
 }
 
 // after a solve whose blocks gave up waiting: the arrival counter is not zero

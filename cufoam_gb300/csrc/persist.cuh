@@ -364,4 +364,67 @@ __device__ __forceinline__ double div_by_reciprocal(double a, double b, double r
     return __fma_rn(__fma_rn(-q, b, a), rb, q);
 }
 
+// ---------------------------------------------------------------------------
+// rows over slots in shared memory (cp, vp: this lane's first slot): the
+// chain of sell_slice_at in the same order
+// ---------------------------------------------------------------------------
+template <class V, int M, class G>
+__device__ __forceinline__ void local_batch(const int32_t *cp, const V *vp, G g, V &acc)
+{
+    V v[M], x[M];
+#pragma unroll
+    for (int u = 0; u < M; ++u) x[u] = g(cp[32 * u]);
+#pragma unroll
+    for (int u = 0; u < M; ++u) v[u] = vp[32 * u];
+#pragma unroll
+    for (int u = 0; u < M; ++u) acc = fma_t(v[u], x[u], acc);
+}
+template <class V, int B, class G>
+__device__ __forceinline__ void local_tail(int r, const int32_t *cp, const V *vp, G g, V &acc)
+{
+    if constexpr (B > 1) {
+        if (r == B - 1) {
+            local_batch<V, B - 1>(cp, vp, g, acc);
+            return;
+        }
+        local_tail<V, B - 1>(r, cp, vp, g, acc);
+    }
+}
+template <class V, int B, class G>
+__device__ __forceinline__ V local_slice(const int32_t *cp, const V *vp, int len, G g)
+{
+    V acc = V(0);
+    int t0 = 0;
+    for (; t0 + B <= len; t0 += B) local_batch<V, B>(cp + 32 * t0, vp + 32 * t0, g, acc);
+    local_tail<V, B>(len - t0, cp + 32 * t0, vp + 32 * t0, g, acc);
+    return acc;
+}
+
+// ---------------------------------------------------------------------------
+// host side, shared by the FP64 and the mixed-precision solves
+// ---------------------------------------------------------------------------
+enum { kScopeGrid = 0, kScopeGridLocal = 1, kScopeCluster = 2 };
+
+// Dynamic shared memory of a block: at most this much in all, and at most
+// CF_PERSIST_VEC_BYTES for vectors alone when the matrix streams from L2 or
+// HBM (the rest of the SM's 256 KB is the L1 of the gathers).
+#ifndef CF_PERSIST_LOCAL_BYTES
+#define CF_PERSIST_LOCAL_BYTES (200 * 1024)
+#endif
+#ifndef CF_PERSIST_VEC_BYTES
+#define CF_PERSIST_VEC_BYTES (144 * 1024)
+#endif
+// Systems up to this many rows run in one cluster of up to 16 blocks: CG step
+// 5.4 us against 8.1 on the grid at 4,096 rows, 6.7 against 8.1 at 8,100, 8.6
+// against 8.3 at 12,100.
+#ifndef CF_PERSIST_CLUSTER_ROWS
+#define CF_PERSIST_CLUSTER_ROWS 10240
+#endif
+
+// the barrier counter and partial sums of the context
+PersistGrid persist_grid(Context *ctx);
+// `grid` blocks, one warp per slice up to 32, cooperative or as one cluster
+void launch_persist_kernel(Context *ctx, const void *kernel, bool cluster, int grid, int slices_per_block,
+                           size_t smem, void **args);
+
 } // namespace cf

@@ -751,7 +751,7 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     const Kernels kk = ref ? body_kernels(solver, sell) : fast_body_kernels(solver, fmt);
     SolveArgs *d_args = ctx->args.as<SolveArgs>();
     // the fast order over the SELL-32 copy: one launch
-    const bool persist = use_graph && !ref && !mixed && persist_usable(ctx, solver, fmt);
+    const bool persist = use_graph && !ref && persist_usable(ctx, solver, fmt, mixed);
     if (use_graph && !mixed && !persist) {
         try {
             ge = loop_graph(ctx, kk, solver, CF_PREC_FP64, cap, ref, d_args, fmt);
@@ -770,7 +770,10 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     MixedResult mres;
     if (persist) {
         CF_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
-        launch_persist(ctx, solver, fmt, A, S, l1, m->sell_max_len, ctx->h_state);
+        if (mixed)
+            launch_persist_mixed(ctx, solver, fmt, A, S, l1, m->sell_max_len, c, ctx->h_state, ctx->h_state_in);
+        else
+            launch_persist(ctx, solver, fmt, A, S, l1, m->sell_max_len, ctx->h_state);
         CF_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
     } else {
     CF_CUDA(cudaMemcpyAsync(d_args, &A, sizeof(SolveArgs), cudaMemcpyHostToDevice, ctx->stream));
@@ -896,6 +899,11 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     CF_CUDA(cudaStreamSynchronize(ctx->stream));
     const DevState R = *ctx->h_state;
     if (persist && R.flags) persist_reset(ctx);
+    if (persist && mixed) {
+        mres.inner_iterations = ctx->h_state_in->k;
+        mres.outer = R.k;
+        mres.status = R.status;
+    }
     if (c.memory == CF_MEM_HOST) {
         download(ctx, x_io, x, sizeof(double) * n, CF_MEM_HOST);
     }
