@@ -52,11 +52,20 @@ void DeviceBuffer::ensure(size_t nbytes)
     bytes = nbytes;
 }
 
+void DeviceBuffer::borrow(void *p, size_t nbytes)
+{
+    release();
+    ptr = p;
+    bytes = nbytes;
+    borrowed = true;
+}
+
 void DeviceBuffer::release()
 {
-    if (ptr) cudaFree(ptr);
+    if (ptr && !borrowed) cudaFree(ptr);
     ptr = nullptr;
     bytes = 0;
+    borrowed = false;
 }
 
 int Context::fast_grid(const void *kernel, size_t dyn_smem) const

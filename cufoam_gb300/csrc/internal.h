@@ -143,7 +143,9 @@ struct SolveArgs {
 struct DeviceBuffer {
     void *ptr = nullptr;
     size_t bytes = 0;
+    bool borrowed = false;        // part of another buffer's allocation
     void ensure(size_t nbytes);   // grow-only
+    void borrow(void *p, size_t nbytes);
     void release();
     ~DeviceBuffer() { release(); }
     template <class T> T *as() const { return static_cast<T *>(ptr); }
@@ -199,8 +201,7 @@ struct Context {
 
     // scratch of the matrix builds (grow-only: a conversion after the first
     // allocates nothing) and the matrix of one-shot ldu2csr conversions
-    DeviceBuffer scratch_flag, scratch_tmp, scratch_cnt, scratch_stats;
-    DeviceBuffer scratch_codes;   // offset set of the one-byte column codes, largest |offset| (matrix.cu)
+    DeviceBuffer scratch_tmp, scratch_cnt, scratch_stats;
     struct Matrix *ldu_scratch = nullptr;
 
     int fast_grid(const void *kernel, size_t dyn_smem) const;
@@ -257,6 +258,10 @@ struct Matrix {
     int32_t n_slices = 0;
     int64_t sell_nnz = 0;      // stored entries including padding
     int32_t sell_max_len = 0;  // slots per row of the longest slice
+    int32_t max_offset = 0;    // largest |col - row|
+    std::vector<int32_t> offsets; // the distinct offsets col - row, ascending (empty: too many for codes)
+    bool slices_scanned = false;  // s_off holds offsets (else the slices' lengths)
+    DeviceBuffer arena, sell_arena; // the allocations the pattern's and the copy's buffers are parts of
     DeviceBuffer s_off, s_col, s_val, s_valT, s_val32, s_valT32;
     // one-byte column codes of the SELL-32 slots and the table of offsets
     // col - row they index (n_codes distinct offsets; 0: 32-bit columns only)

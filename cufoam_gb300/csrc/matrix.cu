@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 
 namespace cf {
 
@@ -18,13 +19,19 @@ namespace cf {
 // ---------------------------------------------------------------------------
 enum AddrError { ADDR_RANGE = 1, ADDR_ORDER = 2, ADDR_START = 4, ADDR_COUNT = 8 };
 
+// also counts every cell's neighbour faces (cnt, unless the caller gave the
+// losort arrays); the kernels after it return at once when *err is set
 __global__ void k_check_faces(int n, int nf, const int32_t *__restrict__ la,
-                              const int32_t *__restrict__ ua, int *err)
+                              const int32_t *__restrict__ ua, int32_t *cnt, int *err)
 {
     CF_FOR_ELEMS(f, nf) {
         const int o = la[f], u = ua[f];
-        if (o < 0 || o >= n || u < 0 || u >= n) atomicOr(err, ADDR_RANGE);
-        else if (u <= o) atomicOr(err, ADDR_ORDER);
+        if (o < 0 || o >= n || u < 0 || u >= n) {
+            atomicOr(err, ADDR_RANGE);
+        } else {
+            if (u <= o) atomicOr(err, ADDR_ORDER);
+            if (cnt) atomicAdd(cnt + u, 1);
+        }
         if (f > 0 && la[f - 1] > o) atomicOr(err, ADDR_ORDER);
     }
 }
@@ -40,6 +47,8 @@ __global__ void k_check_given(int n, int nf, const int32_t *__restrict__ losort,
     CF_FOR_ELEMS(c, n + 1) {
         if (ls[c] < 0 || ls[c] > nf || os[c] < 0 || os[c] > nf) atomicOr(err, ADDR_START);
         if (c < n && (ls[c + 1] < ls[c] || os[c + 1] < os[c])) atomicOr(err, ADDR_START);
+        // the counts must describe exactly n + 2F entries
+        if (c == n && (int64_t)ls[n] - ls[0] + os[n] - os[0] != 2 * (int64_t)nf) atomicOr(err, ADDR_COUNT);
     }
 }
 
@@ -55,11 +64,6 @@ __global__ void k_owner_start(int n, int nf, const int32_t *__restrict__ la, int
         }
         os[c] = lo;
     }
-}
-
-__global__ void k_count_neighbours(int nf, const int32_t *__restrict__ ua, int32_t *cnt)
-{
-    CF_FOR_ELEMS(f, nf) atomicAdd(cnt + ua[f], 1);
 }
 
 // Exclusive scan of m int32 values, three kernels: per-block inclusive scan
@@ -127,8 +131,9 @@ __global__ void k_scan_add(int m, int32_t *out, const int32_t *__restrict__ sums
 // the segment), then sort each segment by face index: the result is the
 // stable order of OpenFOAM's losort.
 __global__ void k_losort_place(int nf, const int32_t *__restrict__ ua,
-                               const int32_t *__restrict__ ls, int32_t *cursor, int32_t *losort)
+                               const int32_t *__restrict__ ls, int32_t *cursor, int32_t *losort, const int *err)
 {
+    if (*err) return;
     CF_FOR_ELEMS(f, nf) {
         const int u = ua[f];
         const int pos = ls[u] + atomicAdd(cursor + u, 1);
@@ -136,8 +141,9 @@ __global__ void k_losort_place(int nf, const int32_t *__restrict__ ua,
     }
 }
 
-__global__ void k_losort_sort(int n, const int32_t *__restrict__ ls, int32_t *losort)
+__global__ void k_losort_sort(int n, const int32_t *__restrict__ ls, int32_t *losort, const int *err)
 {
+    if (*err) return;
     CF_FOR_ELEMS(c, n) {
         const int b = ls[c], e = ls[c + 1];
         for (int i = b + 1; i < e; ++i) {
@@ -152,62 +158,46 @@ __global__ void k_losort_sort(int n, const int32_t *__restrict__ ls, int32_t *lo
     }
 }
 
-__global__ void k_row_offsets(int n, const int32_t *__restrict__ ls, const int32_t *__restrict__ os,
-                              int32_t *ro)
-{
-    const int l0 = ls[0], o0 = os[0];
-    CF_FOR_ELEMS(c, n + 1) ro[c] = (ls[c] - l0) + c + (os[c] - o0);
-}
-
-// One thread per cell, in the reference's entry order.  `col` may be null
-// (value-only refresh); `lower`/`upper` swapped gives A^T on the same
-// pattern (faces are structurally symmetric).
+// One thread per cell, in the reference's entry order; the row starts at
+// (ls[c] - ls[0]) + c + (os[c] - os[0]).  ro and col may be null (a refresh of
+// the values), dinv too (no diagonal-derived vectors: FindDiagInv and
+// FindDiagInvSqrt, gis/SparseSystem/kernels.h:563-603); `lower`/`upper` swapped
+// gives A^T on the same pattern (faces are structurally symmetric).
 __global__ void k_fill_csr(int n, const int32_t *__restrict__ ls, const int32_t *__restrict__ os,
                            const int32_t *__restrict__ losort, const int32_t *__restrict__ la,
                            const int32_t *__restrict__ ua, const double *__restrict__ diag,
-                           const double *__restrict__ lower, const double *__restrict__ upper,
-                           const int32_t *__restrict__ ro, int32_t *col, double *val)
+                           const double *__restrict__ lower, const double *__restrict__ upper, int32_t *ro,
+                           int32_t *col, double *val, double *dinv, double *dinv_sqrt, const int *err)
 {
-    CF_FOR_ELEMS(c, n) {
-        int e = ro[c];
-        for (int idx = ls[c]; idx < ls[c + 1]; ++idx) {
+    if (err && *err) return;
+    const int l0 = ls[0], o0 = os[0];
+    CF_FOR_ELEMS(c, n + 1) {
+        const int lb = ls[c], ob = os[c];
+        int e = (lb - l0) + c + (ob - o0);
+        if (ro) ro[c] = e;
+        if (c == n) break;
+        const int le = ls[c + 1], oe = os[c + 1];
+        for (int idx = lb; idx < le; ++idx) {
             const int face = losort[idx];
             if (col) col[e] = la[face];
             val[e] = lower[face];
             ++e;
         }
+        const double d = diag[c];
         if (col) col[e] = c;
-        val[e] = diag[c];
+        val[e] = d;
         ++e;
-        for (int face = os[c]; face < os[c + 1]; ++face) {
+        for (int face = ob; face < oe; ++face) {
             if (col) col[e] = ua[face];
             val[e] = upper[face];
             ++e;
         }
-    }
-}
-
-// out[0]: max nnz over the 32-row chunks without a row longer than
-// kLongRow (the staging capacity the fast CSR passes need); out[1]: 1 if
-// some row is longer (those chunks are read unstaged, long rows by the
-// whole warp)
-__global__ void k_chunk_stats(int n, const int32_t *__restrict__ ro, int *out)
-{
-    int m = 0, lng = 0;
-    for (int base = (blockIdx.x * blockDim.x + threadIdx.x) * 32; base < n;
-         base += gridDim.x * blockDim.x * 32) {
-        const int top = base + 32 < n ? base + 32 : n;
-        bool has = false;
-        for (int r = base; r < top; ++r) has = has || (ro[r + 1] - ro[r] > kLongRow);
-        if (has) {
-            lng = 1;
-        } else {
-            const int c = ro[top] - ro[base];
-            m = c > m ? c : m;
+        if (dinv) {
+            const double inv = 1.0 / d;
+            dinv[c] = inv;
+            dinv_sqrt[c] = sqrt(inv);
         }
     }
-    atomicMax(out, m);
-    if (lng) atomicMax(out + 1, 1);
 }
 
 __global__ void k_diag_derived(int n, const double *__restrict__ diag, double *dinv,
@@ -302,30 +292,10 @@ __global__ void __launch_bounds__(kBlock) k_spmv_sell_ref(int n, int n_slices, c
 // ---------------------------------------------------------------------------
 // SELL-32 copy (layout described in device.cuh)
 // ---------------------------------------------------------------------------
-// slot s: 32 x the longest row of slice s (slot n_slices = 0); the stored
-// total accumulates in 64 bits in total[0], the longest row in total[1]
-__global__ void k_sell_len(int n, int n_slices, const int32_t *__restrict__ ro, int32_t *slen,
-                           unsigned long long *total)
-{
-    CF_FOR_ELEMS(s, n_slices + 1) {
-        int mx = 0;
-        if (s < n_slices) {
-            const int r1 = min(n, 32 * s + 32);
-            for (int r = 32 * s; r < r1; ++r) mx = max(mx, __ldg(ro + r + 1) - __ldg(ro + r));
-            atomicAdd(total, 32ull * (unsigned long long)mx);
-            if ((unsigned long long)mx > *(volatile unsigned long long *)(total + 1))
-                atomicMax(total + 1, (unsigned long long)mx);
-        }
-        slen[s] = 32 * mx;
-    }
-}
-
-// one thread per slot of the last slice's 32 rows (rows >= n hold value 0,
-// column 0); pattern (scol != nullptr) and / or values
+// values of the SELL-32 slots, one thread per row of a slice (padding: 0)
 template <class S, class V>
-__global__ void k_sell_fill(int n, int n_slices, const int32_t *__restrict__ ro,
-                            const int32_t *__restrict__ col, const S *__restrict__ val,
-                            const int32_t *__restrict__ soff, int32_t *scol, V *sval)
+__global__ void k_sell_fill(int n, int n_slices, const int32_t *__restrict__ ro, const S *__restrict__ val,
+                            const int32_t *__restrict__ soff, V *sval)
 {
     CF_FOR_ELEMS(i, 32 * n_slices) {
         const int s = i >> 5, lane = i & 31;
@@ -333,33 +303,41 @@ __global__ void k_sell_fill(int n, int n_slices, const int32_t *__restrict__ ro,
         const int rs = i < n ? ro[i] : 0, re = i < n ? ro[i + 1] : 0;
         for (int t = 0; t < len; ++t) {
             const int j = rs + t;
-            const int o = b + 32 * t + lane;
-            if (scol) scol[o] = j < re ? col[j] : (i < n ? i : 0);
-            if (sval) sval[o] = j < re ? (V)val[j] : V(0);
+            sval[b + 32 * t + lane] = j < re ? (V)val[j] : V(0);
         }
     }
 }
 
-// One-byte column codes of the SELL-32 slots (SellCodes8, device.cuh): the
-// distinct offsets d = col - row of the CSR entries, and 0 (the padding
-// slots' offset), go into an open-addressing set on the device while the
-// SELL-32 layout is sized; when there are at most kMaxCodes of them the host
-// numbers them in ascending order and a pass over the slots writes each
-// slot's number.
-constexpr int kCodeHash = 1024;              // slots of the set (power of two, > 2 kMaxCodes)
+// What the formats and the kernels' schedules need to know of a pattern,
+// found in one pass and read back in one copy.
+constexpr int kCodeHash = 1024;              // slots of the offset set (power of two, > 2 kMaxCodes)
 constexpr int kCodeTable = kMaxCodes;        // entries of the offset table (unused ones 0)
-constexpr int32_t kNoOffset = INT32_MIN;     // empty slot (|d| < n < 2^31)
+constexpr int kBlockHash = 128;              // slots of a block's own offset set
+// empty slot: every byte 0x80; no offset is that negative (n + 2 F < 2^31)
+constexpr int32_t kNoOffset = (int32_t)0x80808080u;
+
+struct PatternStats {
+    unsigned long long sell_total;  // SELL-32 entries with padding
+    int32_t max_len;                // longest row
+    int32_t max_chunk;              // max nnz over the 32-row chunks without a row longer than kLongRow
+    int32_t has_long;               // some row is longer (those chunks are read unstaged)
+    int32_t maxoff;                 // largest |col - row| (the 16-bit deltas' range)
+    int32_t count;                  // distinct offsets col - row, 0 included (> kMaxCodes: too many)
+    int32_t err;                    // AddrError bits of the build, or the CSR check's
+    int32_t keys[kCodeHash];        // the offset set
+};
 
 __device__ __forceinline__ uint32_t offset_hash(int32_t d) { return ((uint32_t)d * 2654435761u) >> 22; }
 
-// d into the set.  With at most kMaxCodes keys no probe sequence meets more
-// than kMaxCodes occupied slots, so one that meets more proves an overflow:
-// it marks the count past the limit (every thread then stops) instead of
+// d into a set of SLOTS slots (a power of two).  With at most kMaxCodes keys
+// no probe sequence meets more than kMaxCodes occupied slots, so one that
+// meets more proves an overflow: it marks the count past the limit instead of
 // walking a table that thousands of offsets filled.
+template <int SLOTS>
 __device__ void offset_insert(int32_t *keys, int32_t *count, int32_t d)
 {
-    uint32_t h = offset_hash(d);
-    for (int probe = 0; probe <= kMaxCodes + 1; ++probe, h = (h + 1) & (kCodeHash - 1)) {
+    uint32_t h = offset_hash(d) & (SLOTS - 1);
+    for (int probe = 0; probe <= kMaxCodes + 1; ++probe, h = (h + 1) & (SLOTS - 1)) {
         const int32_t k = *(volatile int32_t *)(keys + h);
         if (k == d) return;
         if (k == kNoOffset) {
@@ -374,87 +352,116 @@ __device__ void offset_insert(int32_t *keys, int32_t *count, int32_t d)
     atomicMax(count, kMaxCodes + 1);
 }
 
-// keys = empty, count = 0, largest |offset| = 0
-__global__ void k_offsets_clear(int32_t *keys, int32_t *count)
+// One thread per row, a warp per slice of 32 rows (grid-stride): slice lengths
+// (slen[s] = 32 x its longest row, slen[n_slices] = 0), the row statistics and
+// the offset set.  A thread remembers the last eight offsets it inserted, a
+// block collects its offsets in shared memory and adds them to the global set
+// once: one insertion per entry into the global set's hot lines took 59 us at
+// 219k rows (7-point) beside four passes for the other statistics; this pass
+// takes 18 us at 178k to 517k rows.  A block stops collecting once it has
+// more than kMaxCodes.
+__global__ void __launch_bounds__(kBlock) k_row_stats(int n, int n_slices, const int32_t *__restrict__ ro,
+                                                      const int32_t *__restrict__ col, int32_t *slen,
+                                                      PatternStats *st, const int *err)
 {
-    CF_FOR_ELEMS(i, kCodeHash) keys[i] = kNoOffset;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        count[0] = 0;
-        count[1] = 0;
-    }
-}
-
-// the largest |col - row| over the CSR entries (the 16-bit deltas' range)
-__global__ void k_csr_maxoff(int n, const int32_t *__restrict__ ro, const int32_t *__restrict__ col, int32_t *maxoff)
-{
-    int m = 0;
-    CF_FOR_ELEMS(i, n) {
-        const int re = ro[i + 1];
-        for (int j = ro[i]; j < re; ++j) m = max(m, abs(col[j] - i));
-    }
+    __shared__ int32_t keys[kBlockHash];
+    __shared__ int32_t count;
+    if (err && *err) return;
+    for (int i = threadIdx.x; i < kBlockHash; i += kBlock) keys[i] = kNoOffset;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    if (threadIdx.x == 0) offset_insert<kBlockHash>(keys, &count, 0);   // the padding slots' offset
+    if (blockIdx.x == 0 && threadIdx.x == 0) slen[n_slices] = 0;
+    const int lane = threadIdx.x & 31;
+    unsigned long long total = 0;
+    int mlen = 0, mchunk = 0, lng = 0, moff = 0;
+    int32_t c[8];
 #pragma unroll
-    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(kFull, m, o));
-    if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(maxoff, m);
-}
-
-// the 16-bit delta of every slot, lane-major within the slice like the codes
-__global__ void k_sell_encode16(int n, int n_slices, const int32_t *__restrict__ soff,
-                                const int32_t *__restrict__ scol, int16_t *d16)
-{
-    CF_FOR_ELEMS(i, 32 * n_slices) {
-        const int s = i >> 5, lane = i & 31;
-        const int b = soff[s], len = (soff[s + 1] - b) >> 5;
-        const int rb = sell_row_base(i, n);
-        for (int t = 0; t < len; ++t) d16[b + len * lane + t] = (int16_t)(scol[b + 32 * t + lane] - rb);
-    }
-}
-
-// every CSR entry's offset, and 0; stops early once more than kMaxCodes
-// distinct offsets are in the set (the codes cannot be used then).  Each
-// thread remembers the last eight offsets it inserted in registers, so a
-// stencil's few offsets reach the set (and its hot cache lines) once per
-// thread, not once per entry.
-__global__ void k_csr_offsets(int n, const int32_t *__restrict__ ro, const int32_t *__restrict__ col,
-                              int32_t *keys, int32_t *count)
-{
-    if (blockIdx.x == 0 && threadIdx.x == 0) offset_insert(keys, count, 0);
-    int32_t s0 = kNoOffset, s1 = kNoOffset, s2 = kNoOffset, s3 = kNoOffset;
-    int32_t s4 = kNoOffset, s5 = kNoOffset, s6 = kNoOffset, s7 = kNoOffset;
-    CF_FOR_ELEMS(i, n) {
-        const int re = ro[i + 1];
-        for (int j = ro[i]; j < re; ++j) {
+    for (int u = 0; u < 8; ++u) c[u] = kNoOffset;
+    for (int s = blockIdx.x * kWarps + (threadIdx.x >> 5); s < n_slices; s += gridDim.x * kWarps) {
+        const int i = 32 * s + lane;
+        const int rb = i < n ? ro[i] : 0, re = i < n ? ro[i + 1] : 0, len = re - rb;
+        const int mx = __reduce_max_sync(kFull, len);
+        const int sum = __reduce_add_sync(kFull, len);
+        if (lane == 0) {
+            slen[s] = 32 * mx;
+            total += 32ull * (unsigned long long)mx;
+            mlen = max(mlen, mx);
+            if (mx > kLongRow) lng = 1;
+            else mchunk = max(mchunk, sum);
+        }
+        const bool collect = *(volatile int32_t *)&count <= kMaxCodes;
+        for (int j = rb; j < re; ++j) {
             const int32_t d = col[j] - i;
-            if (d == s0 || d == s1 || d == s2 || d == s3 || d == s4 || d == s5 || d == s6 || d == s7) continue;
-            if (*(volatile int32_t *)count > kMaxCodes) return;
-            offset_insert(keys, count, d);
-            s7 = s6;
-            s6 = s5;
-            s5 = s4;
-            s4 = s3;
-            s3 = s2;
-            s2 = s1;
-            s1 = s0;
-            s0 = d;
+            moff = max(moff, abs(d));
+            if (!collect || d == c[0] || d == c[1] || d == c[2] || d == c[3] || d == c[4] || d == c[5] || d == c[6] ||
+                d == c[7])
+                continue;
+            if (*(volatile int32_t *)&count > kMaxCodes) continue;
+            offset_insert<kBlockHash>(keys, &count, d);
+#pragma unroll
+            for (int u = 7; u > 0; --u) c[u] = c[u - 1];
+            c[0] = d;
         }
     }
+    moff = __reduce_max_sync(kFull, moff);
+    if (lane == 0) {
+        if (total) atomicAdd(&st->sell_total, total);
+        if (mlen > 0) atomicMax(&st->max_len, mlen);
+        if (mchunk > 0) atomicMax(&st->max_chunk, mchunk);
+        if (lng) atomicMax(&st->has_long, 1);
+        if (moff > 0) atomicMax(&st->maxoff, moff);
+    }
+    __syncthreads();
+    if (count > kMaxCodes) {
+        if (threadIdx.x == 0) atomicMax(&st->count, kMaxCodes + 1);
+    } else {
+        for (int i = threadIdx.x; i < kBlockHash; i += kBlock)
+            if (keys[i] != kNoOffset && *(volatile int32_t *)&st->count <= kMaxCodes)
+                offset_insert<kCodeHash>(st->keys, &st->count, keys[i]);
+    }
 }
 
-// each slot's code: the number of its offset (slot_code, by set position);
-// every offset is in the set, found within kCodeHash probes.  A slice's
-// codes are stored lane-major: lane l's len codes at b + len l.
-__global__ void k_sell_encode(int n, int n_slices, const int32_t *__restrict__ soff,
-                              const int32_t *__restrict__ scol, const int32_t *__restrict__ keys,
-                              const uint8_t *__restrict__ slot_code, uint8_t *code)
+// The SELL-32 copy in one pass, a thread per row of a slice (rows >= n hold
+// value 0, column 0): columns, values, and (COMPACT 1) one-byte codes -- the
+// number of the slot's offset col - row in the ascending table tab of ncodes
+// offsets -- or (COMPACT 2) 16-bit deltas, both stored lane-major within the
+// slice (lane l's len codes at b + len l).
+template <int COMPACT>
+__global__ void __launch_bounds__(kBlock) k_sell_build(int n, int n_slices, const int32_t *__restrict__ ro,
+                                                       const int32_t *__restrict__ col,
+                                                       const double *__restrict__ val,
+                                                       const int32_t *__restrict__ soff, int32_t *scol, double *sval,
+                                                       const int32_t *__restrict__ tab, int ncodes, uint8_t *code,
+                                                       int16_t *d16)
 {
+    __shared__ int32_t stab[kMaxCodes];
+    if (COMPACT == 1) {
+        if (threadIdx.x < kMaxCodes) stab[threadIdx.x] = tab[threadIdx.x];
+        __syncthreads();
+    }
     CF_FOR_ELEMS(i, 32 * n_slices) {
         const int s = i >> 5, lane = i & 31;
         const int b = soff[s], len = (soff[s + 1] - b) >> 5;
         const int rb = sell_row_base(i, n);
+        const int rs = i < n ? ro[i] : 0, re = i < n ? ro[i + 1] : 0;
         for (int t = 0; t < len; ++t) {
-            const int32_t d = scol[b + 32 * t + lane] - rb;
-            uint32_t h = offset_hash(d);
-            for (int probe = 0; probe < kCodeHash && keys[h] != d; ++probe) h = (h + 1) & (kCodeHash - 1);
-            code[b + len * lane + t] = slot_code[h];   // lane-major within the slice
+            const int j = rs + t;
+            const int o = b + 32 * t + lane;
+            const int c = j < re ? col[j] : rb;
+            scol[o] = c;
+            sval[o] = j < re ? val[j] : 0.0;
+            if (COMPACT == 1) {
+                const int32_t d = c - rb;
+                int lo = 0, hi = ncodes - 1;   // d is in the table
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (stab[mid] < d) lo = mid + 1;
+                    else hi = mid;
+                }
+                code[b + len * lane + t] = (uint8_t)lo;
+            }
+            if (COMPACT == 2) d16[b + len * lane + t] = (int16_t)(c - rb);
         }
     }
 }
@@ -505,8 +512,9 @@ __launch_bounds__(kBlock, COLS ? CF_PLAIN_SPMV8_MINB : (CF_PLAIN_SPMV_MINB > 0 ?
 // FindDiag (gis/SparseSystem/kernels.h:447-464): the entry with col == row,
 // scanning the row while col <= row; rows without one read as 0.
 __global__ void k_csr_diag(int n, const int32_t *__restrict__ ro, const int32_t *__restrict__ col,
-                           const double *__restrict__ val, double *diag)
+                           const double *__restrict__ val, double *diag, const int *err)
 {
+    if (err && *err) return;
     CF_FOR_ELEMS(i, n) {
         double d = 0.0;
         for (int j = ro[i]; j < ro[i + 1] && col[j] <= i; ++j)
@@ -520,7 +528,7 @@ __global__ void k_csr_check(int n, int n_cols, const int32_t *__restrict__ ro,
 {
     CF_FOR_ELEMS(i, n) {
         const int b = ro[i], e = ro[i + 1];
-        if (b < 0 || e < b || (int64_t)e > nnz) atomicOr(err, 1);
+        if (b < 0 || e < b || (int64_t)e > nnz || (i == n - 1 && (int64_t)e != nnz)) atomicOr(err, 1);
         else
             for (int j = b; j < e; ++j)
                 if (col[j] < 0 || col[j] >= n_cols) atomicOr(err, 2);
@@ -615,70 +623,6 @@ static int grid_for(Context *ctx, int64_t work, int per_block = kBlock)
     return (int)g;
 }
 
-// The offset set of m's pattern (one-byte column codes) and its largest
-// |offset| (16-bit deltas) into the context's scratch: keys [kCodeHash],
-// count, largest |offset|, then the slot -> code map [kCodeHash] bytes.
-// Enqueued only; read back with the SELL-32 size.
-static void queue_offsets(Matrix *m)
-{
-    Context *ctx = m->ctx;
-    ctx->scratch_codes.ensure(sizeof(int32_t) * (kCodeHash + 4) + kCodeHash);
-    int32_t *keys = ctx->scratch_codes.as<int32_t>();
-    k_offsets_clear<<<grid_for(ctx, kCodeHash), kBlock, 0, ctx->stream>>>(keys, keys + kCodeHash);
-    CF_CHECK_LAUNCH();
-    k_csr_offsets<<<grid_for(ctx, m->n), kBlock, 0, ctx->stream>>>(m->n, m->ro.as<int32_t>(), m->col.as<int32_t>(),
-                                                                  keys, keys + kCodeHash);
-    CF_CHECK_LAUNCH();
-    k_csr_maxoff<<<grid_for(ctx, m->n), kBlock, 0, ctx->stream>>>(m->n, m->ro.as<int32_t>(), m->col.as<int32_t>(),
-                                                                 keys + kCodeHash + 1);
-    CF_CHECK_LAUNCH();
-}
-
-// The 16-bit column deltas of m's SELL-32 copy (every |offset| <= 32767).
-static void build_sell_d16(Matrix *m)
-{
-    Context *ctx = m->ctx;
-    m->s_d16.ensure(sizeof(int16_t) * ((size_t)m->sell_nnz + 32));
-    k_sell_encode16<<<grid_for(ctx, 32 * (int64_t)m->n_slices), kBlock, 0, ctx->stream>>>(
-        m->n, m->n_slices, m->s_off.as<int32_t>(), m->s_col.as<int32_t>(), m->s_d16.as<int16_t>());
-    CF_CHECK_LAUNCH();
-    m->has_d16 = true;
-}
-
-// The codes of m's SELL-32 copy from the offset set read back into hk /
-// count, when the pattern has at most kMaxCodes distinct offsets (m->n_codes
-// > 0 then).  Asynchronous: the host tables are staged by the copies.
-static void build_sell_codes(Matrix *m, const std::vector<int32_t> &hk, int32_t count)
-{
-    Context *ctx = m->ctx;
-    m->n_codes = 0;
-    if (count <= 0 || count > kMaxCodes) return;
-    std::vector<int32_t> offs;
-    for (int32_t k : hk)
-        if (k != kNoOffset) offs.push_back(k);
-    if ((int)offs.size() != count) return;
-    std::sort(offs.begin(), offs.end());
-    std::vector<int32_t> tab(kCodeTable, 0);
-    std::copy(offs.begin(), offs.end(), tab.begin());
-    std::vector<uint8_t> slot_code(kCodeHash, 0);
-    for (int h = 0; h < kCodeHash; ++h)
-        if (hk[h] != kNoOffset)
-            slot_code[h] = (uint8_t)(std::lower_bound(offs.begin(), offs.end(), hk[h]) - offs.begin());
-    int32_t *keys = ctx->scratch_codes.as<int32_t>();
-    uint8_t *map = reinterpret_cast<uint8_t *>(keys + kCodeHash + 4);
-    m->s_dtab.ensure(sizeof(int32_t) * kCodeTable);
-    m->s_code.ensure((size_t)m->sell_nnz + 64);
-    // pageable sources: each copy returns once its bytes are staged
-    CF_CUDA(cudaMemcpyAsync(m->s_dtab.ptr, tab.data(), sizeof(int32_t) * kCodeTable, cudaMemcpyHostToDevice,
-                            ctx->stream));
-    CF_CUDA(cudaMemcpyAsync(map, slot_code.data(), kCodeHash, cudaMemcpyHostToDevice, ctx->stream));
-    const int ns = m->n_slices;
-    k_sell_encode<<<grid_for(ctx, 32 * (int64_t)ns), kBlock, 0, ctx->stream>>>(
-        m->n, ns, m->s_off.as<int32_t>(), m->s_col.as<int32_t>(), keys, map, m->s_code.as<uint8_t>());
-    CF_CHECK_LAUNCH();
-    m->n_codes = count;
-}
-
 static void exclusive_scan(Context *ctx, int m, const int32_t *in, int32_t *out, DeviceBuffer &tmp)
 {
     const int nb = (m + kScanBlock - 1) / kScanBlock;
@@ -699,22 +643,66 @@ static int read_flag(Context *ctx, const int *d_flag)
     return h;
 }
 
-// chunk statistics of m's CSR pattern into m->max_chunk / m->has_long
-static void chunk_stats(Context *ctx, Matrix *m)
-{
-    DeviceBuffer &buf = ctx->scratch_stats;
-    buf.ensure(2 * sizeof(int));
-    CF_CUDA(cudaMemsetAsync(buf.ptr, 0, 2 * sizeof(int), ctx->stream));
-    if (m->n > 0) {
-        k_chunk_stats<<<grid_for(ctx, ((int64_t)m->n + 31) / 32), kBlock, 0, ctx->stream>>>(
-            m->n, m->ro.as<int32_t>(), buf.as<int>());
-        CF_CHECK_LAUNCH();
+// Several buffers carved out of one allocation (a device allocation and its
+// release take about 60 us together, whatever their size).
+struct Carve {
+    std::vector<std::pair<DeviceBuffer *, size_t>> parts;
+    void add(DeviceBuffer &b, size_t bytes) { parts.emplace_back(&b, bytes); }
+    void commit(DeviceBuffer &arena) const
+    {
+        size_t total = 0;
+        for (const auto &p : parts) total += (p.second + 255) / 256 * 256;
+        arena.ensure(total);
+        size_t at = 0;
+        for (const auto &p : parts) {
+            p.first->borrow(arena.as<char>() + at, p.second);
+            at += (p.second + 255) / 256 * 256;
+        }
     }
-    int h[2] = {0, 0};
-    CF_CUDA(cudaMemcpyAsync(h, buf.ptr, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+};
+
+// the context's pattern statistics, cleared (enqueued)
+static PatternStats *clear_stats(Context *ctx)
+{
+    ctx->scratch_stats.ensure(sizeof(PatternStats));
+    PatternStats *st = ctx->scratch_stats.as<PatternStats>();
+    CF_CUDA(cudaMemsetAsync(st, 0, offsetof(PatternStats, keys), ctx->stream));
+    CF_CUDA(cudaMemsetAsync(st->keys, 0x80, sizeof(int32_t) * kCodeHash, ctx->stream));
+    return st;
+}
+
+// statistics of m's pattern and the lengths of its slices (into s_off, turned
+// into offsets when the SELL-32 copy is made); enqueued
+static void queue_row_stats(Context *ctx, Matrix *m, PatternStats *st)
+{
+    const int ns = (m->n + 31) / 32;
+    const int g = std::min(ctx->sm_count * 4, (ns + kWarps - 1) / kWarps);
+    k_row_stats<<<g, kBlock, 0, ctx->stream>>>(m->n, ns, m->ro.as<int32_t>(), m->col.as<int32_t>(),
+                                               m->s_off.as<int32_t>(), st, &st->err);
+    CF_CHECK_LAUNCH();
+}
+
+// ... read back (the one synchronisation of a build); returns the error bits
+static int read_stats(Context *ctx, Matrix *m, const PatternStats *d_st)
+{
+    static_assert(sizeof(PatternStats) < 8192, "staged on the stack");
+    PatternStats h;
+    CF_CUDA(cudaMemcpyAsync(&h, d_st, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     CF_CUDA(cudaStreamSynchronize(ctx->stream));
-    m->max_chunk = h[0];
-    m->has_long = h[1] != 0;
+    m->max_chunk = h.max_chunk;
+    m->has_long = h.has_long != 0;
+    m->sell_nnz = (int64_t)h.sell_total;
+    m->sell_max_len = h.max_len;
+    m->max_offset = h.maxoff;
+    m->offsets.clear();
+    if (h.count > 0 && h.count <= kMaxCodes) {
+        for (int32_t k : h.keys)
+            if (k != kNoOffset) m->offsets.push_back(k);
+        std::sort(m->offsets.begin(), m->offsets.end());
+        if ((int)m->offsets.size() != h.count) m->offsets.clear();
+    }
+    m->slices_scanned = false;
+    return h.err;
 }
 
 // Copies the LDU arrays to `m`, validates and completes the addressing,
@@ -737,31 +725,44 @@ static void build_from_ldu(Context *ctx, Matrix *m, const cf_ldu_view &v, bool f
     m->nf = nf;
     m->nnz = (int64_t)n + 2 * (int64_t)nf;
     const size_t pad = 4;
-    m->diag.ensure(sizeof(double) * (n + pad));
-    m->lower.ensure(sizeof(double) * (nf + pad));
-    m->upper.ensure(sizeof(double) * (nf + pad));
-    m->la.ensure(sizeof(int32_t) * (nf + pad));
-    m->ua.ensure(sizeof(int32_t) * (nf + pad));
-    m->losort.ensure(sizeof(int32_t) * (nf + pad));
-    m->lstart.ensure(sizeof(int32_t) * (n + 1 + pad));
-    m->ostart.ensure(sizeof(int32_t) * (n + 1 + pad));
+    const int ns = (n + 31) / 32;
+    Carve parts;
+    parts.add(m->diag, sizeof(double) * (n + pad));
+    parts.add(m->lower, sizeof(double) * (nf + pad));
+    parts.add(m->upper, sizeof(double) * (nf + pad));
+    parts.add(m->la, sizeof(int32_t) * (nf + pad));
+    parts.add(m->ua, sizeof(int32_t) * (nf + pad));
+    parts.add(m->losort, sizeof(int32_t) * (nf + pad));
+    parts.add(m->lstart, sizeof(int32_t) * (n + 1 + pad));
+    parts.add(m->ostart, sizeof(int32_t) * (n + 1 + pad));
+    parts.add(m->ro, sizeof(int32_t) * (n + 1 + pad));
+    parts.add(m->col, sizeof(int32_t) * (m->nnz + pad));
+    parts.add(m->val, sizeof(double) * (m->nnz + pad));
+    if (full) {
+        parts.add(m->dinv, sizeof(double) * (n + pad));
+        parts.add(m->dinv_sqrt, sizeof(double) * (n + pad));
+        parts.add(m->s_off, sizeof(int32_t) * ((size_t)ns + 1));
+    }
+    parts.commit(m->arena);
     upload(ctx, m->diag.ptr, v.diag, sizeof(double) * n, v.memory);
     upload(ctx, m->lower.ptr, v.lower, sizeof(double) * nf, v.memory);
     upload(ctx, m->upper.ptr, v.upper, sizeof(double) * nf, v.memory);
     upload(ctx, m->la.ptr, v.lower_addr, sizeof(int32_t) * nf, v.memory);
     upload(ctx, m->ua.ptr, v.upper_addr, sizeof(int32_t) * nf, v.memory);
 
-    DeviceBuffer &flag = ctx->scratch_flag, &tmp = ctx->scratch_tmp, &cnt = ctx->scratch_cnt;
-    flag.ensure(sizeof(int) * 4);
-    CF_CUDA(cudaMemsetAsync(flag.ptr, 0, sizeof(int) * 4, ctx->stream));
-    int *d_err = flag.as<int>();
+    DeviceBuffer &tmp = ctx->scratch_tmp, &cnt = ctx->scratch_cnt;
+    PatternStats *st = clear_stats(ctx);
+    int *d_err = &st->err;
     const int gf = grid_for(ctx, nf > 0 ? nf : 1);
     const int gc = grid_for(ctx, (int64_t)n + 1);
-    if (nf > 0) {
-        k_check_faces<<<gf, kBlock, 0, ctx->stream>>>(n, nf, m->la.as<int32_t>(), m->ua.as<int32_t>(), d_err);
-        CF_CHECK_LAUNCH();
-    }
+    // Everything is enqueued before the one synchronisation: the kernels that
+    // index with the addressing return at once when a check before them failed.
     if (given) {
+        if (nf > 0) {
+            k_check_faces<<<gf, kBlock, 0, ctx->stream>>>(n, nf, m->la.as<int32_t>(), m->ua.as<int32_t>(), nullptr,
+                                                          d_err);
+            CF_CHECK_LAUNCH();
+        }
         upload(ctx, m->losort.ptr, v.losort, sizeof(int32_t) * nf, v.memory);
         upload(ctx, m->lstart.ptr, v.losort_start, sizeof(int32_t) * (n + 1), v.memory);
         upload(ctx, m->ostart.ptr, v.owner_start, sizeof(int32_t) * (n + 1), v.memory);
@@ -769,66 +770,45 @@ static void build_from_ldu(Context *ctx, Matrix *m, const cf_ldu_view &v, bool f
                                                       m->lstart.as<int32_t>(), m->ostart.as<int32_t>(), d_err);
         CF_CHECK_LAUNCH();
     } else {
-        k_owner_start<<<gc, kBlock, 0, ctx->stream>>>(n, nf, m->la.as<int32_t>(), m->ostart.as<int32_t>());
-        CF_CHECK_LAUNCH();
-    }
-    int err = read_flag(ctx, d_err);
-    require(err == 0, CF_BAD_INPUT,
-            std::string("invalid LDU addressing:") + ((err & ADDR_RANGE) ? " index out of range" : "") +
-                ((err & ADDR_ORDER) ? " faces not sorted by owner or not upper-triangular" : "") +
-                ((err & ADDR_START) ? " bad losortStart/ownerStart" : ""));
-    if (!given) {
         cnt.ensure(sizeof(int32_t) * (size_t)(n + 1));
         CF_CUDA(cudaMemsetAsync(cnt.ptr, 0, sizeof(int32_t) * (size_t)(n + 1), ctx->stream));
         if (nf > 0) {
-            k_count_neighbours<<<gf, kBlock, 0, ctx->stream>>>(nf, m->ua.as<int32_t>(), cnt.as<int32_t>());
+            k_check_faces<<<gf, kBlock, 0, ctx->stream>>>(n, nf, m->la.as<int32_t>(), m->ua.as<int32_t>(),
+                                                          cnt.as<int32_t>(), d_err);
             CF_CHECK_LAUNCH();
         }
+        k_owner_start<<<gc, kBlock, 0, ctx->stream>>>(n, nf, m->la.as<int32_t>(), m->ostart.as<int32_t>());
+        CF_CHECK_LAUNCH();
         exclusive_scan(ctx, n + 1, cnt.as<int32_t>(), m->lstart.as<int32_t>(), tmp);
-        CF_CUDA(cudaMemsetAsync(cnt.ptr, 0, sizeof(int32_t) * (size_t)(n + 1), ctx->stream));
         if (nf > 0) {
+            CF_CUDA(cudaMemsetAsync(cnt.ptr, 0, sizeof(int32_t) * (size_t)(n + 1), ctx->stream));
             k_losort_place<<<gf, kBlock, 0, ctx->stream>>>(nf, m->ua.as<int32_t>(), m->lstart.as<int32_t>(),
-                                                           cnt.as<int32_t>(), m->losort.as<int32_t>());
+                                                           cnt.as<int32_t>(), m->losort.as<int32_t>(), d_err);
             CF_CHECK_LAUNCH();
-            k_losort_sort<<<gc, kBlock, 0, ctx->stream>>>(n, m->lstart.as<int32_t>(), m->losort.as<int32_t>());
+            k_losort_sort<<<gc, kBlock, 0, ctx->stream>>>(n, m->lstart.as<int32_t>(), m->losort.as<int32_t>(), d_err);
             CF_CHECK_LAUNCH();
         }
     }
-    m->ro.ensure(sizeof(int32_t) * (n + 1 + pad));
-    k_row_offsets<<<gc, kBlock, 0, ctx->stream>>>(n, m->lstart.as<int32_t>(), m->ostart.as<int32_t>(),
-                                                   m->ro.as<int32_t>());
-    CF_CHECK_LAUNCH();
-    // the counts must describe exactly n + 2F entries
-    int32_t last = 0;
-    CF_CUDA(cudaMemcpyAsync(&last, m->ro.as<int32_t>() + n, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                            ctx->stream));
-    CF_CUDA(cudaStreamSynchronize(ctx->stream));
-    require((int64_t)last == m->nnz, CF_BAD_INPUT,
-            "losortStart/ownerStart do not describe n + 2*nFaces entries");
-    m->col.ensure(sizeof(int32_t) * (m->nnz + pad));
-    m->val.ensure(sizeof(double) * (m->nnz + pad));
     // zero the padding read by 16-byte vector loads past nnz
     CF_CUDA(cudaMemsetAsync(m->col.as<int32_t>() + m->nnz, 0, sizeof(int32_t) * pad, ctx->stream));
     CF_CUDA(cudaMemsetAsync(m->val.as<double>() + m->nnz, 0, sizeof(double) * pad, ctx->stream));
-    if (n > 0) {
-        k_fill_csr<<<gc, kBlock, 0, ctx->stream>>>(n, m->lstart.as<int32_t>(), m->ostart.as<int32_t>(),
-                                                   m->losort.as<int32_t>(), m->la.as<int32_t>(),
-                                                   m->ua.as<int32_t>(), m->diag.as<double>(),
-                                                   m->lower.as<double>(), m->upper.as<double>(),
-                                                   m->ro.as<int32_t>(), m->col.as<int32_t>(),
-                                                   m->val.as<double>());
-        CF_CHECK_LAUNCH();
-    }
+    k_fill_csr<<<gc, kBlock, 0, ctx->stream>>>(n, m->lstart.as<int32_t>(), m->ostart.as<int32_t>(),
+                                               m->losort.as<int32_t>(), m->la.as<int32_t>(),
+                                               m->ua.as<int32_t>(), m->diag.as<double>(),
+                                               m->lower.as<double>(), m->upper.as<double>(),
+                                               m->ro.as<int32_t>(), m->col.as<int32_t>(), m->val.as<double>(),
+                                               full ? m->dinv.as<double>() : nullptr,
+                                               full ? m->dinv_sqrt.as<double>() : nullptr, d_err);
+    CF_CHECK_LAUNCH();
+    // staging capacity, long rows, the SELL-32 size and the offset set
+    if (full && n > 0) queue_row_stats(ctx, m, st);
+    const int err = read_stats(ctx, m, st);
+    require((err & ~ADDR_COUNT) == 0, CF_BAD_INPUT,
+            std::string("invalid LDU addressing:") + ((err & ADDR_RANGE) ? " index out of range" : "") +
+                ((err & ADDR_ORDER) ? " faces not sorted by owner or not upper-triangular" : "") +
+                ((err & ADDR_START) ? " bad losortStart/ownerStart" : ""));
+    require(err == 0, CF_BAD_INPUT, "losortStart/ownerStart do not describe n + 2*nFaces entries");
     if (!full) return;
-    // staging capacity and long rows
-    chunk_stats(ctx, m);
-    m->dinv.ensure(sizeof(double) * (n + pad));
-    m->dinv_sqrt.ensure(sizeof(double) * (n + pad));
-    if (n > 0) {
-        k_diag_derived<<<gc, kBlock, 0, ctx->stream>>>(n, m->diag.as<double>(), m->dinv.as<double>(),
-                                                       m->dinv_sqrt.as<double>());
-        CF_CHECK_LAUNCH();
-    }
     m->have_valT = m->have_32 = m->have_T32 = m->have_dmin = false;
     ++m->gen;
 }
@@ -860,11 +840,9 @@ void matrix_update_values(Matrix *m, const double *diag, const double *lower, co
         k_fill_csr<<<gc, kBlock, 0, ctx->stream>>>(m->n, m->lstart.as<int32_t>(), m->ostart.as<int32_t>(),
                                                    m->losort.as<int32_t>(), m->la.as<int32_t>(),
                                                    m->ua.as<int32_t>(), m->diag.as<double>(),
-                                                   m->lower.as<double>(), m->upper.as<double>(),
-                                                   m->ro.as<int32_t>(), nullptr, m->val.as<double>());
-        CF_CHECK_LAUNCH();
-        k_diag_derived<<<gc, kBlock, 0, ctx->stream>>>(m->n, m->diag.as<double>(), m->dinv.as<double>(),
-                                                       m->dinv_sqrt.as<double>());
+                                                   m->lower.as<double>(), m->upper.as<double>(), nullptr, nullptr,
+                                                   m->val.as<double>(), m->dinv.as<double>(),
+                                                   m->dinv_sqrt.as<double>(), nullptr);
         CF_CHECK_LAUNCH();
     }
     m->have_valT = m->have_32 = m->have_T32 = m->have_dmin = false;
@@ -891,7 +869,7 @@ void matrix_ensure_transpose(Matrix *m)
         k_fill_csr<<<grid_for(ctx, (int64_t)m->n + 1), kBlock, 0, ctx->stream>>>(
             m->n, m->lstart.as<int32_t>(), m->ostart.as<int32_t>(), m->losort.as<int32_t>(),
             m->la.as<int32_t>(), m->ua.as<int32_t>(), m->diag.as<double>(), m->upper.as<double>(),
-            m->lower.as<double>(), m->ro.as<int32_t>(), nullptr, m->valT.as<double>());
+            m->lower.as<double>(), nullptr, nullptr, m->valT.as<double>(), nullptr, nullptr, nullptr);
         CF_CHECK_LAUNCH();
     }
     m->have_valT = true;
@@ -1005,36 +983,32 @@ Matrix *matrix_from_csr(Context *ctx, int n, int64_t nnz, const int32_t *ro, con
         m->nnz = nnz;
         m->from_csr = true;
         const size_t pad = 4;
-        m->ro.ensure(sizeof(int32_t) * (n + 1 + pad));
-        m->col.ensure(sizeof(int32_t) * (nnz + pad));
-        m->val.ensure(sizeof(double) * (nnz + pad));
+        Carve parts;
+        parts.add(m->ro, sizeof(int32_t) * (n + 1 + pad));
+        parts.add(m->col, sizeof(int32_t) * (nnz + pad));
+        parts.add(m->val, sizeof(double) * (nnz + pad));
+        parts.add(m->diag, sizeof(double) * (n + pad));
+        parts.add(m->dinv, sizeof(double) * (n + pad));
+        parts.add(m->dinv_sqrt, sizeof(double) * (n + pad));
+        parts.add(m->s_off, sizeof(int32_t) * ((size_t)((n + 31) / 32) + 1));
+        parts.commit(m->arena);
         CF_CUDA(cudaMemcpyAsync(m->ro.ptr, ro, sizeof(int32_t) * (n + 1), cudaMemcpyDeviceToDevice, ctx->stream));
         CF_CUDA(cudaMemcpyAsync(m->col.ptr, col, sizeof(int32_t) * nnz, cudaMemcpyDeviceToDevice, ctx->stream));
         CF_CUDA(cudaMemcpyAsync(m->val.ptr, val, sizeof(double) * nnz, cudaMemcpyDeviceToDevice, ctx->stream));
         CF_CUDA(cudaMemsetAsync(m->col.as<int32_t>() + nnz, 0, sizeof(int32_t) * pad, ctx->stream));
         CF_CUDA(cudaMemsetAsync(m->val.as<double>() + nnz, 0, sizeof(double) * pad, ctx->stream));
-        DeviceBuffer flag;
-        flag.ensure(sizeof(int) * 2);
-        CF_CUDA(cudaMemsetAsync(flag.ptr, 0, sizeof(int) * 2, ctx->stream));
+        PatternStats *st = clear_stats(ctx);
         const int gc = grid_for(ctx, (int64_t)n + 1);
-        k_csr_check<<<gc, kBlock, 0, ctx->stream>>>(n, n, m->ro.as<int32_t>(), m->col.as<int32_t>(), nnz,
-                                                    flag.as<int>());
+        k_csr_check<<<gc, kBlock, 0, ctx->stream>>>(n, n, m->ro.as<int32_t>(), m->col.as<int32_t>(), nnz, &st->err);
         CF_CHECK_LAUNCH();
-        int32_t last = 0;
-        CF_CUDA(cudaMemcpyAsync(&last, m->ro.as<int32_t>() + n, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                ctx->stream));
-        const int err = read_flag(ctx, flag.as<int>());
-        require(err == 0 && (int64_t)last == nnz, CF_BAD_INPUT, "invalid CSR matrix");
-        m->diag.ensure(sizeof(double) * (n + pad));
         k_csr_diag<<<gc, kBlock, 0, ctx->stream>>>(n, m->ro.as<int32_t>(), m->col.as<int32_t>(),
-                                                   m->val.as<double>(), m->diag.as<double>());
+                                                   m->val.as<double>(), m->diag.as<double>(), &st->err);
         CF_CHECK_LAUNCH();
-        m->dinv.ensure(sizeof(double) * (n + pad));
-        m->dinv_sqrt.ensure(sizeof(double) * (n + pad));
         k_diag_derived<<<gc, kBlock, 0, ctx->stream>>>(n, m->diag.as<double>(), m->dinv.as<double>(),
                                                        m->dinv_sqrt.as<double>());
         CF_CHECK_LAUNCH();
-        chunk_stats(ctx, m);
+        queue_row_stats(ctx, m, st);
+        require(read_stats(ctx, m, st) == 0, CF_BAD_INPUT, "invalid CSR matrix");
     } catch (...) {
         delete m;
         throw;
@@ -1054,7 +1028,7 @@ void matrix_update_csr_values(Matrix *m, const double *vals, int memory)
     if (m->nnz > 0) upload(ctx, m->val.ptr, vals, sizeof(double) * (size_t)m->nnz, memory);
     const int gc = grid_for(ctx, (int64_t)m->n + 1);
     k_csr_diag<<<gc, kBlock, 0, ctx->stream>>>(m->n, m->ro.as<int32_t>(), m->col.as<int32_t>(), m->val.as<double>(),
-                                               m->diag.as<double>());
+                                               m->diag.as<double>(), nullptr);
     CF_CHECK_LAUNCH();
     k_diag_derived<<<gc, kBlock, 0, ctx->stream>>>(m->n, m->diag.as<double>(), m->dinv.as<double>(),
                                                    m->dinv_sqrt.as<double>());
@@ -1113,66 +1087,61 @@ bool matrix_ensure_sell(Matrix *m, bool transpose, bool fp32)
     Context *ctx = m->ctx;
     if (m->sell < 0) {
         m->sell = 0;
+        m->have_sval = m->have_svalT = m->have_sval32 = m->have_svalT32 = false;
         if (m->format_request != CF_FORMAT_CSR && m->n > 0) {
             const int ns = (m->n + 31) / 32;
-            m->s_off.ensure(sizeof(int32_t) * ((size_t)ns + 1));
-            DeviceBuffer slen, tmp, tot;
-            slen.ensure(sizeof(int32_t) * ((size_t)ns + 1));
-            tot.ensure(2 * sizeof(unsigned long long));
-            CF_CUDA(cudaMemsetAsync(tot.ptr, 0, 2 * sizeof(unsigned long long), ctx->stream));
-            k_sell_len<<<grid_for(ctx, (int64_t)ns + 1), kBlock, 0, ctx->stream>>>(
-                m->n, ns, m->ro.as<int32_t>(), slen.as<int32_t>(), tot.as<unsigned long long>());
-            CF_CHECK_LAUNCH();
             const int req = m->format_request;
             const bool want_codes = req == CF_FORMAT_AUTO || req == CF_FORMAT_SELL_C8;
             const bool want_d16 = req == CF_FORMAT_AUTO || req == CF_FORMAT_SELL_D16;
-            if (want_codes || want_d16) queue_offsets(m);
-            unsigned long long sizes[2] = {0, 0};
-            std::vector<int32_t> hk(want_codes || want_d16 ? kCodeHash + 2 : 0);
-            CF_CUDA(cudaMemcpyAsync(sizes, tot.ptr, sizeof(sizes), cudaMemcpyDeviceToHost, ctx->stream));
-            if (want_codes || want_d16)
-                CF_CUDA(cudaMemcpyAsync(hk.data(), ctx->scratch_codes.ptr, sizeof(int32_t) * (kCodeHash + 2),
-                                        cudaMemcpyDeviceToHost, ctx->stream));
-            CF_CUDA(cudaStreamSynchronize(ctx->stream));
-            const unsigned long long total = sizes[0];
-            const bool fits = total < (unsigned long long)INT32_MAX - 64;
+            const int64_t total = m->sell_nnz;   // the pattern's statistics: known since the build
+            const bool fits = total < (int64_t)INT32_MAX - 64;
             const bool good = fits && (double)total <= 1.2 * (double)m->nnz + 32.0 * 8 &&
                               m->nnz <= 32 * (int64_t)m->n;
             const bool forced = req == CF_FORMAT_SELL || req == CF_FORMAT_SELL_C8 || req == CF_FORMAT_SELL_D16;
+            m->sell = -1;   // a refused request is decided (and refused) again by the next call
             require(!forced || fits, CF_UNSUPPORTED, "SELL-32 copy exceeds 2^31 entries");
+            m->n_codes = want_codes ? (int32_t)m->offsets.size() : 0;
+            m->has_d16 = want_d16 && m->n_codes == 0 && m->max_offset <= 32767;
+            require(req != CF_FORMAT_SELL_C8 || m->n_codes > 0, CF_UNSUPPORTED,
+                    "one-byte column codes need at most " + std::to_string(kMaxCodes) +
+                        " distinct column offsets col - row");
+            require(req != CF_FORMAT_SELL_D16 || m->has_d16, CF_UNSUPPORTED,
+                    "16-bit column deltas need every |col - row| <= 32767");
+            m->sell = 0;
             if (forced || good) {
-                exclusive_scan(ctx, ns + 1, slen.as<int32_t>(), m->s_off.as<int32_t>(), tmp);
+                if (!m->slices_scanned) {
+                    exclusive_scan(ctx, ns + 1, m->s_off.as<int32_t>(), m->s_off.as<int32_t>(), ctx->scratch_tmp);
+                    m->slices_scanned = true;
+                }
                 m->n_slices = ns;
-                m->sell_nnz = (int64_t)total;
-                m->sell_max_len = (int32_t)sizes[1];
-                m->s_col.ensure(sizeof(int32_t) * ((size_t)total + 32));
-                k_sell_fill<double, double><<<grid_for(ctx, 32 * (int64_t)ns), kBlock, 0, ctx->stream>>>(
-                    m->n, ns, m->ro.as<int32_t>(), m->col.as<int32_t>(), nullptr, m->s_off.as<int32_t>(),
-                    m->s_col.as<int32_t>(), (double *)nullptr);
+                const bool codes = m->n_codes > 0;
+                Carve parts;
+                parts.add(m->s_col, sizeof(int32_t) * ((size_t)total + 32));
+                parts.add(m->s_val, sizeof(double) * ((size_t)total + 32));
+                if (codes) {
+                    parts.add(m->s_code, (size_t)total + 64);
+                    parts.add(m->s_dtab, sizeof(int32_t) * kCodeTable);
+                } else if (m->has_d16) {
+                    parts.add(m->s_d16, sizeof(int16_t) * ((size_t)total + 32));
+                }
+                parts.commit(m->sell_arena);
+                if (codes) {
+                    int32_t tab[kCodeTable] = {0};
+                    std::copy(m->offsets.begin(), m->offsets.end(), tab);
+                    // (a pageable source: staged when the call returns)
+                    CF_CUDA(cudaMemcpyAsync(m->s_dtab.ptr, tab, sizeof(tab), cudaMemcpyHostToDevice, ctx->stream));
+                }
+                auto build = codes ? k_sell_build<1> : m->has_d16 ? k_sell_build<2> : k_sell_build<0>;
+                build<<<grid_for(ctx, 32 * (int64_t)ns), kBlock, 0, ctx->stream>>>(
+                    m->n, ns, m->ro.as<int32_t>(), m->col.as<int32_t>(), m->val.as<double>(), m->s_off.as<int32_t>(),
+                    m->s_col.as<int32_t>(), m->s_val.as<double>(), codes ? m->s_dtab.as<int32_t>() : nullptr,
+                    m->n_codes, codes ? m->s_code.as<uint8_t>() : nullptr,
+                    m->has_d16 ? m->s_d16.as<int16_t>() : nullptr);
                 CF_CHECK_LAUNCH();
                 m->sell = 1;
-                m->n_codes = 0;
-                m->has_d16 = false;
-                const int32_t count = (want_codes || want_d16) ? hk[kCodeHash] : 0;
-                const int32_t maxoff = (want_codes || want_d16) ? hk[kCodeHash + 1] : INT32_MAX;
-                if (want_codes) {
-                    hk.resize(kCodeHash);
-                    build_sell_codes(m, hk, count);
-                }
-                if (want_d16 && m->n_codes == 0 && maxoff <= 32767) build_sell_d16(m);
-                if (req == CF_FORMAT_SELL_C8 && m->n_codes == 0) {
-                    m->sell = -1;   // decided again (and refused again) by the next call
-                    throw Error{CF_UNSUPPORTED,
-                                "one-byte column codes need at most " + std::to_string(kMaxCodes) +
-                                    " distinct column offsets col - row"};
-                }
-                if (req == CF_FORMAT_SELL_D16 && !m->has_d16) {
-                    m->sell = -1;
-                    throw Error{CF_UNSUPPORTED, "16-bit column deltas need every |col - row| <= 32767"};
-                }
+                m->have_sval = true;
             }
         }
-        m->have_sval = m->have_svalT = m->have_sval32 = m->have_svalT32 = false;
         ++m->gen;
     }
     if (m->sell != 1) return false;
@@ -1182,16 +1151,12 @@ bool matrix_ensure_sell(Matrix *m, bool transpose, bool fp32)
         const dim3 g(grid_for(ctx, 32 * (int64_t)ns));
         if (f32) {
             dst.ensure(sizeof(float) * ((size_t)m->sell_nnz + 32));
-            k_sell_fill<double, float><<<g, kBlock, 0, ctx->stream>>>(m->n, ns, m->ro.as<int32_t>(),
-                                                                      m->col.as<int32_t>(), src,
-                                                                      m->s_off.as<int32_t>(), nullptr,
-                                                                      dst.as<float>());
+            k_sell_fill<double, float><<<g, kBlock, 0, ctx->stream>>>(m->n, ns, m->ro.as<int32_t>(), src,
+                                                                      m->s_off.as<int32_t>(), dst.as<float>());
         } else {
             dst.ensure(sizeof(double) * ((size_t)m->sell_nnz + 32));
-            k_sell_fill<double, double><<<g, kBlock, 0, ctx->stream>>>(m->n, ns, m->ro.as<int32_t>(),
-                                                                       m->col.as<int32_t>(), src,
-                                                                       m->s_off.as<int32_t>(), nullptr,
-                                                                       dst.as<double>());
+            k_sell_fill<double, double><<<g, kBlock, 0, ctx->stream>>>(m->n, ns, m->ro.as<int32_t>(), src,
+                                                                       m->s_off.as<int32_t>(), dst.as<double>());
         }
         CF_CHECK_LAUNCH();
     };
