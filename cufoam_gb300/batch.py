@@ -46,8 +46,9 @@ def _bind(lib):
     return lib
 
 
-# schedule candidates of the autotuner: (cluster size, threads per CTA, order)
-CANDIDATES = [(cs, bt, 0) for cs in (1, 2, 4, 8, 16) for bt in (128, 256, 512)] + [(4, 256, 1)]
+# schedule candidates of the autotuner: (cluster size, threads per CTA, order);
+# cluster size 0: the library's choice (groups of blocks, or clusters of 16)
+CANDIDATES = [(0, 256, 0)] + [(cs, bt, 0) for cs in (1, 2, 4, 8, 16) for bt in (128, 256, 512)] + [(4, 256, 1)]
 
 
 def _cache_path() -> str:
@@ -141,7 +142,7 @@ class BatchSolver:
         c.precision = {"FP64": _capi.CF_PREC_FP64, "mixed": _capi.CF_PREC_MIXED}[precision]
         c.mixed_inner_rtol = inner_rtol
         cfg = cf_batch_config()
-        cs, bt, order = config or self.config or (0, 256, 0)   # cluster 0: the library picks 16 or 8
+        cs, bt, order = config or self.config or (0, 256, 0)   # cluster 0: the library picks
         cfg.cluster_size, cfg.threads, cfg.order = cs, bt, order
         res = (cf_batch_result * (len(self.systems) * self.n_rhs))()
         ms = C.c_double()

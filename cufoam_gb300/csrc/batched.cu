@@ -29,11 +29,17 @@
 // and forms the FP64 residual b - A x again; the FP64 tolerance decides
 // convergence.
 //
+// Two scopes a system is solved in (ClusterScope, GroupScope): a cluster that
+// takes systems from the queue, or -- for batches of few systems, where the
+// largest one would keep its cluster's quarter of 16 SMs busy long after the
+// others are done -- a fixed group of blocks per system, sized by its work,
+// with software barriers (see group_plan).
+//
 // The same kernel with one system and one component is the single-launch
-// CG of small systems (solve_cg_single_cluster, at the end of this file).
+// CG of small CSR systems (solve_cg_single_cluster, at the end of this file).
 #include <cooperative_groups.h>
 
-#include "device.cuh"
+#include "persist.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -100,6 +106,13 @@ struct BatchArgs {
     float *r32, *p32, *q32, *e32;   // [rows][R]
     double inner_rtol;
     int32_t max_outer;
+    // groups of blocks (GroupScope): each block's group, the groups' arrival
+    // counters (zero at the launch), the blocks' partial sums, and a flag set
+    // when a wait gave up
+    const int4 *group;       // per block: system, rank in its group, the group's blocks, its first block
+    uint32_t *arrivals;      // [n_systems]
+    double *partials;        // [2][3 kBatchMaxR][blocks]
+    int32_t *gave_up;
 };
 
 struct NoPost {
@@ -160,6 +173,145 @@ __device__ __forceinline__ void cluster_sum(cgp::cluster_group &cl, double (&v)[
     }
     __syncthreads();
 }
+
+// ---------------------------------------------------------------------------
+// where one system is solved: sync() and sum() over its blocks, next() the
+// system to solve (-1: none)
+// ---------------------------------------------------------------------------
+struct ClusterScope {
+    static constexpr int entries(int) { return kBatchEntryBatch; }
+    cgp::cluster_group cl;
+    __device__ __forceinline__ ClusterScope(const BatchArgs &) : cl(cgp::this_cluster()) {}
+    __device__ __forceinline__ int blocks() const { return (int)cl.num_blocks(); }
+    __device__ __forceinline__ int rank() const { return (int)cl.block_rank(); }
+    __device__ __forceinline__ void sync() { cl.sync(); }
+    template <int NV, int BT, class Post = NoPost>
+    __device__ __forceinline__ void sum(double (&v)[NV], double *wsm, double *slot, double *out, Post post = Post())
+    {
+        cluster_sum<NV, BT, Post>(cl, v, wsm, slot, out, post);
+    }
+    // the next system of the queue
+    __device__ __forceinline__ int next(const BatchArgs &a, int32_t *s_next)
+    {
+        if (rank() == 0 && threadIdx.x == 0) *s_next = atomicAdd(a.queue, 1);
+        cl.sync();
+        const int pos = *cl.map_shared_rank(s_next, 0);
+        cl.sync();
+        return pos < a.n_systems ? a.order[pos] : -1;
+    }
+    __device__ __forceinline__ void leave() { cl.sync(); }
+    __device__ __forceinline__ bool failed() const { return false; }
+};
+
+// A group of co-resident blocks (a cooperative launch) with a counter in
+// global memory: its blocks arrive with release, wait with acquire, and each
+// sums the group's partials in rank order.  A wait that gives up (kPollLimit)
+// makes every further sum NaN, which ends the solve.
+struct GroupScope {
+    // (48 systems, 662k rows: 1 component 1,018 us with one entry per batch,
+    // 941 with two; 3 components 1,915 and 2,088)
+    static constexpr int entries(int r) { return r == 1 ? 2 : 1; }
+    uint32_t *count;
+    double *part;
+    int32_t *gave_up;
+    int system, me, n, first, stride;
+    uint32_t epoch, red;
+    bool fail, taken;
+    __device__ __forceinline__ GroupScope(const BatchArgs &a)
+    {
+        const int4 g = a.group[blockIdx.x];
+        system = g.x;
+        me = g.y;
+        n = g.z;
+        first = g.w;
+        count = a.arrivals + system;
+        part = a.partials;
+        gave_up = a.gave_up;
+        stride = gridDim.x;
+        epoch = red = 0;
+        fail = taken = false;
+    }
+    __device__ __forceinline__ int blocks() const { return n; }
+    __device__ __forceinline__ int rank() const { return me; }
+    __device__ __forceinline__ void arrive_wait()
+    {
+        red_release(count);
+        const uint32_t want = (epoch + 1) * (uint32_t)n;
+        int k = 0;
+        while ((int32_t)(ld_acquire(count) - want) < 0)
+            if (++k > kPollLimit) {
+                *gave_up = 1;
+                fail = true;
+                break;
+            }
+    }
+    __device__ __forceinline__ void sync()
+    {
+        if (n == 1) {
+            __syncthreads();
+            return;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0 && !fail) arrive_wait();   // (thread 0's fail: the others meet it in sum)
+        ++epoch;
+        __syncthreads();
+    }
+    template <int NV, int BT, class Post = NoPost>
+    __device__ __forceinline__ void sum(double (&v)[NV], double *wsm, double *, double *out, Post post = Post())
+    {
+        constexpr int W = BT / 32;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const double t[1] = {v[i]};
+            const double s = warp_sum_fixed<1>(t);
+            if (lane == 0) wsm[i * W + warp] = s;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            double *p = part + (size_t)(red & 1) * 3 * kBatchMaxR * stride;
+#pragma unroll 1
+            for (int i = 0; i < NV; ++i) {
+                const double t[1] = {lane < W ? wsm[i * W + lane] : 0.0};
+                const double s = warp_sum_fixed<1>(t);
+                if (lane == 0) {
+                    if (n == 1) out[i] = s;
+                    else p[(size_t)i * stride + first + me] = s;
+                }
+            }
+            if (n > 1) {
+                if (lane == 0 && !fail) arrive_wait();
+                __syncwarp();
+                const bool bad = __shfl_sync(kFull, (int)fail, 0) != 0;
+#pragma unroll 1
+                for (int i = 0; i < NV; ++i) {
+                    const double *q = p + (size_t)i * stride + first;
+                    double t[4] = {0.0, 0.0, 0.0, 0.0};   // four chains over the group's partials, fixed order
+                    for (int b = lane; b < n; b += 128) {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (b + 32 * u < n) t[u] += ld_cg(q + b + 32 * u);
+                    }
+                    const double s = warp_sum_fixed<4>(t);
+                    if (lane == 0) out[i] = bad ? nan("") : s;
+                }
+            }
+            if (lane == 0)
+#pragma unroll 1
+                for (int i = 0; i < NV; ++i) post(i, out[i]);
+        }
+        ++epoch;
+        ++red;
+        __syncthreads();
+    }
+    __device__ __forceinline__ int next(const BatchArgs &, int32_t *)
+    {
+        if (taken) return -1;
+        taken = true;
+        return system;
+    }
+    __device__ __forceinline__ void leave() {}
+};
 
 // Row stride of the gathered search direction p: the R components of a
 // cell padded to 4 when R = 3, so that one gather is one 32-byte (FP64) or
@@ -234,7 +386,7 @@ __device__ __forceinline__ void st_row(float *p, int64_t c, const float (&v)[R])
 // g(c, out) gathers the R components of row c; ys = sum_e a_e.
 // SELL-32: the slice's entries, kBatchEntryBatch loaded (streamed, L2
 // evict-first) before their gathers; CSR: the row's own range.
-template <int R, class V, class T, class G>
+template <int R, class V, class T, int B64 = kBatchEntryBatch, class G>
 __device__ __forceinline__ void row_product(const BatchSystem &S, const V *__restrict__ sval,
                                             const V *__restrict__ cval, int s, int row, const bool (&on)[R],
                                             G g, T (&y)[R], T &ys)
@@ -243,7 +395,7 @@ __device__ __forceinline__ void row_product(const BatchSystem &S, const V *__res
     for (int j = 0; j < R; ++j) y[j] = T(0);
     ys = T(0);
     if (S.sell) {
-        constexpr int B = sizeof(V) == 4 ? kBatchEntryBatch32 : kBatchEntryBatch;
+        constexpr int B = sizeof(V) == 4 ? kBatchEntryBatch32 : B64;
 #if CF_BATCH_STREAM_HINT
         const uint64_t pol = l2_evict_first_policy();
 #define CF_BATCH_LD(ptr) ld_stream(ptr, pol)
@@ -303,8 +455,8 @@ struct CompState {
 
 // FP64 residual r = b - A x and ||r||^2 per component over this CTA's slices,
 // summed over the cluster into tot[0..R)
-template <int R, int BT>
-__device__ __forceinline__ void batch_residual(cgp::cluster_group &cl, const BatchSystem &S, int s_lo, int s_hi,
+template <int R, int BT, class Scope>
+__device__ __forceinline__ void batch_residual(Scope &sc, const BatchSystem &S, int s_lo, int s_hi,
                                                const double *b, const double *x, double *r, double *wsm,
                                                double *slot, double *tot)
 {
@@ -333,7 +485,7 @@ __device__ __forceinline__ void batch_residual(cgp::cluster_group &cl, const Bat
                 acc[j] = fma_t(ri, ri, acc[j]);
             }
     }
-    cluster_sum<R, BT>(cl, acc, wsm, slot, tot);
+    sc.template sum<R, BT>(acc, wsm, slot, tot);
 }
 
 // Minimum CTAs per SM for the register budget (1,024 threads: 64
@@ -345,12 +497,12 @@ template <int BT> constexpr int batch_min_blocks()
     return CF_BATCH_THREADS_PER_SM / BT > 0 ? CF_BATCH_THREADS_PER_SM / BT : 1;
 }
 
-template <int R, int BT, bool MIXED>
+template <int R, int BT, bool MIXED, class Scope>
 __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const BatchArgs a)
 {
-    cgp::cluster_group cl = cgp::this_cluster();
-    const int cs = (int)cl.num_blocks();
-    const int rank = (int)cl.block_rank();
+    Scope sc(a);
+    const int cs = sc.blocks();
+    const int rank = sc.rank();
     constexpr int W = BT / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ double wsm[3 * R * W];
@@ -364,12 +516,8 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
     int parity = 0;
 
     for (;;) {
-        if (rank == 0 && threadIdx.x == 0) s_next = atomicAdd(a.queue, 1);
-        cl.sync();
-        const int pos = *cl.map_shared_rank(&s_next, 0);
-        cl.sync();
-        if (pos >= a.n_systems) break;
-        const int sid = a.order[pos];
+        const int sid = sc.next(a, &s_next);
+        if (sid < 0) break;
         if (threadIdx.x == 0) S = a.sys[sid];
         __syncthreads();
         const int n = S.n;
@@ -390,7 +538,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
 #pragma unroll
                     for (int j = 0; j < R; ++j) acc1[j] += x[(int64_t)row * R + j];
             }
-            cluster_sum<R, BT>(cl, acc1, wsm, slot[parity], tot);
+            sc.template sum<R, BT>(acc1, wsm, slot[parity], tot);
             parity ^= 1;
         }
         // ---- normFactor part 2 + initial residual r = b - A x ------------
@@ -428,7 +576,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                         acc3[2 * R + j] = fma_t(ri, ri, acc3[2 * R + j]);
                     }
             }
-            cluster_sum<3 * R, BT>(cl, acc3, wsm, slot[parity], tot);
+            sc.template sum<3 * R, BT>(acc3, wsm, slot[parity], tot);
             parity ^= 1;
         }
         if (threadIdx.x < R) {
@@ -480,7 +628,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                                 acc0[j] += (double)(v * v);
                             }
                     }
-                    cluster_sum<R, BT>(cl, acc0, wsm, slot[parity], tot);
+                    sc.template sum<R, BT>(acc0, wsm, slot[parity], tot);
                     parity ^= 1;
                 }
                 if (threadIdx.x < R) {
@@ -545,7 +693,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                         }
                     }
                     if (!any_in) break;
-                    cl.sync(); // p complete before any CTA gathers it
+                    sc.sync(); // p complete before any CTA gathers it
                     // A: q = A p, (p, q)
                     {
                         const float *p32 = a.p32 + S.vec_offset * pad_r<R>();
@@ -573,7 +721,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                         double acc[R];
 #pragma unroll
                         for (int j = 0; j < R; ++j) acc[j] = accf[j];
-                        cluster_sum<R, BT>(cl, acc, wsm, slot[parity], tot);
+                        sc.template sum<R, BT>(acc, wsm, slot[parity], tot);
                         parity ^= 1;
                     }
                     // B: r -= alpha q, (r, r)
@@ -614,7 +762,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
 #pragma unroll
                         for (int j = 0; j < R; ++j) acc2[j] = accf[j];
                         if (threadIdx.x < R) st.alpha[threadIdx.x] = alpha[threadIdx.x];
-                        cluster_sum<R, BT>(cl, acc2, wsm, slot[parity], tot);
+                        sc.template sum<R, BT>(acc2, wsm, slot[parity], tot);
                         parity ^= 1;
                     }
                     if (threadIdx.x < R) {
@@ -647,8 +795,8 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                                 }
                     }
                 }
-                cl.sync(); // every CTA's x rows are written before anyone gathers them
-                batch_residual<R, BT>(cl, S, s_lo, s_hi, a.b + S.vec_offset * R, a.x + S.vec_offset * R,
+                sc.sync(); // every CTA's x rows are written before anyone gathers them
+                batch_residual<R, BT>(sc, S, s_lo, s_hi, a.b + S.vec_offset * R, a.x + S.vec_offset * R,
                                       a.r + S.vec_offset * R, wsm, slot[parity], tot);
                 parity ^= 1;
                 if (threadIdx.x < R) {
@@ -702,7 +850,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                     }
                 }
                 if (!any) break;
-                cl.sync(); // p complete before any CTA gathers it
+                sc.sync(); // p complete before any CTA gathers it
                 // A: q = A p, (p, q)
                 {
                     const double *p = a.p + S.vec_offset * pad_r<R>();
@@ -713,7 +861,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                     for (int s = s_lo + warp; s < s_hi; s += W) {
                         const int row = s * 32 + lane;
                         double y[R], ys;
-                        row_product<R, double, double>(
+                        row_product<R, double, double, Scope::entries(R)>(
                             S, S.s_val, S.val, s, row, act,
                             [&](int c, double(&o)[R]) { ld_row<R>(p, c, o); }, y, ys);
                         if (row < n) {
@@ -729,7 +877,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                     }
                     // the step lengths, once per CTA (a division is a chain of
                     // dependent FP64 instructions)
-                    cluster_sum<R, BT>(cl, acc, wsm, slot[parity], tot, [&](int j, double pq) {
+                    sc.template sum<R, BT>(acc, wsm, slot[parity], tot, [&](int j, double pq) {
                         st.alpha[j] = st.act[j] ? st.rho[j] / pq : 0.0;
                     });
                     parity ^= 1;
@@ -756,7 +904,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                                     acc2[j] = fma_t(ri, ri, acc2[j]);
                                 }
                     }
-                    cluster_sum<R, BT>(cl, acc2, wsm, slot[parity], tot);
+                    sc.template sum<R, BT>(acc2, wsm, slot[parity], tot);
                     parity ^= 1;
                 }
                 if (threadIdx.x < R) {
@@ -784,7 +932,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
         }
         __syncthreads();
     }
-    cl.sync(); // no CTA leaves while a peer may still read its shared memory
+    sc.leave(); // no CTA leaves while a peer may still read its shared memory
 }
 
 // ---------------------------------------------------------------------------
@@ -797,6 +945,7 @@ struct Batch {
     int64_t rows = 0;
     DeviceBuffer d_sys, d_order, d_queue, d_out, d_b, d_x, d_r, d_p, d_q;
     DeviceBuffer d_r32, d_p32, d_q32, d_e32;
+    DeviceBuffer d_group;           // groups of blocks: table, partial sums, counters
     bool have_32 = false;
     std::vector<int32_t> order;
     ~Batch()
@@ -865,7 +1014,7 @@ static void launch_batch(Context *ctx, const BatchArgs &args, int cs, int max_cl
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const auto kernel = k_batch_cg<R, BT, MIXED>;
+    const auto kernel = k_batch_cg<R, BT, MIXED, ClusterScope>;
     // cs == 0: 16-CTA clusters where they fit on the device, else 8
     const bool pick = cs == 0;
     int nclusters = 0;
@@ -903,6 +1052,118 @@ static void launch_batch_r(Context *ctx, const BatchArgs &args, bool mixed, int 
 {
     if (mixed) launch_batch_m<R, true>(ctx, args, cs, bt, max_clusters, s);
     else launch_batch_m<R, false>(ctx, args, cs, bt, max_clusters, s);
+}
+
+// ---------------------------------------------------------------------------
+// groups of blocks
+// ---------------------------------------------------------------------------
+constexpr int kGroupThreads = 256;
+// groups are taken up to this much more work per block than the clusters'
+// even schedule: at 1.04, 1.09 and 1.30 (100, 160 and 300 boxes) they took
+// 4.28, 3.90 and 4.11 ms against 5.37, 5.77 and 7.69 on clusters of 16 (and
+// 5.84, 4.38, 5.06 on clusters of 8), whose barriers cost the small systems
+// more; systems with very different step counts want the queue
+constexpr double kGroupSlack = 1.35;
+
+template <int R, bool MIXED>
+static const void *group_kernel() { return (const void *)k_batch_cg<R, kGroupThreads, MIXED, GroupScope>; }
+
+static const void *group_kernel_for(int nrhs, bool mixed)
+{
+    switch (nrhs) {
+    case 1: return mixed ? group_kernel<1, true>() : group_kernel<1, false>();
+    case 2: return mixed ? group_kernel<2, true>() : group_kernel<2, false>();
+    case 3: return mixed ? group_kernel<3, true>() : group_kernel<3, false>();
+    default: return mixed ? group_kernel<4, true>() : group_kernel<4, false>();
+    }
+}
+
+// The blocks of each system when `blocks` of them run at once: the smallest
+// largest share of work W with sum ceil(work / W) <= blocks (at most a block
+// per eight slices).  Empty when the queue of clusters would finish much
+// sooner (kGroupSlack): its clusters of 16 blocks take the systems largest
+// first, and a block's share is a sixteenth of its cluster's systems.  Both run
+// the same number of blocks per SM.  Measured on GB300
+// (transient 7-point systems to 1e-8, 3 components, clusters -> groups): 48
+// boxes of 12^3..36^3, 662k rows, 2.75 -> 1.92 ms; 8 such boxes 1.33 -> 0.70; 48
+// boxes of 10^3..18^3 1.22 -> 0.74; 16 of 20^3..24^3 1.23 -> 0.96; mixed precision,
+// 48 boxes 2.51 -> 1.84.  What is left there is L2: the three components of a
+// gathered row are 32 random bytes, about 5 TB/s.
+static std::vector<int> group_plan(const std::vector<int64_t> &work, const std::vector<int> &slices, int blocks,
+                                   int clusters)
+{
+    const int S = (int)work.size();
+    if (S > blocks || clusters < 1) return {};
+    auto share = [&](int s, int64_t w) {
+        const int64_t g = (work[s] + w - 1) / w;
+        return (int)std::max<int64_t>(1, std::min<int64_t>(g, (slices[s] + 7) / 8));
+    };
+    int64_t lo = 1, hi = 1;
+    for (int64_t w : work) hi = std::max(hi, w);
+    while (lo < hi) {
+        const int64_t mid = lo + (hi - lo) / 2;
+        int64_t n = 0;
+        for (int s = 0; s < S; ++s) n += share(s, mid);
+        if (n <= blocks) hi = mid;
+        else lo = mid + 1;
+    }
+    std::vector<int> g(S);
+    double most = 0.0;
+    for (int s = 0; s < S; ++s) {
+        g[s] = share(s, lo);
+        most = std::max(most, (double)work[s] / g[s]);
+    }
+    // the clusters' schedule
+    std::vector<int64_t> sorted(work), load(clusters, 0);
+    std::sort(sorted.begin(), sorted.end(), std::greater<int64_t>());
+    for (int64_t w : sorted) *std::min_element(load.begin(), load.end()) += w;
+    const double queue = (double)*std::max_element(load.begin(), load.end()) / 16.0;
+    if (most > kGroupSlack * queue) g.clear();
+    return g;
+}
+
+// Launches the batch as groups; false when the clusters are the better (or
+// the only possible) schedule.
+static bool launch_groups(Context *ctx, Batch *B, BatchArgs &a, int nrhs, bool mixed, cudaStream_t s)
+{
+    const int S = (int)B->mats.size();
+    const void *kernel = group_kernel_for(nrhs, mixed);
+    int per_sm = 0;
+    if (!persist_usable(ctx, CF_CG, kSell, false) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kGroupThreads, 0) != cudaSuccess || per_sm < 1) {
+        cudaGetLastError();
+        return false;
+    }
+    const int blocks = per_sm * ctx->sm_count;
+    if (S > blocks) return false;
+    std::vector<int64_t> work(S);
+    std::vector<int> slices(S);
+    for (int i = 0; i < S; ++i) {
+        work[i] = B->mats[i]->nnz;
+        slices[i] = (B->mats[i]->n + 31) / 32;
+    }
+    const std::vector<int> g = group_plan(work, slices, blocks, blocks / 16);
+    if (g.empty()) return false;
+    std::vector<int4> table;
+    for (int i = 0; i < S; ++i) {
+        const int first = (int)table.size();
+        for (int r = 0; r < g[i]; ++r) table.push_back(make_int4(i, r, g[i], first));
+    }
+    const int grid = (int)table.size();
+    const size_t tb = (sizeof(int4) * (size_t)grid + 255) / 256 * 256;
+    const size_t pb = sizeof(double) * 2 * 3 * kBatchMaxR * (size_t)grid;
+    B->d_group.ensure(tb + pb + sizeof(uint32_t) * ((size_t)S + 4));
+    char *base = B->d_group.as<char>();
+    a.group = reinterpret_cast<const int4 *>(base);
+    a.partials = reinterpret_cast<double *>(base + tb);
+    a.arrivals = reinterpret_cast<uint32_t *>(base + tb + pb);
+    a.gave_up = reinterpret_cast<int32_t *>(a.arrivals + S);
+    // (a pageable source: staged when the call returns)
+    CF_CUDA(cudaMemcpyAsync(base, table.data(), sizeof(int4) * (size_t)grid, cudaMemcpyHostToDevice, s));
+    CF_CUDA(cudaMemsetAsync(a.arrivals, 0, sizeof(uint32_t) * ((size_t)S + 4), s));
+    void *args[] = {&a};
+    CF_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kGroupThreads), args, 0, s));
+    return true;
 }
 
 // Solve all systems for `nrhs` right-hand sides (b, x: [rows][nrhs]).
@@ -962,7 +1223,7 @@ void batch_solve(Batch *B, const cf_controls &c, int nrhs, const double *b_in, d
     CF_CUDA(cudaMemcpyAsync(B->d_order.ptr, order.data(), sizeof(int32_t) * S, cudaMemcpyHostToDevice,
                             ctx->stream));
     CF_CUDA(cudaMemsetAsync(B->d_queue.ptr, 0, sizeof(int32_t), ctx->stream));
-    BatchArgs a;
+    BatchArgs a{};
     a.sys = B->d_sys.as<BatchSystem>();
     a.order = B->d_order.as<int32_t>();
     a.n_systems = S;
@@ -995,7 +1256,11 @@ void batch_solve(Batch *B, const cf_controls &c, int nrhs, const double *b_in, d
     cudaStream_t cs_stream = nullptr;
     const bool use_graph = c.use_graph != 0;
     CF_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
-    if (use_graph) {
+    // no cluster size asked for: groups of blocks where they finish sooner
+    const bool grouped = cs == 0 && bt == kGroupThreads && maxc == 0 &&
+                         launch_groups(ctx, B, a, nrhs, mixed, ctx->stream);
+    if (grouped) {
+    } else if (use_graph) {
         CF_CUDA(cudaStreamCreateWithFlags(&cs_stream, cudaStreamNonBlocking));
         try {
             CF_CUDA(cudaStreamBeginCapture(cs_stream, cudaStreamCaptureModeThreadLocal));
@@ -1028,7 +1293,11 @@ void batch_solve(Batch *B, const cf_controls &c, int nrhs, const double *b_in, d
         }
     }
     CF_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
+    int32_t gave_up = 0;
+    if (grouped)
+        CF_CUDA(cudaMemcpyAsync(&gave_up, a.gave_up, sizeof(gave_up), cudaMemcpyDeviceToHost, ctx->stream));
     CF_CUDA(cudaStreamSynchronize(ctx->stream));
+    require(gave_up == 0, CF_TIMEOUT, "a block of the batched solve gave up waiting for its group");
     if (ge) cudaGraphExecDestroy(ge);
     if (g) cudaGraphDestroy(g);
     if (cs_stream) cudaStreamDestroy(cs_stream);
@@ -1068,7 +1337,7 @@ void batch_solve(Batch *B, const cf_controls &c, int nrhs, const double *b_in, d
 bool small_cg_ok(Context *ctx)
 {
     if (ctx->small_cg_ok < 0) {
-        const auto kernel = k_batch_cg<1, 256, false>;
+        const auto kernel = k_batch_cg<1, 256, false, ClusterScope>;
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;

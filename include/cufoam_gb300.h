@@ -407,8 +407,10 @@ const char *cf_file_last_error(void);
 typedef struct cf_batch cf_batch;
 
 typedef struct cf_batch_config {
-    int32_t cluster_size;   /* CTAs cooperating on one system: 1, 2, 4, 8, 16 (0 = 16 where it
-                               fits on the device, else 8) */
+    int32_t cluster_size;   /* CTAs cooperating on one system: 1, 2, 4, 8, 16 (0 = the library
+                               picks: with 256 threads and max_clusters 0 a group of blocks per
+                               system, sized by its work, for a batch of few systems; else
+                               clusters of 16 where they fit on the device, else 8) */
     int32_t threads;        /* threads per CTA: 128, 256, 512 (0 = 256) */
     int32_t order;          /* 0 = largest system first, 1 = given order */
     int32_t max_clusters;   /* 0 = one full wave */
