@@ -41,6 +41,7 @@ namespace cf {
 struct PersistPlan {
     int32_t q, r, x, scale;  // y / q, own r, x, the diagonal scaling
     int32_t g;               // own rows of the gathered p or z (with the matrix only)
+    int32_t g2;              // in a cluster: a second gathered vector (Jacobi's r, Richardson's power method)
     int32_t val, col;        // this block's slots of the loop's matrix
     int32_t off;             // its slices' offsets (always there)
 };
@@ -143,10 +144,12 @@ template <> struct PersistCols<kSellD> {
 // memory for the whole solve, and only the gathered vector crosses blocks.
 // SYNC: the grid, or one cluster.
 template <int SOLVER, int FMT, bool LOCALM, class SYNC>
-__global__ void __launch_bounds__(kPBlock, 1)
+__global__ void __launch_bounds__(SYNC::kThreads, 1)
     k_persist(const __grid_constant__ SolveArgs A, const __grid_constant__ PersistArgs P)
 {
     using Tr = PersistTraits<SOLVER>;
+    // in a cluster the gathered vectors live in the blocks' shared memory
+    constexpr bool DSM = SYNC::kCluster;
     __shared__ typename SYNC::Shared sh;
     __shared__ PersistState st;
     extern __shared__ __align__(16) double local_[];
@@ -166,14 +169,15 @@ __global__ void __launch_bounds__(kPBlock, 1)
     const double *b = A.b;
     const double *scale_g = Tr::kScale ? (SOLVER == CF_JMR ? A.corr_scale : A.dinv) : nullptr;
     // block-private vectors, indexed by row - base
-    double *q, *rl, *x, *own;
+    double *q, *rl, *x, *own, *own2 = nullptr;
     const double *scale;
     const int32_t *off;                      // slice offsets, indexed by s - s_lo
     if constexpr (LOCALM) {
         q = local_ + P.plan.q;
         rl = local_ + P.plan.r;
-        x = Tr::kLocalX ? local_ + P.plan.x : xg + base;
+        x = Tr::kLocalX || DSM ? local_ + P.plan.x : xg + base;
         own = local_ + P.plan.g;
+        own2 = local_ + P.plan.g2;
         scale = local_ + P.plan.scale;
         off = reinterpret_cast<const int32_t *>(local_ + P.plan.off);
     } else {
@@ -186,7 +190,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
     }
     const bool x_local = x != xg + base;
     // r also goes to global memory where the product gathers it
-    double *const rg = Tr::kGatherR && rl != A.r[0] + base ? A.r[0] + base : nullptr;
+    double *const rg = !DSM && Tr::kGatherR && rl != A.r[0] + base ? A.r[0] + base : nullptr;
     const double *lval = nullptr;
     const int32_t *lcol = nullptr;
     if (LOCALM || P.plan.off >= 0) {
@@ -200,7 +204,18 @@ __global__ void __launch_bounds__(kPBlock, 1)
         int32_t *dc = reinterpret_cast<int32_t *>(local_ + P.plan.col);
         for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
             dv[e - e0] = __ldg(src + e);
-            dc[e - e0] = __ldg(A.s_col + e);
+            const int c = __ldg(A.s_col + e);
+            if constexpr (DSM) {
+                // the cluster address of row c's element of rl, in the block
+                // that owns its slice
+                const int t = c >> 5, nb = gs.blocks();
+                int o = (int)((int64_t)t * nb / ns);
+                while ((int)((int64_t)ns * (o + 1) / nb) <= t) ++o;
+                const int o_lo = (int)((int64_t)ns * o / nb);
+                dc[e - e0] = (int)(gs.remote(rl, (uint32_t)o) + 8u * (uint32_t)(c - 32 * o_lo));
+            } else {
+                dc[e - e0] = c;
+            }
         }
         for (int i = threadIdx.x; i < 32 * (s_hi - s_lo); i += blockDim.x)
             if (Tr::kScale && base + i < n) local_[P.plan.scale + i] = scale_g[base + i];
@@ -209,6 +224,21 @@ __global__ void __launch_bounds__(kPBlock, 1)
     }
     __syncthreads();
 
+    // what the product gathers: own rows `mine` of a vector in a cluster (the
+    // slots hold the cluster addresses of rl's elements; every vector is at the
+    // same place in every block), else the vector itself
+    auto gather = [&](const double *mine, const double *global) {
+        if constexpr (DSM) {
+            const int shift = (int)(reinterpret_cast<const char *>(mine) - reinterpret_cast<const char *>(rl));
+            return [shift](int a) {
+                double v;
+                asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a + shift));
+                return v;
+            };
+        } else {
+            return [global](int c) { return global[c]; };
+        }
+    };
     // this lane's row of slice s over the loop's matrix
     auto product = [&](const double *val, int s, auto g) {
         const int o = off[s - s_lo], len = (off[s - s_lo + 1] - o) >> 5;
@@ -250,7 +280,9 @@ __global__ void __launch_bounds__(kPBlock, 1)
         double acc[4] = {0.0, 0.0, 0.0, 0.0};
         for (int s = s_lo + warp; s < s_hi; s += nw) {
             const int row = 32 * s + lane, i = row - base;
-            const double y = product_a(s, [&](int c) { return xg[c]; });
+            double y;
+            if constexpr (LOCALM && !Tr::kScaledMatrix) y = product_a(s, gather(x, xg));
+            else y = product_a(s, [&](int c) { return xg[c]; });
             double yb = product_a(s, [&](int) { return cval; });
             if (P.l1) yb = __dmul_rn(yb, xbar);
             if (row < n) {
@@ -270,7 +302,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
                 if (SOLVER == CF_PCG) acc[3] = fma_t(ri, __dmul_rn(scale[i], ri), acc[3]);
                 if (SOLVER == CF_MRJACOBI) {
                     const double zi = __dmul_rn(scale[i], ri);
-                    A.w[1][row] = zi;
+                    if (!DSM) A.w[1][row] = zi;
                     if (LOCALM) own[i] = zi;
                 }
             }
@@ -295,15 +327,23 @@ __global__ void __launch_bounds__(kPBlock, 1)
             const bool last = j == P.power_steps;
             const double sc = st.pow_inv;
             const double *yp = A.w[(j + 1) & 1];
-            double *yn = A.w[j & 1];
-            auto g = [&](int c) { return j == 0 ? inv_n : __dmul_rn(sc, yp[c]); };
+            double *yn = A.w[j & 1] + base;
+            const double *ypl = yp + base;
+            if constexpr (DSM) {
+                ypl = j & 1 ? own : own2;
+                yn = j & 1 ? own2 : own;
+            }
+            auto gy = gather(ypl, yp);
+            auto scaled = [&](double v) { return j == 0 ? inv_n : __dmul_rn(sc, v); };
             double acc[1] = {0.0};
             for (int s = s_lo + warp; s < s_hi; s += nw) {
-                const int row = 32 * s + lane;
-                const double v = product_a(s, g);
+                const int row = 32 * s + lane, i = row - base;
+                double v;
+                if (j == 0) v = product_a(s, [&](int) { return inv_n; });
+                else v = product_a(s, [&](int c) { return __dmul_rn(sc, gy(c)); });
                 if (row < n) {
-                    if (!last) yn[row] = v;
-                    acc[0] = fma_t(last ? g(row) : v, v, acc[0]);
+                    if (!last) yn[i] = v;
+                    acc[0] = fma_t(last ? scaled(j == 0 ? 0.0 : ypl[i]) : v, v, acc[0]);
                 }
             }
             if (!gs.sum(acc, nullptr, [&](const double(&t)[1]) {
@@ -350,7 +390,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
                                 x[i] = fma_t(xi, pv[h], xv[h]);
                                 rv[h] = fma_t(beta, pv[h], rv[h]);
                             }
-                            p[row] = rv[h];
+                            if (!DSM) p[row] = rv[h];
                             if (LOCALM) own[i] = rv[h];
                         }
                 }
@@ -362,7 +402,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
                 double acc[1] = {0.0};
                 for (int s = s_lo + warp; s < s_hi; s += nw) {
                     const int row = 32 * s + lane;
-                    const double y = product(A.s_val, s, [&](int c) { return p[c]; });
+                    const double y = product(A.s_val, s, gather(own, p));
                     if (row < n) {
                         q[row - base] = y;
                         acc[0] = fma_t(own[row - base], y, acc[0]);
@@ -417,7 +457,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
                 double acc[2] = {0.0, 0.0};
                 for (int s = s_lo + warp; s < s_hi; s += nw) {
                     const int row = 32 * s + lane, i = row - base;
-                    const double y = product(val, s, [&](int c) { return gv[c]; });
+                    const double y = product(val, s, gather(SOLVER == CF_MRJACOBI ? own : rl, gv));
                     if (row < n) {
                         q[i] = y;
                         acc[0] = fma_t(rl[i], y, acc[0]);
@@ -457,7 +497,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
                         if (rg) rg[i] = ri;
                         if (SOLVER == CF_MRJACOBI) {
                             const double zi = __dmul_rn(sv[h], ri);
-                            gv[row] = zi;
+                            if (!DSM) gv[row] = zi;
                             if (LOCALM) own[i] = zi;
                         }
                         acc[0] = fma_t(ri, ri, acc[0]);
@@ -469,17 +509,24 @@ __global__ void __launch_bounds__(kPBlock, 1)
         } else if constexpr (SOLVER == CF_JACOBI) {
             // one pass over A D^-1: the residual alternates between r[0] and r[1]
             const double *rin = A.r[(k + 1) & 1];
-            double *rout = A.r[k & 1];
+            double *rout = A.r[k & 1] + base;
+            const double *mine = rin + base;
+            if constexpr (DSM) {
+                mine = k & 1 ? rl : own2;
+                rout = k & 1 ? own2 : rl;
+            } else if constexpr (LOCALM) {
+                mine = rl;
+            }
             double acc[1] = {0.0};
             for (int s = s_lo + warp; s < s_hi; s += nw) {
                 const int row = 32 * s + lane, i = row - base;
-                const double y = product(A.sc_val, s, [&](int c) { return rin[c]; });
+                const double y = product(A.sc_val, s, gather(mine, rin));
                 if (row < n) {
-                    const double r0 = LOCALM ? rl[i] : rin[row];
+                    const double r0 = mine[i];
                     x[i] = fma_t(1.0, __dmul_rn(scale[i], r0), x[i]);
                     const double ri = fma_t(-1.0, y, r0);
-                    rout[row] = ri;
-                    if (LOCALM) rl[i] = ri;
+                    rout[i] = ri;
+                    if (LOCALM && !DSM) rl[i] = ri;
                     acc[0] = fma_t(ri, ri, acc[0]);
                 }
             }
@@ -491,13 +538,13 @@ __global__ void __launch_bounds__(kPBlock, 1)
             const double omega = st.omega;
             for (int s = s_lo + warp; s < s_hi; s += nw) {
                 const int row = 32 * s + lane;
-                if (row < n) xg[row] = fma_t(omega, rl[row - base], xg[row]);
+                if (row < n) x[row - base] = fma_t(omega, rl[row - base], x[row - base]);
             }
             if (!gs.barrier()) goto out;
             double acc[1] = {0.0};
             for (int s = s_lo + warp; s < s_hi; s += nw) {
                 const int row = 32 * s + lane;
-                const double t = product(A.s_val, s, [&](int c) { return xg[c]; });
+                const double t = product(A.s_val, s, gather(x, xg));
                 if (row < n) {
                     const double ri = b[row] - t;
                     rl[row - base] = ri;
@@ -584,7 +631,7 @@ bool persist_usable(Context *ctx, int solver, int format, bool mixed)
         attr[0].val.clusterDim.x = 16;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
-        cfg.blockDim = dim3(kPBlock);
+        cfg.blockDim = dim3(ClusterSync::kThreads);
         cfg.gridDim = dim3(16);
         cfg.attrs = attr;
         cfg.numAttrs = 1;
@@ -665,7 +712,7 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
     const bool own = solver == CF_CG || solver == CF_PCG || solver == CF_MRJACOBI || solver == CF_MRS;
     const int ns = A.n_slices;
     // everything a block of `slices` slices keeps in shared memory, in doubles
-    auto plan_all = [&](int slices) {
+    auto plan_all = [&](int slices, bool cluster) {
         PersistPlan p;
         int at = 0;
         auto take = [&](int doubles) {
@@ -676,9 +723,11 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
         p.off = take(slices / 2 + 2);
         p.q = q ? take(32 * slices) : -1;
         p.r = take(32 * slices);
-        p.x = local_x ? take(32 * slices) : -1;
+        p.x = local_x || cluster ? take(32 * slices) : -1;
         p.scale = scale ? take(32 * slices) : -1;
-        p.g = own ? take(32 * slices) : -1;
+        const bool power = cluster && solver == CF_RICHARDSON;
+        p.g = own || power ? take(32 * slices) : -1;
+        p.g2 = power || (cluster && solver == CF_JACOBI) ? take(32 * slices) : -1;
         p.val = take(32 * slices * max_len);
         p.col = take(16 * slices * max_len);
         return std::make_pair(p, sizeof(double) * (size_t)at);
@@ -690,7 +739,7 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
         // one warp per sub-partition and block before another block is added
         grid = 1;
         while (grid < 16 && 4 * grid < ns) grid <<= 1;
-        const auto pl = plan_all((ns + grid - 1) / grid);
+        const auto pl = plan_all((ns + grid - 1) / grid, true);
         if (pl.second + sizeof(ClusterSync::Shared) <= CF_PERSIST_LOCAL_BYTES) {
             scope = kScopeCluster;
             P.plan = pl.first;
@@ -700,7 +749,7 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
     if (scope == kScopeGrid) {
         grid = std::max(1, std::min(ctx->sm_count, (ns + 3) / 4));
         const int slices = (ns + grid - 1) / grid;
-        const auto pl = slices <= 4096 && max_len <= 64 ? plan_all(slices) : std::make_pair(PersistPlan{}, ~(size_t)0);
+        const auto pl = slices <= 4096 && max_len <= 64 ? plan_all(slices, false) : std::make_pair(PersistPlan{}, ~(size_t)0);
         if (!A.has_long && pl.second <= CF_PERSIST_LOCAL_BYTES) {
             scope = kScopeGridLocal;
             P.plan = pl.first;
@@ -715,7 +764,7 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
                 at += doubles;
                 return o;
             };
-            P.plan.val = P.plan.col = P.plan.scale = P.plan.g = -1;
+            P.plan.val = P.plan.col = P.plan.scale = P.plan.g = P.plan.g2 = -1;
             P.plan.off = take(slices <= 4096, slices / 2 + 2);
             P.plan.q = take(slices <= 4096 && q, 32 * slices);
             P.plan.r = take(slices <= 4096 && !gather_r, 32 * slices);

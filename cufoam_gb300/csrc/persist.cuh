@@ -134,7 +134,15 @@ __device__ __forceinline__ void red_release(uint32_t *p)
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
 }
 
+// Systems up to this many rows run in one cluster of up to 16 blocks: CG step
+// 5.4 us against 8.1 on the grid at 4,096 rows, 6.7 against 8.1 at 8,100, 8.6
+// against 8.3 at 12,100.
+#ifndef CF_PERSIST_CLUSTER_ROWS
+#define CF_PERSIST_CLUSTER_ROWS 10240
+#endif
+
 constexpr int kPClusterMax = 16;       // blocks of a cluster
+static_assert(CF_PERSIST_CLUSTER_ROWS % (32 * kPClusterMax) == 0, "whole warps");
 
 // SLOTS: room for the warp sums of every block of a cluster, by parity
 // (1 where the sums go through global memory)
@@ -177,6 +185,8 @@ __device__ __forceinline__ void block_sum_fixed(const double (&v)[NV], PersistSh
 // and return false when a wait gave up (grid only).
 // ---------------------------------------------------------------------------
 struct GridSync {
+    static constexpr bool kCluster = false;
+    static constexpr int kThreads = kPBlock;
     using Shared = PersistShared<1>;
     PersistGrid g;
     Shared *sh;
@@ -269,6 +279,9 @@ struct GridSync {
 // one thread-block cluster: the hardware barrier, sums through distributed
 // shared memory
 struct ClusterSync {
+    static constexpr bool kCluster = true;
+    // a warp per slice of the largest system a cluster takes: more registers each
+    static constexpr int kThreads = CF_PERSIST_CLUSTER_ROWS / kPClusterMax;
     using Shared = PersistShared<kPClusterMax * kPWarps>;
     Shared *sh;
     uint32_t red;
@@ -414,13 +427,6 @@ enum { kScopeGrid = 0, kScopeGridLocal = 1, kScopeCluster = 2 };
 #ifndef CF_PERSIST_VEC_BYTES
 #define CF_PERSIST_VEC_BYTES (144 * 1024)
 #endif
-// Systems up to this many rows run in one cluster of up to 16 blocks: CG step
-// 5.4 us against 8.1 on the grid at 4,096 rows, 6.7 against 8.1 at 8,100, 8.6
-// against 8.3 at 12,100.
-#ifndef CF_PERSIST_CLUSTER_ROWS
-#define CF_PERSIST_CLUSTER_ROWS 10240
-#endif
-
 // the barrier counter and partial sums of the context
 PersistGrid persist_grid(Context *ctx);
 // `grid` blocks, one warp per slice up to 32, cooperative or as one cluster

@@ -79,7 +79,7 @@ template <> struct MixedCols<kSellD> {
         if (const int row = 32 * (s + h * nw) + lane, i = row - base; s + h * nw < s_hi && row < n && i >= 0)
 
 template <int SOLVER, int FMT, bool LOCALM, class SYNC>
-__global__ void __launch_bounds__(kPBlock, 1)
+__global__ void __launch_bounds__(SYNC::kThreads, 1)
     k_persist_mixed(const __grid_constant__ SolveArgs A, const __grid_constant__ MixedArgs P)
 {
     __shared__ typename SYNC::Shared sh;
