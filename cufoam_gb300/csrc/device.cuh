@@ -145,10 +145,10 @@ struct SeqScratch {
     int32_t events;        // -1: add one by one
 };
 
-// inclusive scan over the block of one 64-bit value per thread
-__device__ __forceinline__ long long seq_block_scan(long long v, long long *wsum)
+// inclusive scan over a group of 256 threads of one 64-bit value per thread
+__device__ __forceinline__ long long seq_block_scan(long long v, long long *wsum, int warp)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const long long t = __shfl_up_sync(kFull, v, o);
@@ -163,16 +163,22 @@ __device__ __forceinline__ long long seq_block_scan(long long v, long long *wsum
     return v + off;
 }
 
-// All 256 threads: the events of part[0 .. G) into rec (value j at rec[j],
-// the integers before it at rec[kSeqEvents + j]) and sc.
-static __device__ __noinline__ void seq_prepare(const double *part, int G, double *rec, SeqScratch *sc)
+// 256 threads (tid 0 .. 255 of their group; every group of the block calls it
+// together: it holds six block barriers on every path): the events of
+// part[0 .. G) into rec (value j at rec[j], the integers before it at
+// rec[kSeqEvents + j]) and sc.  buf: kSeqMax values of shared memory.  Each
+// thread takes its kSeqPer values one after the other from shared memory:
+// unrolled over registers the pass spilled 1.1 KB per thread in a 64-register
+// kernel and took 12,000 to 19,000 cycles; BiCG's step at 256 rows, two sums, fell
+// from 36 to 23 us with this form and 128 registers.
+static __device__ __noinline__ void seq_prepare(const double *part, int G, double *buf, double *rec, SeqScratch *sc,
+                                                int tid)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int k0 = threadIdx.x * kSeqPer;
-    double v[kSeqPer];
+    const int lane = tid & 31, warp = tid >> 5;
+    for (int k = tid; k < kSeqMax; k += kBlock) buf[k] = k < G ? ld_cg(part + k) : 0.0;
+    __syncthreads();
+    const double *v = buf + tid * kSeqPer;
     uint32_t emax = 0, any = 0;
-#pragma unroll
-    for (int u = 0; u < kSeqPer; ++u) v[u] = k0 + u < G ? ld_cg(part + k0 + u) : 0.0;
 #pragma unroll
     for (int u = 0; u < kSeqPer; ++u) {
         emax = max(emax, ((uint32_t)__double2hiint(v[u]) >> 20) & 0x7ffu);
@@ -190,36 +196,31 @@ static __device__ __noinline__ void seq_prepare(const double *part, int G, doubl
         emax = max(emax, sc->wmax[w]);
         any |= sc->wor[w];
     }
-    if (!any || emax < 128u || emax > 1900u || G > kSeqMax) {   // (uniform)
-        if (threadIdx.x == 0) {
+    if (!any || emax < 128u || emax > 1900u || G > kSeqMax) {   // (uniform in the group)
+        if (tid == 0) {
             sc->events = any ? -1 : 0;
             sc->qtot = 0;
         }
-        __syncthreads();
+        for (int i = 0; i < 4; ++i) __syncthreads();
         return;
     }
-    // exact prefixes in units of 2^(emax - 1073)
-    long long f[kSeqPer], fsum = 0;
-#pragma unroll
-    for (int u = 0; u < kSeqPer; ++u) {
-        const long long b = __double_as_longlong(v[u]);
+    // a value in units of 2^(emax - 1073)
+    auto fixed = [&](long long b) {
         const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
         const uint32_t sh = emax - e + 2;
         const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
-        const long long q = sh < 64u ? (long long)(m >> sh) : 0ll;
-        f[u] = b < 0 ? -q : q;
-        fsum += f[u];
-    }
-    long long P = seq_block_scan(fsum, sc->wsum) - fsum;
-    long long q[kSeqPer], qsum = 0;
-    uint32_t ev = 0;
-#pragma unroll
-    for (int u = 0; u < kSeqPer; ++u) {
-        const long long Pb = P, Pa = P + f[u];
-        P = Pa;
+        const long long f = sh < 64u ? (long long)(m >> sh) : 0ll;
+        return b < 0 ? -f : f;
+    };
+    long long fsum = 0;
+#pragma unroll 1
+    for (int u = 0; u < kSeqPer; ++u) fsum += fixed(__double_as_longlong(v[u]));
+    long long P = seq_block_scan(fsum, sc->wsum, warp) - fsum;   // the exact prefix before this thread's values
+    // a value's integers after the prefix Pb, Pb moved past it; true: an event
+    auto classify = [&](long long b, long long &Pb, long long &qu) {
+        const long long Pa = Pb + fixed(b);
         const unsigned long long ab = Pb < 0 ? -Pb : Pb, aa = Pa < 0 ? -Pa : Pa;
         const int pos = 63 - __clzll((long long)ab);            // -1 for 0
-        const long long b = __double_as_longlong(v[u]);
         const int e = (int)((uint32_t)(b >> 52) & 0x7ffu);
         const int d = pos + (int)emax - 50 - e;                 // log2 of the sum's unit over the value's
         const unsigned long long lo = (1ull << (pos & 63)) + kSeqBand, hi = (2ull << (pos & 63)) - kSeqBand;
@@ -230,18 +231,26 @@ static __device__ __noinline__ void seq_prepare(const double *part, int G, doubl
             r = m << 1;
         } else if (d < 54) {
             r = m >> d;
-            const unsigned long long rest = m & ((1ull << d) - 1);
-            const unsigned long long half = d ? 1ull << (d - 1) : 0ull;
-            if (d && rest == half) event = true;
-            if (rest > half) ++r;
+            const unsigned long long rest = d ? m << (64 - d) : 0ull;   // the bits below the unit, left-aligned
+            if (rest == 1ull << 63) event = true;
+            if (rest > 1ull << 63) ++r;
         }
-        if (v[u] == 0.0) {
+        if ((b << 1) == 0) {                                    // +-0
             event = false;
             r = 0;
         }
-        q[u] = event ? 0ll : (b < 0 ? -(long long)r : (long long)r);
-        qsum += q[u];
-        ev |= (event ? 1u : 0u) << u;
+        Pb = Pa;
+        qu = event ? 0ll : (b < 0 ? -(long long)r : (long long)r);
+        return event;
+    };
+    const long long P0 = P;
+    long long qsum = 0;
+    uint32_t ev = 0;
+#pragma unroll 1
+    for (int u = 0; u < kSeqPer; ++u) {
+        long long qu;
+        if (classify(__double_as_longlong(v[u]), P, qu)) ev |= 1u << u;
+        qsum += qu;
     }
     uint32_t cnt = __popc(ev);
     uint32_t pre = cnt;
@@ -252,28 +261,32 @@ static __device__ __noinline__ void seq_prepare(const double *part, int G, doubl
     }
     if (lane == 31) sc->wcnt[warp] = pre;
     __syncthreads();   // wsum of the first scan is consumed, wcnt visible
-    long long Q = seq_block_scan(qsum, sc->wsum);
+    long long Q = seq_block_scan(qsum, sc->wsum, warp);
     uint32_t at = pre - cnt, all = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
         if (w < warp) at += sc->wcnt[w];
         all += sc->wcnt[w];
     }
-    if (threadIdx.x == kBlock - 1) {
+    if (tid == kBlock - 1) {
         sc->qtot = Q;
         sc->events = all <= kSeqEvents ? (int32_t)all : -1;
     }
     Q -= qsum;
-#pragma unroll
-    for (int u = 0; u < kSeqPer; ++u) {
-        if ((ev >> u) & 1u) {
-            if (at < kSeqEvents) {
-                rec[at] = v[u];
-                rec[kSeqEvents + at] = __longlong_as_double(Q);
+    if (ev) {
+        P = P0;
+#pragma unroll 1
+        for (int u = 0; u < kSeqPer; ++u) {
+            long long qu;
+            if (classify(__double_as_longlong(v[u]), P, qu)) {
+                if (at < kSeqEvents) {
+                    rec[at] = v[u];
+                    rec[kSeqEvents + at] = __longlong_as_double(Q);
+                }
+                ++at;
             }
-            ++at;
+            Q += qu;
         }
-        Q += q[u];
     }
     __syncthreads();
 }
@@ -340,9 +353,10 @@ __device__ __forceinline__ bool grid_reduce(T (&acc)[NV], T *partials, int strid
         // block prepares each value's events, warp i adds up value i
         if constexpr (sizeof(T) == 8) {
             __shared__ SeqScratch sc[NV];
+            __shared__ double buf[kSeqMax];
             __syncthreads(); // the block sum's use of sm is over
 #pragma unroll 1
-            for (int i = 0; i < NV; ++i) seq_prepare(partials + i * stride, G, sm + i * 2 * kSeqEvents, &sc[i]);
+            for (int i = 0; i < NV; ++i) seq_prepare(partials + i * stride, G, buf, sm + i * 2 * kSeqEvents, &sc[i], threadIdx.x);
             const int warp = threadIdx.x >> 5;
             double run = 0.0;
             if (warp < NV) run = seq_finish(partials + warp * stride, G, sm + warp * 2 * kSeqEvents, &sc[warp]);

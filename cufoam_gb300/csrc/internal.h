@@ -198,6 +198,7 @@ struct Context {
     int coop_ok = -1;          // cooperative launches supported (-1: not asked yet)
     int cluster16_ok = 0;      // a 16-block cluster of k_persist fits (asked with coop_ok)
     DeviceBuffer persist;      // grid-persistent solves: block partials, barrier counter
+    DeviceBuffer persist_ref;  // ... in the reference order: the reference's block partials
 
     // scratch of the matrix builds (grow-only: a conversion after the first
     // allocates nothing) and the matrix of one-shot ldu2csr conversions
@@ -339,6 +340,9 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
 // steps in out_in->k
 void launch_persist_mixed(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1,
                           int max_len, const cf_controls &c, DevState *out, DevState *out_in);
+// ... and BiCG in the reference order (persist_ref.cu)
+bool persist_ref_usable(Context *ctx, int solver, bool sell);
+void launch_persist_ref(Context *ctx, const SolveArgs &A, const DevState &S, int l1, DevState *out);
 void persist_reset(Context *ctx);
 
 struct Batch;

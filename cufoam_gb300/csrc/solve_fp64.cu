@@ -751,7 +751,8 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     const Kernels kk = ref ? body_kernels(solver, sell) : fast_body_kernels(solver, fmt);
     SolveArgs *d_args = ctx->args.as<SolveArgs>();
     // the fast order over the SELL-32 copy: one launch
-    const bool persist = use_graph && !ref && persist_usable(ctx, solver, fmt, mixed);
+    const bool persist =
+        use_graph && (ref ? persist_ref_usable(ctx, solver, sell) : persist_usable(ctx, solver, fmt, mixed));
     if (use_graph && !mixed && !persist) {
         try {
             ge = loop_graph(ctx, kk, solver, CF_PREC_FP64, cap, ref, d_args, fmt);
@@ -770,7 +771,9 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     MixedResult mres;
     if (persist) {
         CF_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
-        if (mixed)
+        if (ref)
+            launch_persist_ref(ctx, A, S, l1, ctx->h_state);
+        else if (mixed)
             launch_persist_mixed(ctx, solver, fmt, A, S, l1, m->sell_max_len, c, ctx->h_state, ctx->h_state_in);
         else
             launch_persist(ctx, solver, fmt, A, S, l1, m->sell_max_len, ctx->h_state);
