@@ -20,19 +20,20 @@
 // rows -> here):
 //                4k          22k         219k        893k        2.1M rows
 //   CG step      7.0->5.4   16.6->7.9   28.8->12.8  43.9->27.0  72.1->55.7
-//   Jacobi step  4.7->2.3    8.3->3.4   15.3->7.4   28.8->21.3  53.5->45.9
-//   MRJacobi     8.2->5.1   16.0->7.2   24.0->12.3  38.8->29.3  70.4->59.1
+//   Jacobi step  4.7->2.3    8.3->3.4   15.3->7.4   28.8->20.6  53.5->43.9
+//   MRJacobi     8.2->5.1   16.0->7.2   24.0->12.3  38.8->25.8  70.4->53.9
 //   CG set-up     27->28     102->30     160->48     267->94     422->170
 // At 2.1M rows the FP64 unit bounds a CG step: 12 operations per row, 64
 // cycles per warp and sub-partition each, are 83,000 of its 115,000 cycles.
 // The arithmetic of a row and of an element
 // is the loop's: one FMA chain per row in entry order, one FMA per update;
-// only the order of the dot products' partial sums differs.
+// only how the dot products are summed differs.
 #include "persist.cuh"
 
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <type_traits>
 
 namespace cf {
 
@@ -52,6 +53,7 @@ struct PersistArgs {
     double tolerance, rel_tol, omega, diag_abs_min;
     int32_t max_steps, min_steps, hist_cap;
     int32_t abs_tol, l1, power_steps;
+    int32_t head;            // log2 of the rows per thread, and one (FixedDot)
     int32_t keep;            // the matrix fits in L2 beside the vectors: no evict-first hint
     PersistPlan plan;
 };
@@ -150,6 +152,13 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
     using Tr = PersistTraits<SOLVER>;
     // in a cluster the gathered vectors live in the blocks' shared memory
     constexpr bool DSM = SYNC::kCluster;
+    // Where the matrix streams, the FP64 unit bounds the passes (figures at
+    // FixedDot); with a row or two per thread, in shared memory, barriers do and
+    // FMA chains are the shorter code (MRJacobi step at 47k rows 8.4 us against
+    // 8.7).  CG and PCG keep them at all sizes: their counts over thousands of
+    // steps move with the rounding of the sums.
+    using Dot = std::conditional_t<LOCALM, PlainDot, FixedDot>;
+    const int head = P.head;
     __shared__ typename SYNC::Shared sh;
     __shared__ PersistState st;
     extern __shared__ __align__(16) double local_[];
@@ -454,20 +463,20 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
             double *gv = SOLVER == CF_MRJACOBI ? A.w[1] : A.r[0];
             {
                 const double *val = Tr::kScaledMatrix ? A.sc_val : A.s_val;
-                double acc[2] = {0.0, 0.0};
+                Dot acc[2];
                 for (int s = s_lo + warp; s < s_hi; s += nw) {
                     const int row = 32 * s + lane, i = row - base;
                     const double y = product(val, s, gather(SOLVER == CF_MRJACOBI ? own : rl, gv));
                     if (row < n) {
                         q[i] = y;
-                        acc[0] = fma_t(rl[i], y, acc[0]);
-                        acc[1] = fma_t(y, y, acc[1]);
+                        acc[0].add(rl[i], y, head);
+                        acc[1].add(y, y, head);
                     }
                 }
-                if (!gs.sum(acc, nullptr, [&](const double(&t)[2]) { st.omega = t[0] / t[1]; })) goto out;
+                if (!gs.sum(acc, nullptr, [&](const double(&t)[2]) { st.omega = t[0] / t[1]; }, head)) goto out;
             }
             const double alpha = st.omega;
-            double acc[1] = {0.0};
+            Dot acc[1];
             for (int s = s_lo + warp; s < s_hi; s += 2 * nw) {
                 double rv[2], xv[2], yv[2], dv[2], sv[2];
                 bool ok[2];
@@ -500,11 +509,11 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
                             if (!DSM) gv[row] = zi;
                             if (LOCALM) own[i] = zi;
                         }
-                        acc[0] = fma_t(ri, ri, acc[0]);
+                        acc[0].add(ri, ri, head);
                     }
             }
             if (!gs.sum(acc, A.abort_flag,
-                        [&](const double(&t)[1]) { persist_step(A, P, first_block, st, t[0], sh.stop != 0); }))
+                        [&](const double(&t)[1]) { persist_step(A, P, first_block, st, t[0], sh.stop != 0); }, head))
                 goto out;
         } else if constexpr (SOLVER == CF_JACOBI) {
             // one pass over A D^-1: the residual alternates between r[0] and r[1]
@@ -517,7 +526,7 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
             } else if constexpr (LOCALM) {
                 mine = rl;
             }
-            double acc[1] = {0.0};
+            Dot acc[1];
             for (int s = s_lo + warp; s < s_hi; s += nw) {
                 const int row = 32 * s + lane, i = row - base;
                 const double y = product(A.sc_val, s, gather(mine, rin));
@@ -527,11 +536,11 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
                     const double ri = fma_t(-1.0, y, r0);
                     rout[i] = ri;
                     if (LOCALM && !DSM) rl[i] = ri;
-                    acc[0] = fma_t(ri, ri, acc[0]);
+                    acc[0].add(ri, ri, head);
                 }
             }
             if (!gs.sum(acc, A.abort_flag,
-                        [&](const double(&t)[1]) { persist_step(A, P, first_block, st, t[0], sh.stop != 0); }))
+                        [&](const double(&t)[1]) { persist_step(A, P, first_block, st, t[0], sh.stop != 0); }, head))
                 goto out;
         } else {
             // Richardson: x += omega r; r = b - A x
@@ -541,18 +550,18 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
                 if (row < n) x[row - base] = fma_t(omega, rl[row - base], x[row - base]);
             }
             if (!gs.barrier()) goto out;
-            double acc[1] = {0.0};
+            Dot acc[1];
             for (int s = s_lo + warp; s < s_hi; s += nw) {
                 const int row = 32 * s + lane;
                 const double t = product(A.s_val, s, gather(x, xg));
                 if (row < n) {
                     const double ri = b[row] - t;
                     rl[row - base] = ri;
-                    acc[0] = fma_t(ri, ri, acc[0]);
+                    acc[0].add(ri, ri, head);
                 }
             }
             if (!gs.sum(acc, A.abort_flag,
-                        [&](const double(&t)[1]) { persist_step(A, P, first_block, st, t[0], sh.stop != 0); }))
+                        [&](const double(&t)[1]) { persist_step(A, P, first_block, st, t[0], sh.stop != 0); }, head))
                 goto out;
         }
     }
@@ -777,6 +786,9 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
     const double slots = (double)ns * 32.0 * max_len * 12.0, vectors = 40.0 * A.n;
     P.keep = slots + vectors < 0.95 * (double)ctx->l2_bytes ? 1 : 0;
     const void *kernel = persist_kernel(solver, scope, format);
+    const int slices_per_warp = ((ns + grid - 1) / grid + kPWarps - 1) / kPWarps;
+    P.head = 2;
+    while ((1 << (P.head - 1)) <= slices_per_warp) ++P.head;
     SolveArgs a = A;
     void *args[] = {&a, &P};
     launch_persist_kernel(ctx, kernel, scope == kScopeCluster, grid, (ns + grid - 1) / grid, smem, args);

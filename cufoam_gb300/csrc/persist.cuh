@@ -35,6 +35,48 @@ struct PersistGrid {
     int32_t *stop;         // [2] block 0's stop request (time limit), by parity
 };
 
+// (hi 2^44 + mid 2^22 + lo) 2^ex, rounded once: the limbs' sums of a warp, lo and
+// mid below 2^32, |hi| below 2^31.  ANY: a result that may leave the normal range
+// (the check costs a grid sum 0.1 us)
+template <bool ANY>
+__device__ __forceinline__ double fixed_to_double(uint32_t lo, uint32_t mid, int32_t hi, int ex)
+{
+    // value = t 2^44 + f, 0 <= f < 2^44, then sign and magnitude
+    unsigned long long f = (unsigned long long)lo + ((unsigned long long)mid << 22);
+    long long t = (long long)hi + (long long)(f >> 44);
+    f &= (1ull << 44) - 1;
+    const bool neg = t < 0;
+    if (neg) {
+        t = -t;
+        if (f) {
+            t -= 1;
+            f = (1ull << 44) - f;
+        }
+    }
+    unsigned long long m;
+    const int k = 64 - __clzll(t);           // bits of t (0 when it vanished)
+    if (k > 20) {
+        // more than 64 bits in all: drop the lowest k - 20, keeping a sticky bit
+        const int d = k - 20;
+        m = ((unsigned long long)t << (44 - d)) | (f >> d);
+        if (f & ((1ull << d) - 1)) m |= 1;
+        ex += d;
+    } else {
+        m = ((unsigned long long)t << 44) | f;
+    }
+    if (m == 0) return 0.0;
+    const int z = __clzll(m);
+    m <<= z;                                 // leading bit at 63
+    ex -= z;
+    // round to 53 bits, ties to even (a carry moves into the exponent)
+    const unsigned long long rest = m & 0x7ffull;
+    unsigned long long r = m >> 11;
+    if (rest > 0x400ull || (rest == 0x400ull && (r & 1))) ++r;
+    if (ANY && (ex < -1000 || ex > 900)) return scalbn((neg ? -1.0 : 1.0) * (double)r, ex + 11);
+    const unsigned long long out = ((unsigned long long)(ex + 63 + 1022) << 52) + r;
+    return __longlong_as_double((long long)(out | (neg ? 1ull << 63 : 0ull)));
+}
+
 // ---------------------------------------------------------------------------
 // Warp sum of doubles in fixed point: every lane gets the same bits.
 //
@@ -63,6 +105,8 @@ __device__ __forceinline__ double warp_sum_fixed(const double (&v)[K])
         double s = v[0];
 #pragma unroll
         for (int u = 1; u < K; ++u) s += v[u];
+        // all zero, as where a source is zero: MR step at 219k rows 15.9 -> 12.5 us
+        if (emax == 0u && !__any_sync(kFull, s != 0.0)) return 0.0;
 #pragma unroll
         for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
         return s;
@@ -83,41 +127,103 @@ __device__ __forceinline__ double warp_sum_fixed(const double (&v)[K])
     lo = __reduce_add_sync(kFull, lo);     // < 32 K 2^22
     mid = __reduce_add_sync(kFull, mid);
     hi = __reduce_add_sync(kFull, hi);     // |hi| < 32 K 2^19
-    // value = t 2^44 + f, 0 <= f < 2^44, then sign and magnitude
-    unsigned long long f = (unsigned long long)lo + ((unsigned long long)mid << 22);
-    long long t = (long long)hi + (long long)(f >> 44);
-    f &= (1ull << 44) - 1;
-    const bool neg = t < 0;
-    if (neg) {
-        t = -t;
-        if (f) {
-            t -= 1;
-            f = (1ull << 44) - f;
+    return fixed_to_double<false>(lo, mid, hi, (int)emax - 1023 - 62);   // unit: 2^(emax - 1023 - 52 - 10)
+}
+
+// ---------------------------------------------------------------------------
+// Dot products in fixed point.  A thread's sum of products is a 64-bit integer
+// on a grid that follows its largest product, each product the upper 64 bits of
+// the 106-bit product of the mantissas: exact to 2^-62, added without rounding
+// except for bits below 2^(head - 63) of the largest one (head: bits kept free
+// for the sum, log2 of the terms per thread).  FP64 FMA chains round every
+// addition to 2^-53 of the sum.
+//
+// Why: on GB300 an FP64 operation holds a sub-partition's FP64 unit for 64
+// cycles per warp, and the unit bounds the passes at large sizes; the integer
+// form is about 30 instructions on the other pipes, beside the FP64 work.
+// Measured, us per step at 0.3M / 0.9M / 2.1M rows (7-point), FMA chains -> here:
+// MR 15.1 -> 14.2 / 27.2 -> 24.5 / 55.4 -> 49.0, MRJacobi 15.6 -> 14.3 / 29.5 ->
+// 26.5 / 59.4 -> 53.9, Jacobi 9.7 -> 9.5 / 22.0 -> 21.1 / 46.8 -> 44.6.
+// ---------------------------------------------------------------------------
+struct FixedDot {
+    static constexpr int kEmpty = -100000, kFloat = 100000;
+    long long acc = 0;     // the sum in units of 2^(e + head - 2108); in kFloat mode a double's bits
+    int e = kEmpty;        // largest ea + eb (biased exponents) so far
+
+    __device__ __forceinline__ void add(double a, double b, int head)
+    {
+        const long long ab = __double_as_longlong(a), bb = __double_as_longlong(b);
+        const uint32_t ea = (uint32_t)(ab >> 52) & 0x7ffu, eb = (uint32_t)(bb >> 52) & 0x7ffu;
+        if (ea - 1u >= 0x7feu || eb - 1u >= 0x7feu || e == kFloat) {   // zero, subnormal, infinity or NaN
+            // a term 0, inline: whole regions of a vector may be zero
+            if ((2 * ab == 0 && eb < 0x7ffu) || (2 * bb == 0 && ea < 0x7ffu)) return;
+            *this = slow(*this, a, b, head);
+            return;
         }
+        const unsigned long long h = __umul64hi(((unsigned long long)ab << 11) | (1ull << 63),
+                                                ((unsigned long long)bb << 11) | (1ull << 63));
+        const int s = (int)(ea + eb);
+        if (s > e) {
+            const int d = s - e;
+            acc >>= d < 63 ? d : 63;
+            e = s;
+        }
+        const int sh = e - s + head;
+        const long long q = sh < 64 ? (long long)(h >> sh) : 0ll;
+        acc += (ab ^ bb) < 0 ? -q : q;
     }
-    // unit of the grid: 2^(emax - 1023 - 52 - 10)
-    int ex = (int)emax - 1023 - 62;
-    unsigned long long m;
-    const int k = 64 - __clzll(t);           // bits of t (0 when it vanished)
-    if (k > 20) {
-        // more than 64 bits in all: drop the lowest k - 20, keeping a sticky bit
-        const int d = k - 20;
-        m = ((unsigned long long)t << (44 - d)) | (f >> d);
-        if (f & ((1ull << d) - 1)) m |= 1;
-        ex += d;
-    } else {
-        m = ((unsigned long long)t << 44) | f;
+    __device__ double value(int head) const
+    {
+        if (e == kFloat) return __longlong_as_double(acc);
+        return e == kEmpty ? 0.0 : scalbn((double)acc, e + head - 2108);
     }
-    if (m == 0) return 0.0;
-    const int z = __clzll(m);
-    m <<= z;                                 // leading bit at 63
-    ex -= z;
-    // round to 53 bits, ties to even (a carry moves into the exponent)
-    const unsigned long long rest = m & 0x7ffull;
-    unsigned long long r = m >> 11;
-    if (rest > 0x400ull || (rest == 0x400ull && (r & 1))) ++r;
-    const unsigned long long out = ((unsigned long long)(ex + 63 + 1022) << 52) + r;
-    return __longlong_as_double((long long)(out | (neg ? 1ull << 63 : 0ull)));
+    // by value: the accumulator stays in registers around the call
+    static __device__ __noinline__ FixedDot slow(FixedDot f, double a, double b, int head)
+    {
+        const double t = fma_t(a, b, f.value(head));
+        f.acc = __double_as_longlong(t);
+        f.e = kFloat;
+        return f;
+    }
+    // the warp's sum, the same bits in every lane
+    __device__ __forceinline__ double warp_sum(int head) const
+    {
+        const int emax = __reduce_max_sync(kFull, e);
+        if (emax == kFloat) {   // (uniform)
+            double s = value(head);
+#pragma unroll
+            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+            return s;
+        }
+        if (emax == kEmpty) return 0.0;
+        const int d = emax - e;
+        const long long s = acc >> (d < 63 ? d : 63);
+        const uint32_t lo = __reduce_add_sync(kFull, (uint32_t)s & 0x3fffffu);
+        const uint32_t mid = __reduce_add_sync(kFull, (uint32_t)(s >> 22) & 0x3fffffu);
+        const int32_t hi = __reduce_add_sync(kFull, (int32_t)(s >> 44));
+        return fixed_to_double<true>(lo, mid, hi, emax + head - 2108);
+    }
+};
+
+// the same interface over an FP64 FMA chain
+struct PlainDot {
+    double v = 0.0;
+    __device__ __forceinline__ void add(double a, double b, int) { v = fma_t(a, b, v); }
+    __device__ __forceinline__ double warp_sum(int) const
+    {
+        const double t[1] = {v};
+        return warp_sum_fixed<1>(t);
+    }
+};
+__device__ __forceinline__ double warp_total(double v, int)
+{
+    const double t[1] = {v};
+    return warp_sum_fixed<1>(t);
+}
+template <class D>
+__device__ __forceinline__ double warp_total(const D &d, int head)
+{
+    return d.warp_sum(head);
 }
 
 // ---------------------------------------------------------------------------
@@ -155,14 +261,13 @@ template <int SLOTS> struct PersistShared {
 };
 
 // the block's sums of v in s (valid in warp 0)
-template <int NV>
-__device__ __forceinline__ void block_sum_fixed(const double (&v)[NV], PersistShared<1> *sh, double (&s)[NV])
+template <int NV, class T>
+__device__ __forceinline__ void block_sum_fixed(const T (&v)[NV], int head, PersistShared<1> *sh, double (&s)[NV])
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        const double t[1] = {v[i]};
-        const double x = warp_sum_fixed<1>(t);
+        const double x = warp_total(v[i], head);
         if (lane == 0) sh->w[i][warp] = x;
     }
     __syncthreads();
@@ -178,7 +283,8 @@ __device__ __forceinline__ void block_sum_fixed(const double (&v)[NV], PersistSh
 // ---------------------------------------------------------------------------
 // The two scopes a solve runs in.  Both offer
 //   barrier()  all blocks' writes before it are visible after it;
-//   sum(v, abort_flag, post)  sums over all blocks; thread 0 of every block
+//   sum(v, abort_flag, post)  sums over all blocks (doubles, or a dot product's
+//              accumulators with their `head`); thread 0 of every block
 //              runs post(totals) (the step logic, the same bits everywhere)
 //              before any thread goes on.  Also a barrier.  `abort_flag`,
 //              read by block 0, arrives in sh->stop.
@@ -226,13 +332,13 @@ struct GridSync {
         return !sh->fail;
     }
 
-    template <int NV, class Post>
-    __device__ __forceinline__ bool sum(const double (&v)[NV], const volatile int32_t *abort_flag, Post post)
+    template <int NV, class T, class Post>
+    __device__ __forceinline__ bool sum(const T (&v)[NV], const volatile int32_t *abort_flag, Post post, int head = 0)
     {
         const int lane = threadIdx.x & 31;
         const int G = gridDim.x;
         double s[NV];
-        block_sum_fixed(v, sh, s);
+        block_sum_fixed(v, head, sh, s);
         if (threadIdx.x < 32) {
             double *part = g.part + (size_t)(red & 1) * kPMaxNV * kPMaxGrid;
             if (lane == 0) {
@@ -323,15 +429,14 @@ struct ClusterSync {
     // Every warp stores its sum into every block's shared memory; after the
     // cluster barrier warp 0 of each block adds up what it has (no second
     // stage, no remote loads).
-    template <int NV, class Post>
-    __device__ __forceinline__ bool sum(const double (&v)[NV], const volatile int32_t *abort_flag, Post post)
+    template <int NV, class T, class Post>
+    __device__ __forceinline__ bool sum(const T (&v)[NV], const volatile int32_t *abort_flag, Post post, int head = 0)
     {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
         const int par = red & 1;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            const double t[1] = {v[i]};
-            const double x = warp_sum_fixed<1>(t);
+            const double x = warp_total(v[i], head);
             if (lane < (int)n)
                 asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote(&sh->slot[par][i][me * nw + warp],
                                                                               (uint32_t)lane)),
