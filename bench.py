@@ -621,10 +621,8 @@ def run_ours(args):
     bytes_total = sum_over_ranks(sum(solve_bytes(mat_it, mat_csr, n, k) for k in its), dist, dev)
     csr_equiv = sum_over_ranks(sum(solve_bytes(mat_csr, mat_csr, n, k) for k in its), dist, dev)
     value = bytes_total / (ms * 1e-3) / 1e9
-    # nf_sum, nf_dist, res_init, flush, clear, and 3 kernels per step in
-    # passes of 8 steps (the steps of the last pass past convergence return
-    # at once)
-    launches = sum(5 + 3 * 8 * ((k + 7) // 8) for k in its)
+    # one cooperative launch (k_persist) per solve
+    launches = len(its)
 
     # ---- e2e through the public API with pinned host buffers -------------
     # What the plugin does per cuFoamCG::solve in a running case (its device
@@ -673,7 +671,9 @@ def run_ours(args):
     f_dt = time.perf_counter() - t0
     m_e2e.close()
 
-    # ---- dominant kernel: per-launch time with CUDA events (profiled solve)
+    # ---- dominant kernel: k_persist is the whole timed solve; the kernels of
+    # the host-driven loop (the path with useGraph 0), timed one by one with
+    # CUDA events, for comparison
     psi.zero_()
     prof = cf.cuFoamCG("p", M, {"tolerance": TOL, "maxIter": MAX_ITER,
                                 "profileKernels": 1})
@@ -772,14 +772,14 @@ def run_ours(args):
                                "value": round(solve_bytes(mat_it, mat_csr, n, f_its) / f_dt / 1e9, 2),
                                "path": "a new mesh: addressing upload, device ldu2csr and "
                                        "SELL-32 build, then the solve"}},
-        "roofline": {"bound": "hbm", "kernel": "k_f_cg_spmv", "achieved": round(k1_gbs, 1),
-                     "peak": peak, "unit": "GB/s", "frac": round(k1_gbs / peak, 4),
+        "roofline": {"bound": "hbm", "kernel": "k_persist (CG)", "achieved": round(value / world, 1),
+                     "peak": peak, "unit": "GB/s", "frac": round(value / world / peak, 4),
                      "peak_source": peak_kind,
-                     "bytes_per_launch": k1_bytes,
-                     "us_per_launch": round(k1_ms * 1e3, 2),
-                     "traffic": profiled_traffic("k_f_cg_spmv_sell_poisson128.md"),
-                     # the co-binding unit: 8 FP64 operations per row (ncu, same summary)
-                     "fp64_pipe_active": profiled_value("k_f_cg_spmv_sell_poisson128.md",
+                     "bytes_per_launch": int(bytes_total / world / len(its)),
+                     "us_per_launch": round(1e3 * ms / len(its), 2),
+                     "traffic": profiled_traffic("k_persist_cg_poisson128.md"),
+                     # the co-binding unit: 12 FP64 operations per row and step (ncu, same summary)
+                     "fp64_pipe_active": profiled_value("k_persist_cg_poisson128.md",
                                                         "fp64_pipe_active_frac"),
                      # the plain SpMV y = A x (cf_spmv_async, back to back)
                      "spmv_us": round(spmv_ms * 1e3, 2), "spmv_gbs": round(spmv_gbs, 1),
@@ -787,7 +787,8 @@ def run_ours(args):
                      # the same product over the one-byte column codes (9 B per entry)
                      "spmv_c8_us": round(spmv_c8_ms * 1e3, 2), "spmv_c8_gbs": round(spmv_c8_gbs, 1),
                      "spmv_c8_frac": round(spmv_c8_gbs / peak, 4),
-                     # the other two kernels of the CG step, CUDA events per launch
+                     # the three kernels of the host-driven loop, CUDA events per launch
+                     "cg_spmv_us": round(k1_ms * 1e3, 2), "cg_spmv_gbs": round(k1_gbs, 1),
                      "cg_update_us": round(k2_ms * 1e3, 2), "cg_update_gbs": round(k2_gbs, 1),
                      "cg_prep_us": round(k0_ms * 1e3, 2), "cg_prep_gbs": round(k0_gbs, 1),
                      "cg_step_us": round(1e3 * ms / args.steps / max(iters, 1), 2)},
@@ -950,8 +951,8 @@ def batched_vs_sequential(ctx, device, n_systems: int = 512, tol: float = 1e-8,
 
 
 def run_profile(args):
-    """A short run for ncu: the same 128^3 CG solve with host-driven
-    launches (every kernel a separate launch), then five plain SpMVs over the
+    """A short run for ncu: the 128^3 CG solve as one launch (k_persist) and
+    with host-driven launches (every kernel a separate launch), then five plain SpMVs over the
     one-byte column codes (k_spmv_sell<1>) and five over the 32-bit columns
     (k_spmv_sell<0>)."""
     import torch
@@ -963,10 +964,11 @@ def run_profile(args):
     M = cf.LduMatrix.from_ldu(L, ctx)
     src = torch.from_numpy(b).cuda()
     psi = torch.zeros(L.n, dtype=torch.float64, device="cuda")
-    s = cf.cuFoamCG("p", M, {"tolerance": TOL, "maxIter": MAX_ITER, "useGraph": 0})
-    for _ in range(args.steps):
-        psi.zero_()
-        perf = s.solve(psi, src)
+    for graph in (1, 0):
+        s = cf.cuFoamCG("p", M, {"tolerance": TOL, "maxIter": MAX_ITER, "useGraph": graph})
+        for _ in range(args.steps):
+            psi.zero_()
+            perf = s.solve(psi, src)
     x = torch.from_numpy(W.uniform(5, L.n)).cuda()
     for fmt in ("auto", "sell"):
         M.set_format(fmt)

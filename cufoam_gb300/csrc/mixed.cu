@@ -11,6 +11,8 @@
 // tolerance.
 // FP32 halves the bytes of every vector stream and cuts the matrix from 12
 // to 8 bytes per entry.
+// These are the host-driven loop's kernels (CSR matrices, useGraph 0, profiled
+// solves); over SELL-32 the whole refinement is one launch, persist_mixed.cu.
 #include "solver_common.cuh"
 
 #include <algorithm>

@@ -1,4 +1,6 @@
-// solve_fast.cu -- the default (fast) FP64 iteration kernels.
+// solve_fast.cu -- the fast-order FP64 iteration kernels of the multi-kernel
+// loop: CSR matrices, host-driven and profiled solves, BiCG in the fast order
+// (over SELL-32 a solve is otherwise one launch, persist.cu).
 //
 // GB300 executes FP64 at 2 FMA per cycle per SM (ncu:
 // sm__sass_thread_inst_executed_op_dfma peak), so a fused kernel that forms
