@@ -1,0 +1,39 @@
+"""Rules of the device code that no run can show reliably, checked in the
+source.
+
+A block of a cluster may only touch a peer's shared memory once that peer
+runs; nothing but a cluster barrier says so (CUDA programming guide,
+distributed shared memory).  The sums of the single-cluster solves store into
+every block before their own barrier, so the scope's constructor has to hold
+one, after the block's own initialisation."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cufoam_gb300", "csrc")
+
+
+def _body(text, start):
+    """The brace-balanced body that opens at or after `start`."""
+    i = text.index("{", start)
+    depth, j = 0, i
+    while True:
+        depth += {"{": 1, "}": -1}.get(text[j], 0)
+        j += 1
+        if depth == 0:
+            return text[i:j]
+
+
+def _code(name):
+    text = open(os.path.join(CSRC, name)).read()
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
+
+
+def test_cluster_scope_waits_for_its_blocks_before_the_first_remote_store():
+    text = _code("persist.cuh")
+    scope = _body(text, text.index("struct ClusterSync"))
+    ctor = _body(scope, re.search(r"ClusterSync\(const PersistGrid &[^)]*\)[^{]*", scope).end() - 1)
+    assert "st.shared::cluster" not in ctor
+    last = [line.strip() for line in ctor.strip("{} \n").splitlines() if line.strip()][-1]
+    assert last == "barrier();", last
+    barrier = _body(scope, scope.index("bool barrier()"))
+    assert barrier.index("barrier.cluster.arrive.release") < barrier.index("barrier.cluster.wait.acquire")
