@@ -96,6 +96,11 @@ class Context:
         self.check(self._lib.cf_context_set_stream(self._h, C.c_void_p(raw) if raw else None),
                    "set_stream")
 
+    def set_wait_limit(self, polls: int = 0) -> None:
+        """Polls (about half a microsecond each) a block of a solve waits for
+        the others before the solve ends with CF_TIMEOUT; 0: the default."""
+        self.check(self._lib.cf_context_set_wait_limit(self._h, int(polls)), "set_wait_limit")
+
     def device_info(self) -> dict:
         info = _capi.cf_device_info()
         self.check(self._lib.cf_device_query(self._h, C.byref(info)), "device_query")

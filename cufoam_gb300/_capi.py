@@ -117,6 +117,7 @@ def load(build_if_missing: bool = True):
         "cf_context_create": (C.c_int32, [C.c_int32, C.POINTER(P)]),
         "cf_context_destroy": (None, [P]),
         "cf_context_set_stream": (C.c_int32, [P, P]),
+        "cf_context_set_wait_limit": (C.c_int32, [P, C.c_int32]),
         "cf_context_last_error": (C.c_char_p, [P]),
         "cf_device_query": (C.c_int32, [P, C.POINTER(cf_device_info)]),
         "cf_matrix_create_ldu": (C.c_int32, [P, C.POINTER(cf_ldu_view), C.POINTER(P)]),

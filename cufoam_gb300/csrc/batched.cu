@@ -113,6 +113,7 @@ struct BatchArgs {
     uint32_t *arrivals;      // [n_systems]
     double *partials;        // [2][3 kBatchMaxR][blocks]
     int32_t *gave_up;
+    int32_t poll_limit;
 };
 
 struct NoPost {
@@ -205,7 +206,7 @@ struct ClusterScope {
 
 // A group of co-resident blocks (a cooperative launch) with a counter in
 // global memory: its blocks arrive with release, wait with acquire, and each
-// sums the group's partials in rank order.  A wait that gives up (kPollLimit)
+// sums the group's partials in rank order.  A wait that gives up (poll_limit)
 // makes every further sum NaN, which ends the solve.
 struct GroupScope {
     // (48 systems, 662k rows: 1 component 1,018 us with one entry per batch,
@@ -214,6 +215,7 @@ struct GroupScope {
     uint32_t *count;
     double *part;
     int32_t *gave_up;
+    int poll_limit;
     int system, me, n, first, stride;
     uint32_t epoch, red;
     bool fail, taken;
@@ -227,6 +229,7 @@ struct GroupScope {
         count = a.arrivals + system;
         part = a.partials;
         gave_up = a.gave_up;
+        poll_limit = a.poll_limit;
         stride = gridDim.x;
         epoch = red = 0;
         fail = taken = false;
@@ -239,7 +242,7 @@ struct GroupScope {
         const uint32_t want = (epoch + 1) * (uint32_t)n;
         int k = 0;
         while ((int32_t)(ld_acquire(count) - want) < 0)
-            if (++k > kPollLimit) {
+            if (++k > poll_limit) {
                 *gave_up = 1;
                 fail = true;
                 break;
@@ -1158,6 +1161,7 @@ static bool launch_groups(Context *ctx, Batch *B, BatchArgs &a, int nrhs, bool m
     a.partials = reinterpret_cast<double *>(base + tb);
     a.arrivals = reinterpret_cast<uint32_t *>(base + tb + pb);
     a.gave_up = reinterpret_cast<int32_t *>(a.arrivals + S);
+    a.poll_limit = ctx->poll_limit;
     // (a pageable source: staged when the call returns)
     CF_CUDA(cudaMemcpyAsync(base, table.data(), sizeof(int4) * (size_t)grid, cudaMemcpyHostToDevice, s));
     CF_CUDA(cudaMemsetAsync(a.arrivals, 0, sizeof(uint32_t) * ((size_t)S + 4), s));

@@ -387,6 +387,15 @@ cf_status cf_context_set_stream(cf_context *ctx, void *stream)
     });
 }
 
+cf_status cf_context_set_wait_limit(cf_context *ctx, int32_t polls)
+{
+    if (!ctx) return CF_BAD_INPUT;
+    return guarded(ctx, [&] {
+        cf::require(polls >= 0, CF_BAD_INPUT, "the wait limit must not be negative");
+        ctx->impl->poll_limit = polls > 0 ? polls : cf::kPollLimit;
+    });
+}
+
 const char *cf_context_last_error(const cf_context *ctx)
 {
     return ctx ? ctx->impl->last_error.c_str() : "null context";

@@ -167,6 +167,10 @@ struct GraphEntry {
     bool pdl = false;
 };
 
+// polls of a wait between the blocks of a solve before it gives up (about half
+// a microsecond each: 17 s); the solve then ends with CF_TIMEOUT
+constexpr int32_t kPollLimit = 1 << 25;
+
 struct Context {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -196,6 +200,7 @@ struct Context {
     int grid_cap = 0;
     int small_cg_ok = -1;      // 16-CTA clusters schedulable (-1: not asked yet)
     int coop_ok = -1;          // cooperative launches supported (-1: not asked yet)
+    int32_t poll_limit = kPollLimit; // polls of a wait between blocks (cf_context_set_wait_limit)
     int cluster16_ok = 0;      // a 16-block cluster of k_persist fits (asked with coop_ok)
     DeviceBuffer persist;      // grid-persistent solves: block partials, barrier counter
     DeviceBuffer persist_ref;  // ... in the reference order: the reference's block partials

@@ -162,6 +162,10 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
     __shared__ typename SYNC::Shared sh;
     __shared__ PersistState st;
     extern __shared__ __align__(16) double local_[];
+    if (threadIdx.x == 0) {
+        st = PersistState{};
+        st.k = -1;   // (no residual yet)
+    }
     SYNC gs(P.g, &sh);
 
     const int n = A.n, ns = A.n_slices;
@@ -591,9 +595,9 @@ out:
         o->omega = st.omega;
         o->lambda_max = st.lambda;
         o->k = st.k;
-        o->status = sh.fail ? CF_TIMEOUT : st.status;
-        o->flags = sh.fail;
+        o->status = st.status;
     }
+    report_fail(sh.fail, P.out);
     gs.leave();
 }
 
@@ -673,6 +677,7 @@ PersistGrid persist_grid(Context *ctx)
     g.part = ctx->persist.as<double>();
     g.count = reinterpret_cast<uint32_t *>(static_cast<char *>(ctx->persist.ptr) + part);
     g.stop = reinterpret_cast<int32_t *>(g.count + 4);
+    g.poll_limit = ctx->poll_limit;
     return g;
 }
 
@@ -799,6 +804,7 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
     while ((1 << (P.head - 1)) <= slices_per_warp) ++P.head;
     SolveArgs a = A;
     void *args[] = {&a, &P};
+    out->flags = 0;   // (S may be *out: read above)
     launch_persist_kernel(ctx, kernel, scope == kScopeCluster, grid, (ns + grid - 1) / grid, smem, args);
 }
 

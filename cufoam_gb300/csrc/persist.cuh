@@ -22,17 +22,11 @@ constexpr int kPWarps = kPBlock / 32;
 constexpr int kPMaxNV = 4;
 constexpr int kPMaxGrid = 192;         // blocks (SMs) the partial sums are sized for
 
-// polls of the grid barrier before a block gives up (about half a
-// microsecond each: tens of seconds); the solve then ends with CF_TIMEOUT
-#ifndef CF_PERSIST_POLL_LIMIT
-#define CF_PERSIST_POLL_LIMIT (1 << 25)
-#endif
-constexpr int kPollLimit = CF_PERSIST_POLL_LIMIT;
-
 struct PersistGrid {
     uint32_t *count;       // arrivals since the launch (0 between launches)
     double *part;          // [2][kPMaxNV][kPMaxGrid] block partials, by parity
     int32_t *stop;         // [2] block 0's stop request (time limit), by parity
+    int32_t poll_limit;    // polls of a wait before its block gives up
 };
 
 // (hi 2^44 + mid 2^22 + lo) 2^ex, rounded once: the limbs' sums of a warp, lo and
@@ -256,7 +250,7 @@ template <int SLOTS> struct PersistShared {
     double w[kPMaxNV][kPWarps];
     double slot[2][kPMaxNV][SLOTS];
     int32_t slot_stop[2];
-    int32_t fail;              // the grid barrier gave up
+    int32_t fail;              // this block gave up waiting at the grid barrier
     int32_t stop;              // block 0 asked for an early end
 };
 
@@ -288,7 +282,10 @@ __device__ __forceinline__ void block_sum_fixed(const T (&v)[NV], int head, Pers
 //              runs post(totals) (the step logic, the same bits everywhere)
 //              before any thread goes on.  Also a barrier.  `abort_flag`,
 //              read by block 0, arrives in sh->stop.
-// and return false when a wait gave up (grid only).
+// and return false when a wait gave up (grid only).  The block then leaves at
+// once, without its share of the answer, while block 0 may have seen every
+// arrival: each block reports its own failure (report_fail), and any of them
+// makes the solve a CF_TIMEOUT.
 // ---------------------------------------------------------------------------
 struct GridSync {
     static constexpr bool kCluster = false;
@@ -317,7 +314,7 @@ struct GridSync {
         const uint32_t want = (epoch + 1) * gridDim.x;
         int n = 0;
         while ((int32_t)(ld_acquire(g.count) - want) < 0)
-            if (++n > kPollLimit) {
+            if (++n > g.poll_limit) {
                 sh->fail = 1;
                 break;
             }
@@ -473,6 +470,12 @@ struct ClusterSync {
     // no block leaves while a peer may still read its shared memory
     __device__ __forceinline__ void leave() { barrier(); }
 };
+
+// out->flags (zeroed by the host before the launch): some block gave up waiting
+__device__ __forceinline__ void report_fail(int32_t fail, DevState *out)
+{
+    if (threadIdx.x == 0 && fail) out->flags = 1;
+}
 
 // a / b with the correctly rounded reciprocal rb = 1 / b at hand: the
 // rounding of a division (Markstein: one residual step from a correctly

@@ -85,6 +85,10 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
     __shared__ typename SYNC::Shared sh;
     __shared__ MixedState st;
     extern __shared__ __align__(16) unsigned char smem_[];
+    if (threadIdx.x == 0) {
+        st = MixedState{};
+        st.k = -1;   // (no residual yet)
+    }
     SYNC gs(P.g, &sh);
 
     const int n = A.n, ns = A.n_slices;
@@ -562,10 +566,10 @@ out:
         o->norm = st.norm;
         o->omega = 0.0;
         o->k = st.k;
-        o->status = sh.fail || st.stop ? CF_TIMEOUT : st.result;
-        o->flags = sh.fail;
+        o->status = st.stop ? CF_TIMEOUT : st.result;
         P.out_in->k = (int32_t)(st.total < INT_MAX ? st.total : INT_MAX);
     }
+    report_fail(sh.fail, P.out);
     gs.leave();
 }
 
@@ -669,6 +673,7 @@ void launch_persist_mixed(Context *ctx, int solver, int format, const SolveArgs 
                                          : mixed_pick<kMxBCS>(scope, format);
     SolveArgs a = A;
     void *args[] = {&a, &P};
+    out->flags = 0;   // (S may be *out: read above)
     launch_persist_kernel(ctx, kernel, scope == kScopeCluster, grid, (ns + grid - 1) / grid, smem, args);
 }
 

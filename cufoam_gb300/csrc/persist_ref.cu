@@ -81,6 +81,10 @@ __global__ void __launch_bounds__(kRefBlock, 1)
     extern __shared__ __align__(16) unsigned char smem_[];
     RefShared &sh = *reinterpret_cast<RefShared *>(smem_);
     __shared__ RefState st;
+    if (threadIdx.x == 0) {
+        st = RefState{};
+        st.k = -1;   // (no residual yet)
+    }
     GridSync gs(P.g, &sh.sync);
     const int n = A.n, G = P.ref_grid;
     const int tid = threadIdx.x & (kBlock - 1), group = threadIdx.x / kBlock;
@@ -363,9 +367,9 @@ out:
         o->norm = st.norm;
         o->omega = 0.0;
         o->k = st.k;
-        o->status = sh.sync.fail ? CF_TIMEOUT : st.status;
-        o->flags = sh.sync.fail;
+        o->status = st.status;
     }
+    report_fail(sh.sync.fail, P.out);
     gs.leave();
 }
 
@@ -395,6 +399,7 @@ void launch_persist_ref(Context *ctx, const SolveArgs &A, const DevState &S, int
     P.ref_grid = ctx->ref_grid;
     SolveArgs a = A;
     void *args[] = {&a, &P};
+    out->flags = 0;   // (S may be *out: read above)
     launch_persist_kernel(ctx, (const void *)k_persist_bicg, false, ctx->sm_count, kRefBlock / 32, sizeof(RefShared), args);
 }
 

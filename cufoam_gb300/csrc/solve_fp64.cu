@@ -900,11 +900,14 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
         }
     }
     CF_CUDA(cudaStreamSynchronize(ctx->stream));
-    const DevState R = *ctx->h_state;
-    if (persist && R.flags) persist_reset(ctx);
+    DevState R = *ctx->h_state;
+    if (persist && R.flags) {   // a block gave up waiting: psi is not an answer, whatever block 0 saw
+        persist_reset(ctx);
+        R.status = CF_TIMEOUT;
+    }
     if (persist && mixed) {
         mres.inner_iterations = ctx->h_state_in->k;
-        mres.outer = R.k;
+        mres.outer = std::max(R.k, 0);
         mres.status = R.status;
     }
     if (c.memory == CF_MEM_HOST) {
@@ -912,7 +915,7 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     }
     int hist_len = 0;
     if (want_hist) {
-        hist_len = std::min(R.k + 1, hist_cap);
+        hist_len = std::min(R.k + 1, hist_cap);   // (R.k is -1 when block 0 gave up before a residual)
         if (hist_time) {
             std::vector<unsigned long long> t((size_t)hist_len);
             download(ctx, t.data(), A.hist_t, sizeof(unsigned long long) * (size_t)hist_len, CF_MEM_HOST);
@@ -933,7 +936,7 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
         perf->initial_residual = R.norm0 / R.nf;
         perf->final_residual = R.norm / R.nf;
         perf->omega = (solver == CF_RICHARDSON) ? R.omega : 0.0;
-        perf->n_iterations = mixed ? mres.inner_iterations : R.k;
+        perf->n_iterations = mixed ? mres.inner_iterations : std::max(R.k, 0);
         perf->n_outer = mixed ? mres.outer : 0;
         perf->status = mixed ? mres.status : R.status;
         perf->history_length = hist_len;

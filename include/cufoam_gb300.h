@@ -207,6 +207,10 @@ void cf_context_destroy(cf_context *ctx);
  * keeps alive; cudaStreamLegacy and cudaStreamPerThread are accepted), or on
  * a private non-blocking stream of the library when it is NULL. */
 cf_status cf_context_set_stream(cf_context *ctx, void *cuda_stream);
+/* How often a block of a solve polls (about half a microsecond each) for the
+ * others before it gives up; the solve then ends with CF_TIMEOUT, psi is
+ * undefined, and the context stays usable.  0 restores the default, 2^25. */
+cf_status cf_context_set_wait_limit(cf_context *ctx, int32_t polls);
 const char *cf_context_last_error(const cf_context *ctx);
 cf_status cf_device_query(cf_context *ctx, cf_device_info *out);
 
