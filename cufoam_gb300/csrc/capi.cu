@@ -68,6 +68,11 @@ void DeviceBuffer::release()
     borrowed = false;
 }
 
+void raise_smem_limit(const void *kernel, size_t bytes)
+{
+    CF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 int Context::fast_grid(const void *kernel, size_t dyn_smem) const
 {
     int per_sm = 0;

@@ -302,7 +302,13 @@ void matrix_ensure_dmin(Matrix *m);
 void ldu2csr_into(Context *ctx, const cf_ldu_view &v, int32_t *ro, int32_t *col,
                   double *val, int memory);
 
+// entries a warp of the CSR passes stages: kStageCapMax, fewer for short rows, 0: unstaged
+constexpr int kStageCapMax = 1024;
 int stage_cap_for(const Matrix *m);
+// Raises a kernel's dynamic shared memory limit.  The limit belongs to the
+// function on the device and is shared by all contexts and threads, so every
+// caller of one kernel passes the same number, the largest it launches with.
+void raise_smem_limit(const void *kernel, size_t bytes);
 bool matrix_ensure_sell(Matrix *m, bool transpose, bool fp32);
 Matrix *matrix_from_csr(Context *ctx, int n, int64_t nnz, const int32_t *ro, const int32_t *col,
                         const double *val);

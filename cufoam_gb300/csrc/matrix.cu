@@ -1195,7 +1195,7 @@ int stage_cap_for(const Matrix *m)
 {
     // stage a warp's rows when they fit a modest per-warp buffer
     if (m->max_chunk <= 256) return 256;
-    if (m->max_chunk <= 1024) return 1024;
+    if (m->max_chunk <= kStageCapMax) return kStageCapMax;
     return 0;
 }
 
@@ -1227,8 +1227,7 @@ void spmv(Matrix *m, bool transpose, const double *x, double *y, bool ref_order)
     const int cap = stage_cap_for(m);
     const size_t smem = cap > 0 ? kWarps * stage_bytes_per_warp<double>(cap) : 0;
     auto kern = ref_order ? k_spmv : k_spmv_fast;
-    if (smem > 48 * 1024)
-        CF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) raise_smem_limit((const void *)kern, kWarps * stage_bytes_per_warp<double>(kStageCapMax));
     const int g = ctx->fast_grid((const void *)kern, smem);
     kern<<<g, kBlock, smem, ctx->stream>>>(m->n, cap, m->ro.as<int32_t>(), m->col.as<int32_t>(),
                                            transpose ? m->valT.as<double>() : m->val.as<double>(), x, y);

@@ -684,8 +684,7 @@ PersistGrid persist_grid(Context *ctx)
 void launch_persist_kernel(Context *ctx, const void *kernel, bool cluster, int grid, int slices_per_block,
                            size_t smem, void **args)
 {
-    if (smem > 8 * 1024)   // (with the static part above the default limit of 48 KB)
-        CF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    raise_smem_limit(kernel, persist_smem_limit(cluster));
     const int warps = std::max(4, std::min(kPWarps, (slices_per_block + 3) / 4 * 4));
     if (!cluster) {
         CF_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(32 * warps), args, smem, ctx->stream));

@@ -538,6 +538,14 @@ enum { kScopeGrid = 0, kScopeGridLocal = 1, kScopeCluster = 2 };
 #ifndef CF_PERSIST_VEC_BYTES
 #define CF_PERSIST_VEC_BYTES (144 * 1024)
 #endif
+// The dynamic limit of a persistent kernel: one value for all its solves.  (A
+// kernel's limit belongs to the function on the device, not to a context: a
+// solve that set its own size could lower it under another thread's launch.)
+constexpr size_t persist_smem_limit(bool cluster)
+{
+    const size_t most = CF_PERSIST_VEC_BYTES > CF_PERSIST_LOCAL_BYTES ? CF_PERSIST_VEC_BYTES : CF_PERSIST_LOCAL_BYTES;
+    return cluster ? CF_PERSIST_LOCAL_BYTES - sizeof(ClusterSync::Shared) : most;
+}
 // the barrier counter and partial sums of the context
 PersistGrid persist_grid(Context *ctx);
 // `grid` blocks, one warp per slice up to 32, cooperative or as one cluster

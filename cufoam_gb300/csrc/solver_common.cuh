@@ -291,7 +291,7 @@ static Launch launch_cfg(Context *ctx, const void *kern, bool is_spmv, int cap, 
     Launch l;
     l.smem = (is_spmv && cap > 0) ? kWarps * ((size_t)(cap + 8) * (value_bytes + sizeof(int32_t))) : 0;
     if (l.smem > 24 * 1024)   // (with the static part above the default limit of 48 KB)
-        CF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem));
+        raise_smem_limit(kern, kWarps * ((size_t)(kStageCapMax + 8) * (value_bytes + sizeof(int32_t))));
     l.grid = ref_order ? ctx->ref_grid : ctx->fast_grid(kern, l.smem);
     return l;
 }
