@@ -201,7 +201,7 @@ struct Context {
     int small_cg_ok = -1;      // 16-CTA clusters schedulable (-1: not asked yet)
     int coop_ok = -1;          // cooperative launches supported (-1: not asked yet)
     int32_t poll_limit = kPollLimit; // polls of a wait between blocks (cf_context_set_wait_limit)
-    int cluster16_ok = 0;      // a 16-block cluster of k_persist fits (asked with coop_ok)
+    std::map<const void *, bool> cluster_fits; // per single-cluster kernel asked about: persist_cluster_fits
     DeviceBuffer persist;      // grid-persistent solves: block partials, barrier counter
     DeviceBuffer persist_ref;  // ... in the reference order: the reference's block partials
 

@@ -644,26 +644,34 @@ bool persist_usable(Context *ctx, int solver, int format, bool mixed)
             coop = 0;
         }
         ctx->coop_ok = coop;
-        // a 16-block cluster of the single-cluster scope
-        const void *k = persist_kernel(CF_CG, kScopeCluster, kSell);
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 16;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.blockDim = dim3(ClusterSync::kThreads);
-        cfg.gridDim = dim3(16);
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int nclusters = 0;
-        const bool ok =
-            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&nclusters, k, &cfg) == cudaSuccess && nclusters >= 1;
-        cudaGetLastError();
-        ctx->cluster16_ok = ok ? 1 : 0;
     }
     return ctx->coop_ok == 1;
+}
+
+// Asked for the kernel to be launched, with its own registers and the most
+// dynamic shared memory it is given, once per context: where the answer is no,
+// its solves run on the grid.
+bool persist_cluster_fits(Context *ctx, const void *kernel)
+{
+    const auto seen = ctx->cluster_fits.find(kernel);
+    if (seen != ctx->cluster_fits.end()) return seen->second;
+    raise_smem_limit(kernel, persist_smem_limit(true));
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kPClusterMax;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.blockDim = dim3(ClusterSync::kThreads);
+    cfg.gridDim = dim3(kPClusterMax);
+    cfg.dynamicSmemBytes = persist_smem_limit(true);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters >= 1;
+    cudaGetLastError();
+    return ctx->cluster_fits[kernel] = ok;
 }
 
 PersistGrid persist_grid(Context *ctx)
@@ -756,7 +764,8 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
 
     int scope = kScopeGrid, grid = 1;
     size_t smem = 0;
-    if (A.n <= CF_PERSIST_CLUSTER_ROWS && !A.has_long && ctx->cluster16_ok == 1) {
+    if (A.n <= CF_PERSIST_CLUSTER_ROWS && !A.has_long &&
+        persist_cluster_fits(ctx, persist_kernel(solver, kScopeCluster, format))) {
         // one warp per sub-partition and block before another block is added
         grid = 1;
         while (grid < 16 && 4 * grid < ns) grid <<= 1;

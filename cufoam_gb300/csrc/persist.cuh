@@ -546,6 +546,8 @@ constexpr size_t persist_smem_limit(bool cluster)
     const size_t most = CF_PERSIST_VEC_BYTES > CF_PERSIST_LOCAL_BYTES ? CF_PERSIST_VEC_BYTES : CF_PERSIST_LOCAL_BYTES;
     return cluster ? CF_PERSIST_LOCAL_BYTES - sizeof(ClusterSync::Shared) : most;
 }
+// whether a cluster of kPClusterMax blocks of a single-cluster kernel can be resident
+bool persist_cluster_fits(Context *ctx, const void *kernel);
 // the barrier counter and partial sums of the context
 PersistGrid persist_grid(Context *ctx);
 // `grid` blocks, one warp per slice up to 32, cooperative or as one cluster

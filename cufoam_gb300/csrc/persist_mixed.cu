@@ -645,7 +645,12 @@ void launch_persist_mixed(Context *ctx, int solver, int format, const SolveArgs 
     int scope = kScopeGrid, grid = 1;
     size_t smem = 0;
     const bool small_rows = !A.has_long && max_len <= kLongRow;
-    if (small_rows && A.n <= CF_PERSIST_CLUSTER_ROWS && ctx->cluster16_ok == 1) {
+    auto pick = [&](int in) {
+        return kind == kMxCG   ? mixed_pick<kMxCG>(in, format)
+               : kind == kMxMR ? mixed_pick<kMxMR>(in, format)
+                               : mixed_pick<kMxBCS>(in, format);
+    };
+    if (small_rows && A.n <= CF_PERSIST_CLUSTER_ROWS && persist_cluster_fits(ctx, pick(kScopeCluster))) {
         while (grid < 16 && 4 * grid < ns) grid <<= 1;
         const auto pl = plan((ns + grid - 1) / grid, true, CF_PERSIST_LOCAL_BYTES - sizeof(ClusterSync::Shared));
         if (complete(pl.first)) {
@@ -668,9 +673,7 @@ void launch_persist_mixed(Context *ctx, int solver, int format, const SolveArgs 
     }
     const double slot = format == kSellC ? 5.0 : format == kSellD ? 6.0 : 8.0;
     P.keep = slot * 32.0 * ns * max_len + 40.0 * A.n < 0.95 * (double)ctx->l2_bytes ? 1 : 0;
-    const void *kernel = kind == kMxCG   ? mixed_pick<kMxCG>(scope, format)
-                         : kind == kMxMR ? mixed_pick<kMxMR>(scope, format)
-                                         : mixed_pick<kMxBCS>(scope, format);
+    const void *kernel = pick(scope);
     SolveArgs a = A;
     void *args[] = {&a, &P};
     out->flags = 0;   // (S may be *out: read above)

@@ -28,6 +28,21 @@ def _code(name):
     return re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
 
 
+def test_cluster_occupancy_is_asked_for_the_launched_kernel_and_size():
+    """A kernel's cluster may fit where another's does not (registers, static
+    and dynamic shared memory): the query names the kernel of the launch and
+    the largest dynamic size a launch may have, and every choice of the single
+    cluster asks it."""
+    text = _code("persist.cu")
+    fits = _body(text, text.index("bool persist_cluster_fits("))
+    assert "cfg.dynamicSmemBytes = persist_smem_limit(true);" in fits
+    assert "cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg)" in fits
+    for name in ("persist.cu", "persist_mixed.cu"):
+        code = _code(name)
+        uses = re.findall(r"if \(([^{]*CF_PERSIST_CLUSTER_ROWS[^{]*)\) \{", code)
+        assert uses and all("persist_cluster_fits(ctx, " in u and "kScopeCluster" in u for u in uses)
+
+
 def test_cluster_scope_waits_for_its_blocks_before_the_first_remote_store():
     text = _code("persist.cuh")
     scope = _body(text, text.index("struct ClusterSync"))
