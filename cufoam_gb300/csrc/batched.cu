@@ -32,8 +32,9 @@
 // Two scopes a system is solved in (ClusterScope, GroupScope): a cluster that
 // takes systems from the queue, or -- for batches of few systems, where the
 // largest one would keep its cluster's quarter of 16 SMs busy long after the
-// others are done -- a fixed group of blocks per system, sized by its work,
-// with software barriers (see group_plan).
+// others are done -- a group of blocks per system, sized by its work, with
+// software barriers (see group_plan), and dealt anew where systems need many
+// more steps than others (see solve_groups).
 //
 // The same kernel with one system and one component is the single-launch
 // CG of small CSR systems (solve_cg_single_cluster, at the end of this file).
@@ -114,6 +115,11 @@ struct BatchArgs {
     double *partials;        // [2][3 kBatchMaxR][blocks]
     int32_t *gave_up;
     int32_t poll_limit;
+    // after step pause_at of a system (of a sweep) its group saves the solve's state and
+    // leaves (open[system] = 1); a RESUMED launch goes on from such states
+    int32_t pause_at;
+    int32_t *open;           // [n_systems]
+    void *carry;             // [n_systems] BatchCarry<R>
 };
 
 struct NoPost {
@@ -180,6 +186,7 @@ __device__ __forceinline__ void cluster_sum(cgp::cluster_group &cl, double (&v)[
 // system to solve (-1: none)
 // ---------------------------------------------------------------------------
 struct ClusterScope {
+    static constexpr bool kPauses = false;
     static constexpr int entries(int) { return kBatchEntryBatch; }
     cgp::cluster_group cl;
     __device__ __forceinline__ ClusterScope(const BatchArgs &) : cl(cgp::this_cluster()) {}
@@ -209,6 +216,7 @@ struct ClusterScope {
 // sums the group's partials in rank order.  A wait that gives up (poll_limit)
 // makes every further sum NaN, which ends the solve.
 struct GroupScope {
+    static constexpr bool kPauses = true;
     // (48 systems, 662k rows: 1 component 1,018 us with one entry per batch,
     // 941 with two; 3 components 1,915 and 2,088)
     static constexpr int entries(int r) { return r == 1 ? 2 : 1; }
@@ -456,6 +464,13 @@ struct CompState {
     int act[R], act_in[R], iters[R];
 };
 
+// A paused solve: the scalars; x (or e), r and p are in global memory.
+template <int R>
+struct BatchCarry {
+    CompState<R> st;
+    int32_t k, sweep;          // last step (of the sweep), the sweep
+};
+
 // FP64 residual r = b - A x and ||r||^2 per component over this CTA's slices,
 // summed over the cluster into tot[0..R)
 template <int R, int BT, class Scope>
@@ -500,7 +515,8 @@ template <int BT> constexpr int batch_min_blocks()
     return CF_BATCH_THREADS_PER_SM / BT > 0 ? CF_BATCH_THREADS_PER_SM / BT : 1;
 }
 
-template <int R, int BT, bool MIXED, class Scope>
+// RESUMED: the launch goes on from saved states
+template <int R, int BT, bool MIXED, class Scope, bool RESUMED = false>
 __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const BatchArgs a)
 {
     Scope sc(a);
@@ -516,92 +532,121 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
     // that they do not hold registers through the row loops
     __shared__ BatchSystem S;
     __shared__ int32_t s_next;
+    __shared__ int32_t s_pause;        // mixed: the last step was pause_at
+    __shared__ int32_t s_mid, s_sweep; // RESUMED: the last step of a sweep that has begun (else 0); the sweep
     int parity = 0;
+    // the state of system sid after step k: rank 0 saves it, and every block leaves
+    auto pause = [&](int sid, int k, int sweep) {
+        if (rank != 0) return;
+        BatchCarry<R> &c = static_cast<BatchCarry<R> *>(a.carry)[sid];
+        for (int i = threadIdx.x; i < (int)(sizeof(st) / 4); i += BT)
+            reinterpret_cast<int32_t *>(&c.st)[i] = reinterpret_cast<const int32_t *>(&st)[i];
+        if (threadIdx.x == 0) {
+            c.k = k;
+            c.sweep = sweep;
+            a.open[sid] = 1;
+        }
+    };
 
     for (;;) {
         const int sid = sc.next(a, &s_next);
         if (sid < 0) break;
-        if (threadIdx.x == 0) S = a.sys[sid];
+        if (threadIdx.x == 0) {
+            S = a.sys[sid];
+            s_pause = 0;
+        }
         __syncthreads();
         const int n = S.n;
         const int ns = (n + 31) >> 5;
         // this CTA's slices; a thread owns rows s * 32 + lane of the slices
         // s = s_lo + warp + k W in every phase
         const int s_lo = (int)((int64_t)ns * rank / cs), s_hi = (int)((int64_t)ns * (rank + 1) / cs);
+        int k0 = 0;                  // FP64: the last step before this launch
 
-        // ---- normFactor part 1: mean of psi per component ----------------
-        {
-            const double *x = a.x + S.vec_offset * R;
-            double acc1[R];
-#pragma unroll
-            for (int j = 0; j < R; ++j) acc1[j] = 0.0;
-            for (int s = s_lo + warp; s < s_hi; s += W) {
-                const int row = s * 32 + lane;
-                if (row < n)
-#pragma unroll
-                    for (int j = 0; j < R; ++j) acc1[j] += x[(int64_t)row * R + j];
+        if constexpr (RESUMED) {
+            const BatchCarry<R> &c = static_cast<const BatchCarry<R> *>(a.carry)[sid];
+            for (int i = threadIdx.x; i < (int)(sizeof(st) / 4); i += BT)
+                reinterpret_cast<int32_t *>(&st)[i] = reinterpret_cast<const int32_t *>(&c.st)[i];
+            if (threadIdx.x == 0) {
+                s_mid = c.k;
+                s_sweep = c.sweep;
             }
-            sc.template sum<R, BT>(acc1, wsm, slot[parity], tot);
-            parity ^= 1;
-        }
-        // ---- normFactor part 2 + initial residual r = b - A x ------------
-        {
-            const double *x = a.x + S.vec_offset * R, *b = a.b + S.vec_offset * R;
-            double *r = a.r + S.vec_offset * R;
-            double xbar[R];
+            k0 = c.k;
+        } else {
+            // ---- normFactor part 1: mean of psi per component ----------------
+            {
+                const double *x = a.x + S.vec_offset * R;
+                double acc1[R];
 #pragma unroll
-            for (int j = 0; j < R; ++j) xbar[j] = tot[j] / n;
-            bool on[R];
+                for (int j = 0; j < R; ++j) acc1[j] = 0.0;
+                for (int s = s_lo + warp; s < s_hi; s += W) {
+                    const int row = s * 32 + lane;
+                    if (row < n)
 #pragma unroll
-            for (int j = 0; j < R; ++j) on[j] = true;
-            double acc3[3 * R];
-#pragma unroll
-            for (int j = 0; j < 3 * R; ++j) acc3[j] = 0.0;
-            for (int s = s_lo + warp; s < s_hi; s += W) {
-                const int row = s * 32 + lane;
-                double y[R], ys;
-                row_product<R, double, double>(S, S.s_val, S.val, s, row, on,
-                                               [&](int c, double(&o)[R]) {
-#pragma unroll
-                                                   for (int j = 0; j < R; ++j) o[j] = __ldcg(x + (int64_t)c * R + j);
-                                               },
-                                               y, ys);
-                if (row < n)
-#pragma unroll
-                    for (int j = 0; j < R; ++j) {
-                        const int64_t o = (int64_t)row * R + j;
-                        const double yb = ys * xbar[j];
-                        const double bi = b[o];
-                        const double d1 = y[j] - yb, d2 = bi - yb, ri = bi - y[j];
-                        r[o] = ri;
-                        acc3[j] = fma_t(d1, d1, acc3[j]);
-                        acc3[R + j] = fma_t(d2, d2, acc3[R + j]);
-                        acc3[2 * R + j] = fma_t(ri, ri, acc3[2 * R + j]);
-                    }
+                        for (int j = 0; j < R; ++j) acc1[j] += x[(int64_t)row * R + j];
+                }
+                sc.template sum<R, BT>(acc1, wsm, slot[parity], tot);
+                parity ^= 1;
             }
-            sc.template sum<3 * R, BT>(acc3, wsm, slot[parity], tot);
-            parity ^= 1;
-        }
-        if (threadIdx.x < R) {
-            const int j = threadIdx.x;
-            st.nf[j] = sqrt(tot[j]) + sqrt(tot[R + j]) + 1e-20;
-            st.tol[j] = a.tolerance * st.nf[j];
-            st.rho[j] = tot[2 * R + j];
-            st.rho_old[j] = 0.0;
-            st.nrm[j] = sqrt(st.rho[j]);
-            st.alpha[j] = 0.0;
-            st.act[j] = isfinite(st.nrm[j]) && st.nrm[j] > st.tol[j] && a.max_iter >= 1;
-            st.iters[j] = 0;
-            if (rank == 0) {
-                a.out[(int64_t)sid * R + j].nf = st.nf[j];
-                a.out[(int64_t)sid * R + j].norm0 = st.nrm[j];
+            // ---- normFactor part 2 + initial residual r = b - A x ------------
+            {
+                const double *x = a.x + S.vec_offset * R, *b = a.b + S.vec_offset * R;
+                double *r = a.r + S.vec_offset * R;
+                double xbar[R];
+#pragma unroll
+                for (int j = 0; j < R; ++j) xbar[j] = tot[j] / n;
+                bool on[R];
+#pragma unroll
+                for (int j = 0; j < R; ++j) on[j] = true;
+                double acc3[3 * R];
+#pragma unroll
+                for (int j = 0; j < 3 * R; ++j) acc3[j] = 0.0;
+                for (int s = s_lo + warp; s < s_hi; s += W) {
+                    const int row = s * 32 + lane;
+                    double y[R], ys;
+                    row_product<R, double, double>(S, S.s_val, S.val, s, row, on,
+                                                   [&](int c, double(&o)[R]) {
+#pragma unroll
+                                                       for (int j = 0; j < R; ++j) o[j] = __ldcg(x + (int64_t)c * R + j);
+                                                   },
+                                                   y, ys);
+                    if (row < n)
+#pragma unroll
+                        for (int j = 0; j < R; ++j) {
+                            const int64_t o = (int64_t)row * R + j;
+                            const double yb = ys * xbar[j];
+                            const double bi = b[o];
+                            const double d1 = y[j] - yb, d2 = bi - yb, ri = bi - y[j];
+                            r[o] = ri;
+                            acc3[j] = fma_t(d1, d1, acc3[j]);
+                            acc3[R + j] = fma_t(d2, d2, acc3[R + j]);
+                            acc3[2 * R + j] = fma_t(ri, ri, acc3[2 * R + j]);
+                        }
+                }
+                sc.template sum<3 * R, BT>(acc3, wsm, slot[parity], tot);
+                parity ^= 1;
+            }
+            if (threadIdx.x < R) {
+                const int j = threadIdx.x;
+                st.nf[j] = sqrt(tot[j]) + sqrt(tot[R + j]) + 1e-20;
+                st.tol[j] = a.tolerance * st.nf[j];
+                st.rho[j] = tot[2 * R + j];
+                st.rho_old[j] = 0.0;
+                st.nrm[j] = sqrt(st.rho[j]);
+                st.alpha[j] = 0.0;
+                st.act[j] = isfinite(st.nrm[j]) && st.nrm[j] > st.tol[j] && a.max_iter >= 1;
+                st.iters[j] = 0;
+                if (rank == 0) {
+                    a.out[(int64_t)sid * R + j].nf = st.nf[j];
+                    a.out[(int64_t)sid * R + j].norm0 = st.nrm[j];
+                }
             }
         }
         __syncthreads();
 
         if constexpr (MIXED) {
             // ---- FP32 CG sweeps on A e = r / ||r|| inside FP64 refinement ----
-            for (int sweep = 0; sweep < a.max_outer; ++sweep) {
+            for (int sweep = RESUMED ? s_sweep : 0; sweep < a.max_outer; ++sweep) {
                 bool act[R], any = false;
 #pragma unroll
                 for (int j = 0; j < R; ++j) {
@@ -610,46 +655,55 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                 }
                 if (!any) break;
                 // inner right-hand side r / ||r||, e = 0, and its squared norm
-                {
-                    const double *r = a.r + S.vec_offset * R;
-                    float *r32 = a.r32 + S.vec_offset * R, *e32 = a.e32 + S.vec_offset * R;
-                    float inv[R];
+                // (a resumed solve is inside its sweep)
+                if (!RESUMED || !s_mid) {
+                    {
+                        const double *r = a.r + S.vec_offset * R;
+                        float *r32 = a.r32 + S.vec_offset * R, *e32 = a.e32 + S.vec_offset * R;
+                        float inv[R];
 #pragma unroll
-                    for (int j = 0; j < R; ++j) inv[j] = act[j] ? (float)(1.0 / st.nrm[j]) : 0.f;
-                    double acc0[R];
+                        for (int j = 0; j < R; ++j) inv[j] = act[j] ? (float)(1.0 / st.nrm[j]) : 0.f;
+                        double acc0[R];
 #pragma unroll
-                    for (int j = 0; j < R; ++j) acc0[j] = 0.0;
-                    for (int s = s_lo + warp; s < s_hi; s += W) {
-                        const int row = s * 32 + lane;
-                        if (row < n)
+                        for (int j = 0; j < R; ++j) acc0[j] = 0.0;
+                        for (int s = s_lo + warp; s < s_hi; s += W) {
+                            const int row = s * 32 + lane;
+                            if (row < n)
 #pragma unroll
-                            for (int j = 0; j < R; ++j) {
-                                const int64_t o = (int64_t)row * R + j;
-                                const float v = (float)(r[o] * (double)inv[j]);
-                                r32[o] = v;
-                                e32[o] = 0.f;
-                                acc0[j] += (double)(v * v);
-                            }
+                                for (int j = 0; j < R; ++j) {
+                                    const int64_t o = (int64_t)row * R + j;
+                                    const float v = (float)(r[o] * (double)inv[j]);
+                                    r32[o] = v;
+                                    e32[o] = 0.f;
+                                    acc0[j] += (double)(v * v);
+                                }
+                        }
+                        sc.template sum<R, BT>(acc0, wsm, slot[parity], tot);
+                        parity ^= 1;
                     }
-                    sc.template sum<R, BT>(acc0, wsm, slot[parity], tot);
-                    parity ^= 1;
+                    if (threadIdx.x < R) {
+                        const int j = threadIdx.x;
+                        st.rho32[j] = (float)tot[j];
+                        st.rho32_old[j] = 0.f;
+                        st.alpha[j] = 0.0;
+                        st.act_in[j] = st.act[j];
+                        // the last sweep only has to reach the FP64 target
+                        st.eta[j] = (float)fmax(a.inner_rtol, fmin(0.5, 0.8 * st.tol[j] / st.nrm[j]));
+                    }
+                    __syncthreads();
                 }
-                if (threadIdx.x < R) {
-                    const int j = threadIdx.x;
-                    st.rho32[j] = (float)tot[j];
-                    st.rho32_old[j] = 0.f;
-                    st.alpha[j] = 0.0;
-                    st.act_in[j] = st.act[j];
-                    // the last sweep only has to reach the FP64 target
-                    st.eta[j] = (float)fmax(a.inner_rtol, fmin(0.5, 0.8 * st.tol[j] / st.nrm[j]));
-                }
-                __syncthreads();
-                for (int k = 1;; ++k) {
+                for (int k = RESUMED ? s_mid + 1 : 1;; ++k) {
                     bool ain[R], any_in = false;
 #pragma unroll
                     for (int j = 0; j < R; ++j) {
                         ain[j] = st.act_in[j];
                         any_in = any_in || ain[j];
+                    }
+                    // (a flag in shared memory: a test of k == pause_at here cost the
+                    // mixed solves of one component 6%, 48 boxes 1.57 -> 1.67 ms)
+                    if (Scope::kPauses && s_pause) {
+                        pause(sid, k - 1, sweep);
+                        return;
                     }
                     // P: e += alpha_{k-1} p (deferred), p = r + beta p
                     {
@@ -780,6 +834,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                             st.alpha[j] = 0.0;
                         }
                     }
+                    if (Scope::kPauses && threadIdx.x == 0) s_pause = k == a.pause_at;
                     __syncthreads();
                 }
                 // the inner loop ended with a P pass that applied every
@@ -799,6 +854,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                     }
                 }
                 sc.sync(); // every CTA's x rows are written before anyone gathers them
+                if (RESUMED && threadIdx.x == 0) s_mid = 0;
                 batch_residual<R, BT>(sc, S, s_lo, s_hi, a.b + S.vec_offset * R, a.x + S.vec_offset * R,
                                       a.r + S.vec_offset * R, wsm, slot[parity], tot);
                 parity ^= 1;
@@ -816,7 +872,7 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
             }
         } else {
             // ---- CG iterations, all components together ----------------------
-            for (int k = 1;; ++k) {
+            for (int k = RESUMED ? k0 + 1 : 1;; ++k) {
                 bool act[R], any = false;
 #pragma unroll
                 for (int j = 0; j < R; ++j) {
@@ -924,6 +980,10 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<BT>()) k_batch_cg(const B
                     }
                 }
                 __syncthreads();
+                if (Scope::kPauses && k == a.pause_at) {
+                    pause(sid, k, 0);
+                    return;
+                }
             }
         }
         if (rank == 0 && threadIdx.x < R) {
@@ -1065,41 +1125,46 @@ constexpr int kGroupThreads = 256;
 // even schedule: at 1.04, 1.09 and 1.30 (100, 160 and 300 boxes) they took
 // 4.28, 3.90 and 4.11 ms against 5.37, 5.77 and 7.69 on clusters of 16 (and
 // 5.84, 4.38, 5.06 on clusters of 8), whose barriers cost the small systems
-// more; systems with very different step counts want the queue
+// more
 constexpr double kGroupSlack = 1.35;
+// steps before open systems are dealt the blocks anew (solve_groups)
+constexpr int kGroupSteps = 100;
 
-template <int R, bool MIXED>
-static const void *group_kernel() { return (const void *)k_batch_cg<R, kGroupThreads, MIXED, GroupScope>; }
+template <int R>
+static const void *group_kernel(bool mixed, bool resumed)
+{
+    return mixed ? resumed ? (const void *)k_batch_cg<R, kGroupThreads, true, GroupScope, true>
+                           : (const void *)k_batch_cg<R, kGroupThreads, true, GroupScope>
+           : resumed ? (const void *)k_batch_cg<R, kGroupThreads, false, GroupScope, true>
+                     : (const void *)k_batch_cg<R, kGroupThreads, false, GroupScope>;
+}
 
-static const void *group_kernel_for(int nrhs, bool mixed)
+static const void *group_kernel_for(int nrhs, bool mixed, bool resumed)
 {
     switch (nrhs) {
-    case 1: return mixed ? group_kernel<1, true>() : group_kernel<1, false>();
-    case 2: return mixed ? group_kernel<2, true>() : group_kernel<2, false>();
-    case 3: return mixed ? group_kernel<3, true>() : group_kernel<3, false>();
-    default: return mixed ? group_kernel<4, true>() : group_kernel<4, false>();
+    case 1: return group_kernel<1>(mixed, resumed);
+    case 2: return group_kernel<2>(mixed, resumed);
+    case 3: return group_kernel<3>(mixed, resumed);
+    default: return group_kernel<4>(mixed, resumed);
     }
 }
 
+// Blocks a system has work for: one per `per` slices.
+static int64_t group_most(int slices, int per) { return std::max(1, (slices + per - 1) / per); }
+
 // The blocks of each system when `blocks` of them run at once: the smallest
-// largest share of work W with sum ceil(work / W) <= blocks (at most a block
-// per eight slices).  Empty when the queue of clusters would finish much
-// sooner (kGroupSlack): its clusters of 16 blocks take the systems largest
-// first, and a block's share is a sixteenth of its cluster's systems.  Both run
-// the same number of blocks per SM.  Measured on GB300
+// largest share of work W with sum ceil(work / W) <= blocks.  Measured on GB300
 // (transient 7-point systems to 1e-8, 3 components, clusters -> groups): 48
 // boxes of 12^3..36^3, 662k rows, 2.75 -> 1.92 ms; 8 such boxes 1.33 -> 0.70; 48
 // boxes of 10^3..18^3 1.22 -> 0.74; 16 of 20^3..24^3 1.23 -> 0.96; mixed precision,
 // 48 boxes 2.51 -> 1.84.  What is left there is L2: the three components of a
 // gathered row are 32 random bytes, about 5 TB/s.
 static std::vector<int> group_plan(const std::vector<int64_t> &work, const std::vector<int> &slices, int blocks,
-                                   int clusters)
+                                   int per)
 {
     const int S = (int)work.size();
-    if (S > blocks || clusters < 1) return {};
     auto share = [&](int s, int64_t w) {
-        const int64_t g = (work[s] + w - 1) / w;
-        return (int)std::max<int64_t>(1, std::min<int64_t>(g, (slices[s] + 7) / 8));
+        return (int)std::max<int64_t>(1, std::min<int64_t>((work[s] + w - 1) / w, group_most(slices[s], per)));
     };
     int64_t lo = 1, hi = 1;
     for (int64_t w : work) hi = std::max(hi, w);
@@ -1111,63 +1176,114 @@ static std::vector<int> group_plan(const std::vector<int64_t> &work, const std::
         else lo = mid + 1;
     }
     std::vector<int> g(S);
+    for (int s = 0; s < S; ++s) g[s] = share(s, lo);
+    return g;
+}
+
+// Whether the queue of clusters would finish much sooner (kGroupSlack): its
+// clusters of 16 blocks take the systems largest first, and a block's share is
+// a sixteenth of its cluster's systems.  Both run the same number of blocks per
+// SM.
+static bool queue_is_better(const std::vector<int64_t> &work, const std::vector<int> &g, int clusters)
+{
     double most = 0.0;
-    for (int s = 0; s < S; ++s) {
-        g[s] = share(s, lo);
-        most = std::max(most, (double)work[s] / g[s]);
-    }
-    // the clusters' schedule
+    for (size_t s = 0; s < work.size(); ++s) most = std::max(most, (double)work[s] / g[s]);
     std::vector<int64_t> sorted(work), load(clusters, 0);
     std::sort(sorted.begin(), sorted.end(), std::greater<int64_t>());
     for (int64_t w : sorted) *std::min_element(load.begin(), load.end()) += w;
     const double queue = (double)*std::max_element(load.begin(), load.end()) / 16.0;
-    if (most > kGroupSlack * queue) g.clear();
-    return g;
+    return most > kGroupSlack * queue;
 }
 
-// Launches the batch as groups; false when the clusters are the better (or
+// Solves the batch in groups; false when the clusters are the better (or
 // the only possible) schedule.
-static bool launch_groups(Context *ctx, Batch *B, BatchArgs &a, int nrhs, bool mixed, cudaStream_t s)
+//
+// Groups are sized for systems of like step counts.  Where a group has fewer
+// blocks than a cluster, the systems that are not done after kGroupSteps steps
+// are dealt all blocks anew and go on from their state, and again after 3, 7,
+// 15 ... times as many (a step count, so that a repeated solve has the same
+// bits; the FP32 steps of a sweep where the precision is mixed).  Measured on
+// GB300 with 3 components, ms on clusters of 16 / groups without / with pauses,
+// FP64: 100 boxes of 12^3..36^3 with five of them at five times the steps 16.4 /
+// 24.3 / 15.5, with the largest alone 25.0 / 29.9 / 16.7; 160 boxes of
+// 12^3..28^3, eight such, 13.3 / 20.3 / 13.6; 300 of 12^3..24^3, the largest,
+// 15.8 / 23.9 / 15.1; 48 of 12^3..36^3, a medium one, 7.8 / 9.8 / 7.7.  Mixed, with a
+// block per 16 slices after a pause (its steps are shorter against the
+// barriers): 100 boxes, five of them, 11.4 / 18.0 / 11.2.  Batches that end
+// before the first pause are unchanged.
+static bool solve_groups(Context *ctx, Batch *B, BatchArgs &a, int nrhs, bool mixed, cudaStream_t s)
 {
     const int S = (int)B->mats.size();
-    const void *kernel = group_kernel_for(nrhs, mixed);
+    const void *kernel = group_kernel_for(nrhs, mixed, false), *resumed = group_kernel_for(nrhs, mixed, true);
     int per_sm = 0;
-    if (!persist_usable(ctx, CF_CG, kSell, false) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kGroupThreads, 0) != cudaSuccess || per_sm < 1) {
-        cudaGetLastError();
-        return false;
+    if (!persist_usable(ctx, CF_CG, kSell, false)) return false;
+    for (const void *k : {kernel, resumed}) {
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kGroupThreads, 0) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            return false;
+        }
+        per_sm = per_sm ? std::min(per_sm, n) : n;
     }
-    const int blocks = per_sm * ctx->sm_count;
-    if (S > blocks) return false;
-    std::vector<int64_t> work(S);
-    std::vector<int> slices(S);
-    for (int i = 0; i < S; ++i) {
-        work[i] = B->mats[i]->nnz;
-        slices[i] = (B->mats[i]->n + 31) / 32;
-    }
-    const std::vector<int> g = group_plan(work, slices, blocks, blocks / 16);
-    if (g.empty()) return false;
-    std::vector<int4> table;
-    for (int i = 0; i < S; ++i) {
-        const int first = (int)table.size();
-        for (int r = 0; r < g[i]; ++r) table.push_back(make_int4(i, r, g[i], first));
-    }
-    const int grid = (int)table.size();
-    const size_t tb = (sizeof(int4) * (size_t)grid + 255) / 256 * 256;
-    const size_t pb = sizeof(double) * 2 * 3 * kBatchMaxR * (size_t)grid;
-    B->d_group.ensure(tb + pb + sizeof(uint32_t) * ((size_t)S + 4));
+    const int blocks = per_sm * ctx->sm_count, clusters = blocks / 16;
+    if (S > blocks || clusters < 1) return false;
+    std::vector<int> open(S);
+    std::iota(open.begin(), open.end(), 0);
+    std::vector<int64_t> work;
+    std::vector<int> slices;
+    auto collect = [&] {
+        work.clear();
+        slices.clear();
+        for (int i : open) {
+            work.push_back(B->mats[i]->nnz);
+            slices.push_back((B->mats[i]->n + 31) / 32);
+        }
+    };
+    collect();
+    std::vector<int> g = group_plan(work, slices, blocks, 8);
+    if (queue_is_better(work, g, clusters)) return false;
+
+    const size_t tb = (sizeof(int4) * (size_t)blocks + 255) / 256 * 256;
+    const size_t pb = sizeof(double) * 2 * 3 * kBatchMaxR * (size_t)blocks;
+    const size_t fb = sizeof(int32_t) * (2 * (size_t)S + 4);
+    B->d_group.ensure(tb + pb + fb + 256 + sizeof(BatchCarry<kBatchMaxR>) * (size_t)S);
     char *base = B->d_group.as<char>();
     a.group = reinterpret_cast<const int4 *>(base);
     a.partials = reinterpret_cast<double *>(base + tb);
     a.arrivals = reinterpret_cast<uint32_t *>(base + tb + pb);
     a.gave_up = reinterpret_cast<int32_t *>(a.arrivals + S);
+    a.open = a.gave_up + 4;
+    a.carry = base + (tb + pb + fb + 255) / 256 * 256;
     a.poll_limit = ctx->poll_limit;
-    // (a pageable source: staged when the call returns)
-    CF_CUDA(cudaMemcpyAsync(base, table.data(), sizeof(int4) * (size_t)grid, cudaMemcpyHostToDevice, s));
-    CF_CUDA(cudaMemsetAsync(a.arrivals, 0, sizeof(uint32_t) * ((size_t)S + 4), s));
-    void *args[] = {&a};
-    CF_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kGroupThreads), args, 0, s));
-    return true;
+    a.pause_at = INT_MAX;
+    for (int steps = kGroupSteps;; steps = steps < INT_MAX / 4 ? 2 * steps + kGroupSteps : INT_MAX) {
+        std::vector<int4> table;
+        bool small = false;   // a group with fewer blocks than a cluster
+        for (size_t i = 0; i < open.size(); ++i) {
+            const int first = (int)table.size();
+            for (int r = 0; r < g[i]; ++r) table.push_back(make_int4(open[i], r, g[i], first));
+            small = small || g[i] < std::min<int64_t>(16, group_most(slices[i], 8));
+        }
+        a.pause_at = small && steps < a.max_iter ? steps : INT_MAX;
+        // (a pageable source: staged when the call returns)
+        CF_CUDA(cudaMemcpyAsync(base, table.data(), sizeof(int4) * table.size(), cudaMemcpyHostToDevice, s));
+        CF_CUDA(cudaMemsetAsync(a.arrivals, 0, fb, s));
+        void *args[] = {&a};
+        CF_CUDA(cudaLaunchCooperativeKernel(kernel, dim3((unsigned)table.size()), dim3(kGroupThreads), args, 0, s));
+        CF_CUDA(cudaEventRecord(ctx->ev_stop, s));
+        std::vector<int32_t> h(S + 4);   // gave_up, open
+        CF_CUDA(cudaMemcpyAsync(h.data(), a.gave_up, sizeof(int32_t) * h.size(), cudaMemcpyDeviceToHost, s));
+        CF_CUDA(cudaStreamSynchronize(s));
+        require(h[0] == 0, CF_TIMEOUT, "a block of the batched solve gave up waiting for its group");
+        if (a.pause_at == INT_MAX) return true;
+        open.clear();
+        for (int i = 0; i < S; ++i)
+            if (h[4 + i]) open.push_back(i);
+        if (open.empty()) return true;
+        collect();
+        g = group_plan(work, slices, blocks, mixed ? 16 : 8);
+        kernel = resumed;
+    }
 }
 
 // Solve all systems for `nrhs` right-hand sides (b, x: [rows][nrhs]).
@@ -1262,7 +1378,7 @@ void batch_solve(Batch *B, const cf_controls &c, int nrhs, const double *b_in, d
     CF_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
     // no cluster size asked for: groups of blocks where they finish sooner
     const bool grouped = cs == 0 && bt == kGroupThreads && maxc == 0 &&
-                         launch_groups(ctx, B, a, nrhs, mixed, ctx->stream);
+                         solve_groups(ctx, B, a, nrhs, mixed, ctx->stream);
     if (grouped) {
     } else if (use_graph) {
         CF_CUDA(cudaStreamCreateWithFlags(&cs_stream, cudaStreamNonBlocking));
@@ -1296,12 +1412,8 @@ void batch_solve(Batch *B, const cf_controls &c, int nrhs, const double *b_in, d
         default: launch_batch_r<4>(ctx, a, mixed, cs, bt, maxc, ctx->stream); break;
         }
     }
-    CF_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
-    int32_t gave_up = 0;
-    if (grouped)
-        CF_CUDA(cudaMemcpyAsync(&gave_up, a.gave_up, sizeof(gave_up), cudaMemcpyDeviceToHost, ctx->stream));
+    if (!grouped) CF_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
     CF_CUDA(cudaStreamSynchronize(ctx->stream));
-    require(gave_up == 0, CF_TIMEOUT, "a block of the batched solve gave up waiting for its group");
     if (ge) cudaGraphExecDestroy(ge);
     if (g) cudaGraphDestroy(g);
     if (cs_stream) cudaStreamDestroy(cs_stream);
