@@ -265,6 +265,9 @@ struct Matrix {
     int64_t sell_nnz = 0;      // stored entries including padding
     int32_t sell_max_len = 0;  // slots per row of the longest slice
     int32_t max_offset = 0;    // largest |col - row|
+    // a persistent solve's blocks over slices of uneven length (persist_shares)
+    DeviceBuffer shares;       // [share_blocks + 1] first slices (share_blocks 0: none)
+    int32_t share_blocks = 0, share_most = 0;
     std::vector<int32_t> offsets; // the distinct offsets col - row, ascending (empty: too many for codes)
     bool slices_scanned = false;  // s_off holds offsets (else the slices' lengths)
     DeviceBuffer arena, sell_arena; // the allocations the pattern's and the copy's buffers are parts of
@@ -345,12 +348,12 @@ bool small_cg_ok(Context *ctx);
 
 // a whole FP64 solve in the fast order as one launch (persist.cu)
 bool persist_usable(Context *ctx, int solver, int format, bool mixed);
-void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1, int max_len,
+void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1, Matrix *m,
                     DevState *out);
 // ... and a whole mixed-precision solve (persist_mixed.cu); the total of FP32
 // steps in out_in->k
 void launch_persist_mixed(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1,
-                          int max_len, const cf_controls &c, DevState *out, DevState *out_in);
+                          Matrix *m, const cf_controls &c, DevState *out, DevState *out_in);
 // ... and BiCG in the reference order (persist_ref.cu)
 bool persist_ref_usable(Context *ctx, int solver, bool sell);
 void launch_persist_ref(Context *ctx, const SolveArgs &A, const DevState &S, int l1, DevState *out);

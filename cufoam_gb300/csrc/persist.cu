@@ -55,6 +55,7 @@ struct PersistArgs {
     int32_t abs_tol, l1, power_steps;
     int32_t head;            // log2 of the rows per thread, and one (FixedDot)
     int32_t keep;            // the matrix fits in L2 beside the vectors: no evict-first hint
+    const int32_t *first;    // streamed: the blocks' first slices (null: equal numbers)
     PersistPlan plan;
 };
 
@@ -172,8 +173,9 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int rank = gs.rank();
     const bool first_block = rank == 0;
-    const int s_lo = (int)((int64_t)ns * rank / gs.blocks());
-    const int s_hi = (int)((int64_t)ns * (rank + 1) / gs.blocks());
+    const bool table = !LOCALM && P.first;
+    const int s_lo = table ? P.first[rank] : (int)((int64_t)ns * rank / gs.blocks());
+    const int s_hi = table ? P.first[rank + 1] : (int)((int64_t)ns * (rank + 1) / gs.blocks());
     const int base = 32 * s_lo;              // first row of this block
     const uint64_t pol = P.keep ? l2_evict_normal_policy() : l2_evict_first_policy();
     const auto cols = PersistCols<FMT>::make(A);
@@ -714,10 +716,64 @@ void launch_persist_kernel(Context *ctx, const void *kernel, bool cluster, int g
     CF_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
 }
 
-// `max_len`: slots per row of the longest slice.
-void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1, int max_len,
+// Equal numbers of slices are unequal work where the rows of one part of the
+// numbering are longer (a refined or polyhedral region): every pass waits for the
+// blocks of the long part.  There the blocks are dealt equal costs, a slice's
+// slots per row plus kShareVector for the vector passes (a CG step has 12 FP64
+// operations per 7-point row, five of them outside the product).  Measured on
+// GB300, us per 60 steps, the last tenth of the rows 15 long and the others 7,
+// equal numbers -> equal costs, CG / Jacobi / mixed CG: 0.5M rows 1,639 -> 1,393 /
+// 1,229 -> 931 / 1,035 -> 923; 2M rows 4,907 -> 3,903 / 4,119 -> 2,855 / 2,891 ->
+// 2,303 (the multi-kernel loop, which deals slices round robin: 4,623 / 3,562 /
+// 3,457).
+constexpr int kShareVector = 5;
+// ... where the longest slice costs this much more than the mean one
+constexpr double kShareUneven = 1.05;
+
+// first[0 .. grid]: the blocks' first slices, at equal steps of the running cost;
+// returns the most slices of a block
+static int share_slices(const int32_t *off, int ns, int grid, int32_t *first)
+{
+    auto cost = [&](int s) { return (int64_t)off[s] / 32 + (int64_t)kShareVector * s; };
+    const int64_t total = cost(ns);
+    int s = 0, most = 0;
+    first[0] = 0;
+    for (int b = 1; b <= grid; ++b) {
+        const int64_t want = total * b / grid;
+        while (s < ns && cost(s) < want) ++s;
+        first[b] = b == grid ? ns : s;
+        most = std::max(most, first[b] - first[b - 1]);
+    }
+    return most;
+}
+
+const int32_t *persist_shares(Matrix *m, int grid, int &most)
+{
+    const int ns = m->n_slices;
+    most = (ns + grid - 1) / grid;
+    if (m->sell_max_len + kShareVector <= kShareUneven * ((double)m->sell_nnz / (32.0 * ns) + kShareVector))
+        return nullptr;
+    if (m->share_blocks != grid) {   // (once per pattern)
+        std::vector<int32_t> off((size_t)ns + 1), first((size_t)grid + 1);
+        m->share_blocks = 0;
+        CF_CUDA(cudaMemcpyAsync(off.data(), m->s_off.ptr, sizeof(int32_t) * off.size(), cudaMemcpyDeviceToHost,
+                                m->ctx->stream));
+        CF_CUDA(cudaStreamSynchronize(m->ctx->stream));
+        m->share_most = share_slices(off.data(), ns, grid, first.data());
+        m->shares.ensure(sizeof(int32_t) * first.size());
+        // (a pageable source: staged when the call returns)
+        CF_CUDA(cudaMemcpyAsync(m->shares.ptr, first.data(), sizeof(int32_t) * first.size(), cudaMemcpyHostToDevice,
+                                m->ctx->stream));
+        m->share_blocks = grid;
+    }
+    most = m->share_most;
+    return m->shares.as<int32_t>();
+}
+
+void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1, Matrix *m,
                     DevState *out)
 {
+    const int max_len = m->sell_max_len;   // slots per row of the longest slice
     PersistArgs P;
     std::memset(&P, 0, sizeof(P));
     P.g = persist_grid(ctx);
@@ -762,7 +818,7 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
         return std::make_pair(p, sizeof(double) * (size_t)at);
     };
 
-    int scope = kScopeGrid, grid = 1;
+    int scope = kScopeGrid, grid = 1, most = 0;   // (most: slices of a block)
     size_t smem = 0;
     if (A.n <= CF_PERSIST_CLUSTER_ROWS && !A.has_long &&
         persist_cluster_fits(ctx, persist_kernel(solver, kScopeCluster, format))) {
@@ -786,6 +842,7 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
             smem = pl.second;
         } else {
             // vectors only, as many as fit: q and r first, then x
+            P.first = persist_shares(m, grid, most);
             int at = 0;
             const int cap = CF_PERSIST_VEC_BYTES / (int)sizeof(double);
             auto take = [&](bool want, int doubles) {
@@ -795,25 +852,26 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
                 return o;
             };
             P.plan.val = P.plan.col = P.plan.scale = P.plan.g = P.plan.g2 = -1;
-            P.plan.off = take(slices <= 4096, slices / 2 + 2);
-            P.plan.q = take(slices <= 4096 && q, 32 * slices);
-            P.plan.r = take(slices <= 4096 && !gather_r, 32 * slices);
-            P.plan.x = take(slices <= 4096 && local_x, 32 * slices);
+            P.plan.off = take(most <= 4096, most / 2 + 2);
+            P.plan.q = take(most <= 4096 && q, 32 * most);
+            P.plan.r = take(most <= 4096 && !gather_r, 32 * most);
+            P.plan.x = take(most <= 4096 && local_x, 32 * most);
             smem = sizeof(double) * (size_t)at;
         }
     }
     // 893k rows (75 MB of slots, 36 MB of vectors): CG step 29.1 us with the
     // evict-first hint, 27.0 without; 2.1M rows (176 MB) need it
-    const double slots = (double)ns * 32.0 * max_len * 12.0, vectors = 40.0 * A.n;
+    const double slots = 12.0 * (double)m->sell_nnz, vectors = 40.0 * A.n;
     P.keep = slots + vectors < 0.95 * (double)ctx->l2_bytes ? 1 : 0;
     const void *kernel = persist_kernel(solver, scope, format);
-    const int slices_per_warp = ((ns + grid - 1) / grid + kPWarps - 1) / kPWarps;
+    if (!most) most = (ns + grid - 1) / grid;
+    const int slices_per_warp = (most + kPWarps - 1) / kPWarps;
     P.head = 2;
     while ((1 << (P.head - 1)) <= slices_per_warp) ++P.head;
     SolveArgs a = A;
     void *args[] = {&a, &P};
     out->flags = 0;   // (S may be *out: read above)
-    launch_persist_kernel(ctx, kernel, scope == kScopeCluster, grid, (ns + grid - 1) / grid, smem, args);
+    launch_persist_kernel(ctx, kernel, scope == kScopeCluster, grid, most, smem, args);
 }
 
 // after a solve whose blocks gave up waiting: the arrival counter is not zero

@@ -548,6 +548,9 @@ constexpr size_t persist_smem_limit(bool cluster)
 }
 // whether a cluster of kPClusterMax blocks of a single-cluster kernel can be resident
 bool persist_cluster_fits(Context *ctx, const void *kernel);
+// The slices of `grid` blocks over a streamed matrix: the device table of their
+// first slices (null: equal numbers), and the most one of them has.
+const int32_t *persist_shares(Matrix *m, int grid, int &most);
 // the barrier counter and partial sums of the context
 PersistGrid persist_grid(Context *ctx);
 // `grid` blocks, one warp per slice up to 32, cooperative or as one cluster

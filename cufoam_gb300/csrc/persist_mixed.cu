@@ -47,6 +47,7 @@ struct MixedArgs {
     int32_t jmr;             // the residual is D^-1/2 (b - A x)
     int32_t keep;            // the FP32 matrix fits in L2: no evict-first hint
     double *x_keep, *r_keep; // x and r before a correction
+    const int32_t *first;    // streamed: the blocks' first slices (null: equal numbers)
     MixedPlan plan;
 };
 
@@ -95,8 +96,9 @@ __global__ void __launch_bounds__(SYNC::kThreads, 1)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int rank = gs.rank();
     const bool first = rank == 0;
-    const int s_lo = (int)((int64_t)ns * rank / gs.blocks());
-    const int s_hi = (int)((int64_t)ns * (rank + 1) / gs.blocks());
+    const bool table = !LOCALM && P.first;
+    const int s_lo = table ? P.first[rank] : (int)((int64_t)ns * rank / gs.blocks());
+    const int s_hi = table ? P.first[rank + 1] : (int)((int64_t)ns * (rank + 1) / gs.blocks());
     const int base = 32 * s_lo;
     const uint64_t pol = P.keep ? l2_evict_normal_policy() : l2_evict_first_policy();
     const uint64_t pol64 = l2_evict_first_policy();
@@ -587,8 +589,9 @@ static const void *mixed_pick(int scope, int format)
 }
 
 void launch_persist_mixed(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1,
-                          int max_len, const cf_controls &c, DevState *out, DevState *out_in)
+                          Matrix *m, const cf_controls &c, DevState *out, DevState *out_in)
 {
+    const int max_len = m->sell_max_len;   // slots per row of the longest slice
     MixedArgs P;
     std::memset(&P, 0, sizeof(P));
     P.g = persist_grid(ctx);
@@ -642,7 +645,7 @@ void launch_persist_mixed(Context *ctx, int solver, int format, const SolveArgs 
         return p.off >= 0 && p.val >= 0 && p.col >= 0 && p.q >= 0 && p.r >= 0 && p.d >= 0 &&
                (kind == kMxMR || p.own >= 0) && (kind != kMxBCS || (p.rh >= 0 && p.t >= 0 && p.own2 >= 0));
     };
-    int scope = kScopeGrid, grid = 1;
+    int scope = kScopeGrid, grid = 1, most = 0;   // (most: slices of a block)
     size_t smem = 0;
     const bool small_rows = !A.has_long && max_len <= kLongRow;
     auto pick = [&](int in) {
@@ -666,18 +669,20 @@ void launch_persist_mixed(Context *ctx, int solver, int format, const SolveArgs 
         if (small_rows && complete(pl.first)) {
             scope = kScopeGridLocal;
         } else {
-            pl = plan(slices, false, CF_PERSIST_VEC_BYTES);
+            P.first = persist_shares(m, grid, most);
+            pl = plan(most, false, CF_PERSIST_VEC_BYTES);
         }
         P.plan = pl.first;
         smem = pl.second;
     }
     const double slot = format == kSellC ? 5.0 : format == kSellD ? 6.0 : 8.0;
-    P.keep = slot * 32.0 * ns * max_len + 40.0 * A.n < 0.95 * (double)ctx->l2_bytes ? 1 : 0;
+    P.keep = slot * (double)m->sell_nnz + 40.0 * A.n < 0.95 * (double)ctx->l2_bytes ? 1 : 0;
     const void *kernel = pick(scope);
     SolveArgs a = A;
     void *args[] = {&a, &P};
     out->flags = 0;   // (S may be *out: read above)
-    launch_persist_kernel(ctx, kernel, scope == kScopeCluster, grid, (ns + grid - 1) / grid, smem, args);
+    launch_persist_kernel(ctx, kernel, scope == kScopeCluster, grid, most ? most : (ns + grid - 1) / grid, smem,
+                          args);
 }
 
 } // namespace cf

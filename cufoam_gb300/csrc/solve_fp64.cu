@@ -774,9 +774,9 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
         if (ref)
             launch_persist_ref(ctx, A, S, l1, ctx->h_state);
         else if (mixed)
-            launch_persist_mixed(ctx, solver, fmt, A, S, l1, m->sell_max_len, c, ctx->h_state, ctx->h_state_in);
+            launch_persist_mixed(ctx, solver, fmt, A, S, l1, m, c, ctx->h_state, ctx->h_state_in);
         else
-            launch_persist(ctx, solver, fmt, A, S, l1, m->sell_max_len, ctx->h_state);
+            launch_persist(ctx, solver, fmt, A, S, l1, m, ctx->h_state);
         CF_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
     } else {
     CF_CUDA(cudaMemcpyAsync(d_args, &A, sizeof(SolveArgs), cudaMemcpyHostToDevice, ctx->stream));
