@@ -323,13 +323,15 @@ static __device__ __noinline__ double seq_finish(const double *part, int G, cons
 // order for the reference order, else a strided sum + block tree), so the
 // result is deterministic.  Returns true in the last block, where `out`
 // holds the totals (in thread 0).  The arrival counter is reset for the
-// next launch.  No block ever waits for another.
-template <int NV, class T>
+// next launch.  No block ever waits for another.  REF false: callers of the
+// fast order alone, which need no scratch for the sequential sums (it comes out
+// of the L1 of the CSR passes).
+template <int NV, class T, bool REF = true>
 __device__ __forceinline__ bool grid_reduce(T (&acc)[NV], T *partials, int stride,
                                             uint32_t *counter, bool ref_order, T (&out)[NV])
 {
     // (the reference order's sequential sums use it for their events)
-    __shared__ T sm[NV * (sizeof(T) == 8 ? 2 * kSeqEvents : kBlock)];
+    __shared__ T sm[NV * (REF && sizeof(T) == 8 ? 2 * kSeqEvents : kBlock)];
     __shared__ bool s_last;
     pdl_trigger();
 #if CF_FAST_BLOCK_SUM
@@ -348,10 +350,10 @@ __device__ __forceinline__ bool grid_reduce(T (&acc)[NV], T *partials, int strid
     if (!s_last) return false;
     __threadfence();
     const int G = gridDim.x;
-    if (ref_order) {
+    if (REF && ref_order) {
         // the partials in block order, one sequential sum per value: the
         // block prepares each value's events, warp i adds up value i
-        if constexpr (sizeof(T) == 8) {
+        if constexpr (REF && sizeof(T) == 8) {
             __shared__ SeqScratch sc[NV];
             __shared__ double buf[kSeqMax];
             __syncthreads(); // the block sum's use of sm is over

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kBlock) k_dd_sum(DdArgs d)
         }
     }
     double tot[NV];
-    if (grid_reduce<NV, double>(acc, d.partials, d.stride, d.counter, false, tot) && threadIdx.x == 0)
+    if (grid_reduce<NV, double, false>(acc, d.partials, d.stride, d.counter, false, tot) && threadIdx.x == 0)
 #pragma unroll
         for (int i = 0; i < NV; ++i) d.out[i] = tot[i];
 }

@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(kBlock, CF_SPMV_MIN_BLOCKS) k_mx_residual(cons
         acc[0] = fma_t(ri, ri, acc[0]);
     });
     double tot[1];
-    if (grid_reduce<1, double>(acc, a->partials, a->partial_stride, &a->st->counters[SLOT_MISC],
-                               false, tot) && threadIdx.x == 0) {
+    if (grid_reduce<1, double, false>(acc, a->partials, a->partial_stride, &a->st->counters[SLOT_MISC],
+                                      false, tot) && threadIdx.x == 0) {
         DevState *st = a->st;
         const double norm = sqrt(tot[0]);
         const int k = st->k + 1; // outer steps
@@ -114,8 +114,8 @@ __global__ void __launch_bounds__(kBlock) k_mx_setup(const SolveArgs *__restrict
         acc[0] = fma_t(v, v, acc[0]);
     }
     float tot[1];
-    if (grid_reduce<1, float>(acc, a->partials32, a->partial_stride, &si->counters[SLOT_INIT], false,
-                              tot) && threadIdx.x == 0) {
+    if (grid_reduce<1, float, false>(acc, a->partials32, a->partial_stride, &si->counters[SLOT_INIT], false,
+                                     tot) && threadIdx.x == 0) {
         const float rr = tot[0];
         const double norm0 = sqrtf(rr);
         si->rho0 = rr;
@@ -159,8 +159,8 @@ __global__ void __launch_bounds__(kBlock, CF_MX_CG_MIN_BLOCKS) k_mx_cg_spmv(cons
         acc[0] = fma_t(pi, y, acc[0]);
     });
     float tot[1];
-    if (grid_reduce<1, float>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_A], false,
-                              tot) && threadIdx.x == 0) {
+    if (grid_reduce<1, float, false>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_A], false,
+                                     tot) && threadIdx.x == 0) {
         st->xi = (float)st->rho0 / tot[0];
         st->x_pending = 0;
     }
@@ -181,8 +181,8 @@ __global__ void __launch_bounds__(kBlock) k_mx_cg_update(const SolveArgs *__rest
         acc[0] = fma_t(ri, ri, acc[0]);
     }
     float tot[1];
-    if (grid_reduce<1, float>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_B], false,
-                              tot) && threadIdx.x == 0) {
+    if (grid_reduce<1, float, false>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_B], false,
+                                     tot) && threadIdx.x == 0) {
         st->rho1 = st->rho0;
         st->rho0 = tot[0];
         st->x_pending = 1;
@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(kBlock, CF_MX_BCS_MIN_BLOCKS) k_mx_bcs_spmv1(c
         acc[0] = fma_t(rh[row], y, acc[0]);
     });
     float tot[1];
-    if (grid_reduce<1, float>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_A], false,
-                              tot) && threadIdx.x == 0) {
+    if (grid_reduce<1, float, false>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_A], false,
+                                     tot) && threadIdx.x == 0) {
         const float alpha = (float)st->rho0 / tot[0];
         if (isfinite(alpha) && tot[0] != 0.f) {
             st->xi = alpha;
@@ -279,8 +279,8 @@ __global__ void __launch_bounds__(kBlock, CF_MX_BCS_MIN_BLOCKS) k_mx_bcs_spmv2(c
         acc[1] = fma_t(y, y, acc[1]);
     });
     float tot[2];
-    if (grid_reduce<2, float>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_C], false,
-                              tot) && threadIdx.x == 0)
+    if (grid_reduce<2, float, false>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_C], false,
+                                     tot) && threadIdx.x == 0)
         st->omega = tot[1] > 0.f ? tot[0] / tot[1] : 0.f;
 }
 
@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(kBlock) k_mx_bcs_update(const SolveArgs *__res
         acc[1] = fma_t(rh[i], ri, acc[1]);
     }
     float tot[2];
-    if (grid_reduce<2, float>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_B], false,
-                              tot) && threadIdx.x == 0) {
+    if (grid_reduce<2, float, false>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_B], false,
+                                     tot) && threadIdx.x == 0) {
         const double norm = sqrtf(tot[0]);
         const int k = st->k + 1;
         st->k = k;
@@ -352,8 +352,8 @@ __global__ void __launch_bounds__(kBlock, CF_MX_MIN_BLOCKS) k_mx_mr_spmv(const S
         acc[1] = fma_t(v, v, acc[1]);
     });
     float tot[2];
-    if (grid_reduce<2, float>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_A], false,
-                              tot) && threadIdx.x == 0)
+    if (grid_reduce<2, float, false>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_A], false,
+                                     tot) && threadIdx.x == 0)
         st->omega = tot[0] / tot[1];
 }
 
@@ -394,8 +394,8 @@ __global__ void __launch_bounds__(kBlock) k_mx_mr_update(const SolveArgs *__rest
         acc[0] = fma_t(ri, ri, acc[0]);
     }
     float tot[1];
-    if (grid_reduce<1, float>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_B], false,
-                              tot) && threadIdx.x == 0)
+    if (grid_reduce<1, float, false>(acc, a->partials32, a->partial_stride, &st->counters[SLOT_B], false,
+                                     tot) && threadIdx.x == 0)
         finish_step(a, st, sqrtf(tot[0]));
 }
 

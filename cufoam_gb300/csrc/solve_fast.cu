@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kBlock, CF_SPMV_MIN_BLOCKS) k_f_cg_spmv(const 
         acc[0] = fma_t(p[row], y, acc[0]);
     });
     double tot[1];
-    if (grid_reduce<1, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_A], false, tot) &&
+    if (grid_reduce<1, double, false>(acc, a->partials, a->partial_stride, &st->counters[SLOT_A], false, tot) &&
         threadIdx.x == 0) {
         st->xi = st->rho0 / tot[0];
         st->x_pending = 0;
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kBlock, CF_CG_UPDATE_MIN_BLOCKS) k_f_cg_update
         acc[0] = fma_t(ri, ri, acc[0]);
     }
     double tot[1];
-    if (grid_reduce<1, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_B], false, tot) &&
+    if (grid_reduce<1, double, false>(acc, a->partials, a->partial_stride, &st->counters[SLOT_B], false, tot) &&
         threadIdx.x == 0) {
         st->rho1 = st->rho0;
         st->rho0 = tot[0];
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kBlock) k_f_pcg_update(const SolveArgs *__rest
     }
     double acc[2] = {(rr[0] + rr[1]) + (rr[2] + rr[3]), (rz[0] + rz[1]) + (rz[2] + rz[3])};
     double tot[2];
-    if (grid_reduce<2, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_B], false, tot) &&
+    if (grid_reduce<2, double, false>(acc, a->partials, a->partial_stride, &st->counters[SLOT_B], false, tot) &&
         threadIdx.x == 0) {
         st->rho1 = st->rho0;
         st->rho0 = tot[1];
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kBlock, CF_BICG_SPMV_MIN_BLOCKS) k_f_bicg_spmv
                        acc[0] = fma_t(ps[row], y1, acc[0]);
                    });
     double tot[1];
-    if (grid_reduce<1, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_A], false, tot) &&
+    if (grid_reduce<1, double, false>(acc, a->partials, a->partial_stride, &st->counters[SLOT_A], false, tot) &&
         threadIdx.x == 0) {
         const double xi = st->rho0 / tot[0];
         st->x_pending = 0;
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(kBlock, CF_SPMV_MIN_BLOCKS) k_f_jac_step(const
         acc[0] = fma_t(ri, ri, acc[0]);
     });
     double tot[1];
-    if (grid_reduce<1, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_A], false, tot) &&
+    if (grid_reduce<1, double, false>(acc, a->partials, a->partial_stride, &st->counters[SLOT_A], false, tot) &&
         threadIdx.x == 0)
         finish_step(a, st, sqrt(tot[0]));
 }
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kBlock, CF_SPMV_MIN_BLOCKS) k_f_rich_spmv(cons
         acc[0] = fma_t(ri, ri, acc[0]);
     });
     double tot[1];
-    if (grid_reduce<1, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_A], false, tot) &&
+    if (grid_reduce<1, double, false>(acc, a->partials, a->partial_stride, &st->counters[SLOT_A], false, tot) &&
         threadIdx.x == 0)
         finish_step(a, st, sqrt(tot[0]));
 }
@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(kBlock, CF_SPMV_MIN_BLOCKS) k_f_mr_spmv(const 
         acc[1] = fma_t(v, v, acc[1]);
     });
     double tot[2];
-    if (grid_reduce<2, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_A], false, tot) &&
+    if (grid_reduce<2, double, false>(acc, a->partials, a->partial_stride, &st->counters[SLOT_A], false, tot) &&
         threadIdx.x == 0)
         st->omega = tot[0] / tot[1];
 }
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(kBlock) k_f_bicg_update(const SolveArgs *__res
     }
     double acc[2] = {(p0[0] + p0[1]) + (p0[2] + p0[3]), (p1[0] + p1[1]) + (p1[2] + p1[3])};
     double tot[2];
-    if (grid_reduce<2, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_B], false, tot) &&
+    if (grid_reduce<2, double, false>(acc, a->partials, a->partial_stride, &st->counters[SLOT_B], false, tot) &&
         threadIdx.x == 0) {
         const double norm = sqrt(tot[0]);
         const int k = st->k + 1;
@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(kBlock) k_f_mr_update(const SolveArgs *__restr
     }
     double acc[1] = {(part[0] + part[1]) + (part[2] + part[3])};
     double tot[1];
-    if (grid_reduce<1, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_B], false, tot) &&
+    if (grid_reduce<1, double, false>(acc, a->partials, a->partial_stride, &st->counters[SLOT_B], false, tot) &&
         threadIdx.x == 0)
         finish_step(a, st, sqrt(tot[0]));
 }

@@ -22,9 +22,15 @@
 
 namespace cf {
 
+// The kernels before the iterations come in both orders (REF: the reference's),
+// since the scratch of the sequential sums, 14 KB, halves the blocks per SM of a
+// CSR pass that stages 1,024 entries a warp: 500k rows of 1 .. 9 forward links,
+// a solve of 60 steps with one kernel for both orders and with two, CG 4.01 ->
+// 3.96 ms, MRJacobi 3.82 -> 3.77.
 // ---------------------------------------------------------------------------
 // normFactor (gis/gis.cu:106-123; OpenFOAM's L1 form as an option)
 // ---------------------------------------------------------------------------
+template <bool REF>
 __global__ void __launch_bounds__(kBlock) k_nf_sum(const SolveArgs *__restrict__ a)
 {
     const int n = a->n;
@@ -32,11 +38,12 @@ __global__ void __launch_bounds__(kBlock) k_nf_sum(const SolveArgs *__restrict__
     double acc[1] = {0.0};
     CF_FOR_ELEMS(i, n) acc[0] = acc[0] + x[i]; // ReductionKernel: t += v[i]
     double tot[1];
-    if (grid_reduce<1, double>(acc, a->partials, a->partial_stride, &a->st->counters[SLOT_NF1],
-                               a->ref_order, tot) && threadIdx.x == 0)
+    if (grid_reduce<1, double, REF>(acc, a->partials, a->partial_stride, &a->st->counters[SLOT_NF1],
+                                    REF, tot) && threadIdx.x == 0)
         a->st->xbar = tot[0] / n;
 }
 
+template <bool REF>
 __global__ void __launch_bounds__(kBlock) k_nf_dist(const SolveArgs *__restrict__ a, int l1)
 {
     const int n = a->n, cap = a->stage_cap;
@@ -63,8 +70,8 @@ __global__ void __launch_bounds__(kBlock) k_nf_dist(const SolveArgs *__restrict_
         __syncwarp();
     }
     double tot[2];
-    if (grid_reduce<2, double>(acc, a->partials, a->partial_stride, &a->st->counters[SLOT_NF2],
-                               a->ref_order, tot) && threadIdx.x == 0) {
+    if (grid_reduce<2, double, REF>(acc, a->partials, a->partial_stride, &a->st->counters[SLOT_NF2],
+                                    REF, tot) && threadIdx.x == 0) {
         DevState *st = a->st;
         const double nf = l1 ? tot[0] + 1e-20 : sqrt(tot[0]) + sqrt(tot[1]) + 1e-20;
         st->nf = nf;
@@ -76,6 +83,7 @@ __global__ void __launch_bounds__(kBlock) k_nf_dist(const SolveArgs *__restrict_
 // initial residual r = b - A x (ResidualKernel), ||r||
 // mode 0: plain; 1: JMR (r = D^-1/2 (b - A x)); 2: BiCG (also r* = r)
 // ---------------------------------------------------------------------------
+template <bool REF>
 __global__ void __launch_bounds__(kBlock) k_res_init(const SolveArgs *__restrict__ a, int mode)
 {
     const int n = a->n, cap = a->stage_cap;
@@ -99,8 +107,8 @@ __global__ void __launch_bounds__(kBlock) k_res_init(const SolveArgs *__restrict
         __syncwarp();
     }
     double tot[2];
-    if (grid_reduce<2, double>(acc, a->partials, a->partial_stride, &a->st->counters[SLOT_INIT],
-                               a->ref_order, tot) && threadIdx.x == 0) {
+    if (grid_reduce<2, double, REF>(acc, a->partials, a->partial_stride, &a->st->counters[SLOT_INIT],
+                                    REF, tot) && threadIdx.x == 0) {
         finish_init(a, a->st, tot[0], mode == 2);
         if (mode == 3) a->st->rho0 = tot[1]; // PCG: (r, D^-1 r)
     }
@@ -298,6 +306,7 @@ __global__ void __launch_bounds__(kBlock) k_bicg_update(const SolveArgs *__restr
 //   x_k = x_{k-1} + omega r_{k-1}; r_k = b - A x_k  (one kernel per step:
 //   x and r are double-buffered, the new x is formed on the fly)
 // ---------------------------------------------------------------------------
+template <bool REF>
 __global__ void __launch_bounds__(kBlock) k_pow_step(const SolveArgs *__restrict__ a, int s)
 {
     const int n = a->n, cap = a->stage_cap;
@@ -320,11 +329,12 @@ __global__ void __launch_bounds__(kBlock) k_pow_step(const SolveArgs *__restrict
         __syncwarp();
     }
     double tot[1];
-    if (grid_reduce<1, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_POW],
-                               a->ref_order, tot) && threadIdx.x == 0)
+    if (grid_reduce<1, double, REF>(acc, a->partials, a->partial_stride, &st->counters[SLOT_POW],
+                                    REF, tot) && threadIdx.x == 0)
         st->pow_inv = 1 / sqrt(tot[0]);
 }
 
+template <bool REF>
 __global__ void __launch_bounds__(kBlock) k_pow_final(const SolveArgs *__restrict__ a, int steps)
 {
     const int n = a->n, cap = a->stage_cap;
@@ -343,8 +353,8 @@ __global__ void __launch_bounds__(kBlock) k_pow_final(const SolveArgs *__restric
         __syncwarp();
     }
     double tot[1];
-    if (grid_reduce<1, double>(acc, a->partials, a->partial_stride, &st->counters[SLOT_POW],
-                               a->ref_order, tot) && threadIdx.x == 0) {
+    if (grid_reduce<1, double, REF>(acc, a->partials, a->partial_stride, &st->counters[SLOT_POW],
+                                    REF, tot) && threadIdx.x == 0) {
         st->lambda_max = tot[0];
         st->omega = 2.0 / (tot[0] + st->diag_abs_min);
     }
@@ -520,6 +530,14 @@ static Kernels body_kernels(int solver, bool sell)
     return k;
 }
 
+// the kernel of this solve's order, outside a loop graph
+static void launch_in_order(Context *ctx, const void *in_ref, const void *in_fast, bool is_spmv, int cap, bool ref,
+                            void **args)
+{
+    const void *kern = ref ? in_ref : in_fast;
+    launch(ctx, ctx->stream, kern, launch_cfg(ctx, kern, is_spmv, cap, ref), args);
+}
+
 static size_t vec_bytes(int n) { return sizeof(double) * ((size_t)n + 8); }
 
 // CSR systems (rows too uneven for SELL-32) up to this many rows solve in one
@@ -568,10 +586,10 @@ double norm_factor(Matrix *m, const double *b, const double *x, int norm_type, b
     CF_CUDA(cudaMemcpyAsync(d_args, &A, sizeof(SolveArgs), cudaMemcpyHostToDevice, ctx->stream));
     CF_CUDA(cudaMemcpyAsync(A.st, &S, sizeof(DevState), cudaMemcpyHostToDevice, ctx->stream));
     void *args1[] = {&d_args};
-    launch(ctx, ctx->stream, (const void *)k_nf_sum, launch_cfg(ctx, (const void *)k_nf_sum, false, cap, ref), args1);
+    launch_in_order(ctx, (const void *)k_nf_sum<true>, (const void *)k_nf_sum<false>, false, cap, ref, args1);
     int l1 = norm_type == CF_NORM_OPENFOAM_L1 ? 1 : 0;
     void *a2[] = {&d_args, &l1};
-    launch(ctx, ctx->stream, (const void *)k_nf_dist, launch_cfg(ctx, (const void *)k_nf_dist, !sell, cap, ref), a2);
+    launch_in_order(ctx, (const void *)k_nf_dist<true>, (const void *)k_nf_dist<false>, !sell, cap, ref, a2);
     CF_CUDA(cudaMemcpyAsync(ctx->h_state, A.st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
     CF_CUDA(cudaStreamSynchronize(ctx->stream));
     return ctx->h_state->nf;
@@ -786,11 +804,9 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     CF_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
     // ---- normFactor -> tolerance * normFactor --------------------------
     {
-        launch(ctx, ctx->stream, (const void *)k_nf_sum,
-               launch_cfg(ctx, (const void *)k_nf_sum, false, cap, ref), args1);
+        launch_in_order(ctx, (const void *)k_nf_sum<true>, (const void *)k_nf_sum<false>, false, cap, ref, args1);
         void *a2[] = {&d_args, (void *)&l1};
-        launch(ctx, ctx->stream, (const void *)k_nf_dist,
-               launch_cfg(ctx, (const void *)k_nf_dist, !sell, cap, ref), a2);
+        launch_in_order(ctx, (const void *)k_nf_dist<true>, (const void *)k_nf_dist<false>, !sell, cap, ref, a2);
     }
     // ---- Richardson relaxation factor -----------------------------------
     if (solver == CF_RICHARDSON && !mixed) {
@@ -799,12 +815,12 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
             int steps = c.power_max_steps;
             for (int s = 0; s < steps; ++s) {
                 void *a2[] = {&d_args, &s};
-                launch(ctx, ctx->stream, (const void *)k_pow_step,
-                       launch_cfg(ctx, (const void *)k_pow_step, !sell, cap, ref), a2);
+                launch_in_order(ctx, (const void *)k_pow_step<true>, (const void *)k_pow_step<false>, !sell, cap, ref,
+                                a2);
             }
             void *a3[] = {&d_args, &steps};
-            launch(ctx, ctx->stream, (const void *)k_pow_final,
-                   launch_cfg(ctx, (const void *)k_pow_final, !sell, cap, ref), a3);
+            launch_in_order(ctx, (const void *)k_pow_final<true>, (const void *)k_pow_final<false>, !sell, cap, ref,
+                            a3);
         }
     }
     // ---- initial residual ----------------------------------------------
@@ -813,8 +829,7 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
         int mode = solver == CF_JMR ? 1 : mixed ? 0 : (solver == CF_BICG ? 2 : (solver == CF_PCG ? 3 : 0));
         if (!ref && !mixed && (solver == CF_MRJACOBI || solver == CF_MRS)) mode = 4;
         void *a2[] = {&d_args, &mode};
-        launch(ctx, ctx->stream, (const void *)k_res_init,
-               launch_cfg(ctx, (const void *)k_res_init, !sell, cap, ref), a2);
+        launch_in_order(ctx, (const void *)k_res_init<true>, (const void *)k_res_init<false>, !sell, cap, ref, a2);
     }
     // ---- iterations: device-driven while loop, or host-driven chunks ----
     CF_CUDA(cudaEventRecord(ctx->ev_mid, ctx->stream));

@@ -52,3 +52,11 @@ def test_cluster_scope_waits_for_its_blocks_before_the_first_remote_store():
     assert last == "barrier();", last
     barrier = _body(scope, scope.index("bool barrier()"))
     assert barrier.index("barrier.cluster.arrive.release") < barrier.index("barrier.cluster.wait.acquire")
+
+
+def test_fast_order_reductions_carry_no_scratch_of_the_reference_order():
+    """Static shared memory of the CSR passes comes out of their L1: callers
+    that never sum in the reference order say so at compile time."""
+    calls = [c for name in ("solve_fast.cu", "mixed.cu", "distributed.cu")
+             for c in re.findall(r"grid_reduce<([^>]*)>\(([^;{]*?)\) &&", _code(name))]
+    assert calls and all(args.split(",")[-1].strip() == "false" for args, _ in calls)
