@@ -95,7 +95,8 @@ __device__ __forceinline__ int block_inclusive_scan(int v, int *sm)
     return v;
 }
 
-__global__ void k_scan_blocks(int m, const int32_t *__restrict__ in, int32_t *out, int32_t *sums)
+// (in may be out: a thread writes the element it read)
+__global__ void k_scan_blocks(int m, const int32_t *in, int32_t *out, int32_t *sums)
 {
     __shared__ int sm[32];
     const int i = blockIdx.x * kScanBlock + threadIdx.x;

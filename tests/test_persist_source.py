@@ -60,3 +60,13 @@ def test_fast_order_reductions_carry_no_scratch_of_the_reference_order():
     calls = [c for name in ("solve_fast.cu", "mixed.cu", "distributed.cu")
              for c in re.findall(r"grid_reduce<([^>]*)>\(([^;{]*?)\) &&", _code(name))]
     assert calls and all(args.split(",")[-1].strip() == "false" for args, _ in calls)
+
+
+def test_the_in_place_scan_may_alias():
+    """The slice lengths are turned into offsets in place: the kernel that
+    reads and writes them must not promise the compiler distinct arrays (such
+    loads may go through the read-only cache)."""
+    text = _code("matrix.cu")
+    in_place = re.search(r"exclusive_scan\(ctx, [^,]*, (\w+->s_off\.as<int32_t>\(\)), \1,", text)
+    scan = re.search(r"void k_scan_blocks\(([^)]*)\)", text).group(1)
+    assert in_place and "__restrict__" not in scan
