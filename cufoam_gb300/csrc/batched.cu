@@ -1820,7 +1820,7 @@ SmallSolveResult solve_small_single_cluster(Matrix *m, int solver, const cf_cont
     a.max_iter = c.max_iter <= 0 ? INT_MAX : c.max_iter;
     a.tolerance = c.tolerance;
     a.omega = c.richardson_omega;
-    a.power_steps = c.power_max_steps > 0 ? c.power_max_steps : 30;
+    a.power_steps = c.power_max_steps > 0 ? c.power_max_steps : kPowerSteps;
     a.b = b;
     a.x = x;
     a.r = r;

@@ -332,7 +332,7 @@ void cf_controls_init(cf_controls *c)
     c->norm_type = CF_NORM_REFERENCE_L2;
     c->bicg_int_bound = 1e-10;   // cuFoamBiCG/cuFoamBiCG.C:68
     c->richardson_omega = 0.0;   // cuFoamRichardson/cuFoamRichardson.C:66
-    c->power_max_steps = 30;
+    c->power_max_steps = cf::kPowerSteps;
     c->mixed_max_outer = 50;
     c->mixed_inner_rtol = 0.0; // the solver's default
     c->history = nullptr;

@@ -488,7 +488,7 @@ void solve_distributed(Matrix *m, int solver, const cf_controls &c, const cf_int
             double *x1 = p, *x2 = q;
             k_dd_fill<<<eg, kBlock, 0, st>>>(n, 1.0 / n_global, x2);
             CF_CHECK_LAUNCH();
-            const int steps = c.power_max_steps > 0 ? c.power_max_steps : 30;
+            const int steps = c.power_max_steps > 0 ? c.power_max_steps : kPowerSteps;
             for (int s = 0; s < steps; ++s) {
                 std::swap(x1, x2);
                 D.apply(x1, x2);

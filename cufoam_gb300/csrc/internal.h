@@ -171,6 +171,8 @@ struct GraphEntry {
 // a microsecond each: 17 s); the solve then ends with CF_TIMEOUT
 constexpr int32_t kPollLimit = 1 << 25;
 
+constexpr int32_t kPowerSteps = 30;   // power-method steps by default
+
 struct Context {
     int device = 0;
     cudaStream_t stream = nullptr;

@@ -660,9 +660,10 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     // k_small_solve, the whole solve behind hardware cluster barriers)
     const bool small_kind = solver == CF_CG || solver == CF_JACOBI || solver == CF_RICHARDSON ||
                             solver == CF_MR || solver == CF_MRJACOBI || solver == CF_MRS || solver == CF_JMR;
-    if (!sell && small_kind && !ref && !mixed && !tr && n <= kSmallCgRows && !want_hist &&
-        c.time_limit_s <= 0 && c.profile_kernels == 0 && c.rel_tol == 0 && c.min_iter <= 0 &&
-        c.norm_type == CF_NORM_REFERENCE_L2 && !c.absolute_tolerance && c.use_graph != 0 && small_cg_ok(ctx)) {
+    const bool is_small = small_kind && !ref && !mixed && !tr && n <= kSmallCgRows && !want_hist &&
+                       c.time_limit_s <= 0 && c.profile_kernels == 0 && c.rel_tol == 0 && c.min_iter <= 0 &&
+                       c.norm_type == CF_NORM_REFERENCE_L2 && !c.absolute_tolerance && c.use_graph != 0;
+    if (is_small && !sell && small_cg_ok(ctx)) {
         const SmallSolveResult R =
             solver == CF_CG
                 ? solve_cg_single_cluster(m, c, b, x, ctx->vec[2].as<double>(), ctx->vec[4].as<double>(),
@@ -741,7 +742,8 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     A.st = ctx->state.as<DevState>();
     A.hist = want_hist ? ctx->hist.as<double>() : nullptr;
     A.hist_t = hist_time ? ctx->hist_t.as<unsigned long long>() : nullptr;
-    A.power_steps = c.power_max_steps;
+    // (no number of steps: the default on small systems, in either format)
+    A.power_steps = is_small && c.power_max_steps <= 0 ? kPowerSteps : std::max(c.power_max_steps, 0);
     A.abort_flag = (c.time_limit_s > 0) ? ctx->d_abort : nullptr;
 
     if (mixed) mixed_prepare(ctx, m, solver, A);
@@ -812,7 +814,7 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     if (solver == CF_RICHARDSON && !mixed) {
         const double om = c.richardson_omega;
         if (-1e-15 < om && om < 1e-15) {
-            int steps = c.power_max_steps;
+            int steps = A.power_steps;
             for (int s = 0; s < steps; ++s) {
                 void *a2[] = {&d_args, &s};
                 launch_in_order(ctx, (const void *)k_pow_step<true>, (const void *)k_pow_step<false>, !sell, cap, ref,
