@@ -483,7 +483,8 @@ __device__ __forceinline__ void report_fail(int32_t fail, DevState *out)
 __device__ __forceinline__ double div_by_reciprocal(double a, double b, double rb)
 {
     const uint32_t ea = ((uint32_t)__double2hiint(a) >> 20) & 0x7ffu, eb = ((uint32_t)__double2hiint(b) >> 20) & 0x7ffu;
-    if (ea - 200u > 1600u || eb - 200u > 1600u) return a / b;   // zero, near the range's ends, or not finite
+    // zero, not finite, or beyond 2^+-400, where the quotient may leave the normal range
+    if (ea - 623u > 800u || eb - 623u > 800u) return a / b;
     const double q = __dmul_rn(a, rb);
     return __fma_rn(__fma_rn(-q, b, a), rb, q);
 }
