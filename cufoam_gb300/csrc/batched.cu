@@ -208,7 +208,6 @@ struct ClusterScope {
         return pos < a.n_systems ? a.order[pos] : -1;
     }
     __device__ __forceinline__ void leave() { cl.sync(); }
-    __device__ __forceinline__ bool failed() const { return false; }
 };
 
 // A group of co-resident blocks (a cooperative launch) with a counter in
@@ -392,6 +391,22 @@ __device__ __forceinline__ void st_row(float *p, int64_t c, const float (&v)[R])
     }
 }
 
+// A CSR row's entries added to the products y and the sum ys of its values.
+template <int R, class V, class T, class G>
+__device__ __forceinline__ void csr_row_product(const BatchSystem &S, const V *__restrict__ cval, int row,
+                                                const bool (&on)[R], G g, T (&y)[R], T &ys)
+{
+    const int e1 = __ldg(S.ro + row + 1);
+    for (int e = __ldg(S.ro + row); e < e1; ++e) {
+        const T v = (T)__ldg(cval + e);
+        T xv[R];
+        g(__ldg(S.col + e), xv);
+#pragma unroll
+        for (int j = 0; j < R; ++j) y[j] = fma_t(v, on[j] ? xv[j] : T(0), y[j]);
+        ys += v;
+    }
+}
+
 // The R-wide product of row `row` (this lane's row of 32-row slice s):
 // y[j] = sum_e a_e g(col_e)[j] over the components j with on[j], where
 // g(c, out) gathers the R components of row c; ys = sum_e a_e.
@@ -441,15 +456,7 @@ __device__ __forceinline__ void row_product(const BatchSystem &S, const V *__res
         }
 #undef CF_BATCH_LD
     } else if (row < S.n) {
-        const int e1 = __ldg(S.ro + row + 1);
-        for (int e = __ldg(S.ro + row); e < e1; ++e) {
-            const T v = (T)__ldg(cval + e);
-            T xv[R];
-            g(__ldg(S.col + e), xv);
-#pragma unroll
-            for (int j = 0; j < R; ++j) y[j] = fma_t(v, on[j] ? xv[j] : T(0), y[j]);
-            ys += v;
-        }
+        csr_row_product<R, V, T>(S, cval, row, on, g, y, ys);
     }
 }
 
@@ -1439,7 +1446,7 @@ void batch_solve(Batch *B, const cf_controls &c, int nrhs, const double *b_in, d
 }
 
 // ---------------------------------------------------------------------------
-// One small system: the whole CG solve in one cluster-persistent launch
+// One small CSR system: the whole CG solve in one cluster-persistent launch
 // ---------------------------------------------------------------------------
 // Rows per CTA the single-system path aims for when it sizes its cluster
 // (one row per thread: its passes are latency chains, so the most threads
@@ -1484,7 +1491,6 @@ SmallSolveResult solve_cg_single_cluster(Matrix *m, const cf_controls &c, const 
 {
     Context *ctx = m->ctx;
     const int n = m->n;
-    const bool sell = matrix_ensure_sell(m, false, false);
     struct Block {
         BatchSystem sys;
         int32_t order[4];
@@ -1495,16 +1501,11 @@ SmallSolveResult solve_cg_single_cluster(Matrix *m, const cf_controls &c, const 
     blk.ensure(sizeof(Block));
     Block h{};
     h.sys.n = n;
-    h.sys.sell = sell ? 1 : 0;
+    h.sys.sell = 0;
     h.sys.vec_offset = 0;
     h.sys.ro = m->ro.as<int32_t>();
     h.sys.col = m->col.as<int32_t>();
     h.sys.val = m->val.as<double>();
-    h.sys.val32 = nullptr;
-    h.sys.s_off = sell ? m->s_off.as<int32_t>() : nullptr;
-    h.sys.s_col = sell ? m->s_col.as<int32_t>() : nullptr;
-    h.sys.s_val = sell ? m->s_val.as<double>() : nullptr;
-    h.sys.s_val32 = nullptr;
     Block *d = blk.as<Block>();
     CF_CUDA(cudaMemcpyAsync(d, &h, sizeof(Block), cudaMemcpyHostToDevice, ctx->stream));
     BatchArgs a{};
@@ -1549,7 +1550,7 @@ int64_t batch_offset(const Batch *B, int s) { return B->offsets[s]; }
 namespace cf {
 
 // ---------------------------------------------------------------------------
-// Jacobi, Richardson and the MR family on one small system in one
+// Jacobi, Richardson and the MR family on one small CSR system in one
 // cluster-persistent launch (the CG kernel's schedule: one cluster of up to
 // 16 CTAs, rows split by 32-row slices, hardware cluster barriers where the
 // multi-kernel loop has kernel boundaries), fast summation order.  The
@@ -1603,8 +1604,11 @@ __global__ void __launch_bounds__(256, 1) k_small_solve(const SmallArgs a)
     const bool on[1] = {true};
     double *x = a.x, *r = a.r, *d = a.d, *y = a.y;
     const double *b = a.b;
-    auto gather = [](const double *v) {
-        return [v](int c, double(&o)[1]) { o[0] = __ldcg(v + c); };
+    auto product = [&](const double *v, int row, double(&yv)[1], double &ys) {
+        yv[0] = ys = 0.0;
+        if (row < n)
+            csr_row_product<1, double, double>(S, S.val, row, on, [v](int c, double(&o)[1]) { o[0] = __ldcg(v + c); },
+                                               yv, ys);
     };
     auto reduce = [&](double (&acc)[1]) {
         cluster_sum<1, 256>(cl, acc, wsm, slot[parity], tot);
@@ -1620,9 +1624,9 @@ __global__ void __launch_bounds__(256, 1) k_small_solve(const SmallArgs a)
     const double xbar = reduce(acc1) / n;
     {
         double acc3[3] = {0.0, 0.0, 0.0};
-        small_rows(n, s_lo, s_hi, [&](int s, int row, bool ok) {
+        small_rows(n, s_lo, s_hi, [&](int, int row, bool ok) {
             double yv[1], ys;
-            row_product<1, double, double>(S, S.s_val, S.val, s, row, on, gather(x), yv, ys);
+            product(x, row, yv, ys);
             if (ok) {
                 const double yb = ys * xbar, bi = b[row];
                 const double d1 = yv[0] - yb, d2 = bi - yb;
@@ -1661,9 +1665,9 @@ __global__ void __launch_bounds__(256, 1) k_small_solve(const SmallArgs a)
             });
             cl.sync(); // every CTA's x1 rows are written before anyone gathers them
             double acc[1] = {0.0};
-            small_rows(n, s_lo, s_hi, [&](int s, int row, bool ok) {
+            small_rows(n, s_lo, s_hi, [&](int, int row, bool ok) {
                 double yv[1], ys;
-                row_product<1, double, double>(S, S.s_val, S.val, s, row, on, gather(d), yv, ys);
+                product(d, row, yv, ys);
                 if (ok) {
                     y[row] = yv[0];
                     acc[0] = fma_t(yv[0], yv[0], acc[0]);
@@ -1676,9 +1680,9 @@ __global__ void __launch_bounds__(256, 1) k_small_solve(const SmallArgs a)
         }
         cl.sync(); // x2 complete before anyone gathers it
         double acc[1] = {0.0}, amin = HUGE_VAL;
-        small_rows(n, s_lo, s_hi, [&](int s, int row, bool ok) {
+        small_rows(n, s_lo, s_hi, [&](int, int row, bool ok) {
             double yv[1], ys;
-            row_product<1, double, double>(S, S.s_val, S.val, s, row, on, gather(y), yv, ys);
+            product(y, row, yv, ys);
             if (ok) {
                 acc[0] = fma_t(y[row], yv[0], acc[0]);
                 amin = fmin(amin, fabs(a.diag[row]));
@@ -1723,9 +1727,9 @@ __global__ void __launch_bounds__(256, 1) k_small_solve(const SmallArgs a)
                 if (ok) x[row] = fma_t(om, r[row], x[row]);
             });
             cl.sync(); // x complete before anyone gathers it
-            small_rows(n, s_lo, s_hi, [&](int s, int row, bool ok) {
+            small_rows(n, s_lo, s_hi, [&](int, int row, bool ok) {
                 double yv[1], ys;
-                row_product<1, double, double>(S, S.s_val, S.val, s, row, on, gather(x), yv, ys);
+                product(x, row, yv, ys);
                 if (ok) {
                     const double ri = b[row] - yv[0];
                     r[row] = ri;
@@ -1743,9 +1747,9 @@ __global__ void __launch_bounds__(256, 1) k_small_solve(const SmallArgs a)
                 dv = d;
             }
             double t2[2] = {0.0, 0.0};
-            small_rows(n, s_lo, s_hi, [&](int s, int row, bool ok) {
+            small_rows(n, s_lo, s_hi, [&](int, int row, bool ok) {
                 double yv[1], ys;
-                row_product<1, double, double>(S, S.s_val, S.val, s, row, on, gather(dv), yv, ys);
+                product(dv, row, yv, ys);
                 if (ok) {
                     double yi = yv[0];
                     if (solver == CF_JMR) yi = __dmul_rn(a.dsq[row], yi);
@@ -1796,7 +1800,6 @@ SmallSolveResult solve_small_single_cluster(Matrix *m, int solver, const cf_cont
 {
     Context *ctx = m->ctx;
     const int n = m->n;
-    const bool sell = matrix_ensure_sell(m, false, false);
     struct Block {
         BatchSystem sys;
         SmallSolveOut out;
@@ -1805,13 +1808,10 @@ SmallSolveResult solve_small_single_cluster(Matrix *m, int solver, const cf_cont
     blk.ensure(sizeof(Block));
     Block h{};
     h.sys.n = n;
-    h.sys.sell = sell ? 1 : 0;
+    h.sys.sell = 0;
     h.sys.ro = m->ro.as<int32_t>();
     h.sys.col = m->col.as<int32_t>();
     h.sys.val = m->val.as<double>();
-    h.sys.s_off = sell ? m->s_off.as<int32_t>() : nullptr;
-    h.sys.s_col = sell ? m->s_col.as<int32_t>() : nullptr;
-    h.sys.s_val = sell ? m->s_val.as<double>() : nullptr;
     Block *dblk = blk.as<Block>();
     CF_CUDA(cudaMemcpyAsync(dblk, &h, sizeof(Block), cudaMemcpyHostToDevice, ctx->stream));
     SmallArgs a{};

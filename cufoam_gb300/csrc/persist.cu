@@ -62,7 +62,7 @@ struct PersistArgs {
 // Per-block step state, the same bits in every block (thread 0 writes it
 // between barriers).
 struct PersistState {
-    double rho0, rrho, xi, beta, omega, tol, tol_lo, tol_hi, nf, norm, norm0, xbar, pow_inv, lambda;
+    double rho0, rrho, xi, beta, omega, tol, tol_hi, nf, norm, norm0, xbar, pow_inv, lambda;
     int32_t k, done, status;
 };
 
@@ -103,7 +103,6 @@ __device__ __forceinline__ void persist_begin(const SolveArgs &A, const PersistA
     // within rounding of tol^2
     const double t2 = st.tol * st.tol;
     const bool usable = t2 > 1e-280 && t2 < 1e280;
-    st.tol_lo = usable ? t2 * (1.0 - 1e-14) : -1.0;
     st.tol_hi = usable ? t2 * (1.0 + 1e-14) : HUGE_VAL;
     st.k = 0;
     const bool finite = isfinite(norm0);
@@ -616,6 +615,28 @@ static const void *persist_pick(int scope, int format)
                               : (const void *)k_persist<SOLVER, kSell, false, GridSync>;
 }
 
+// the vectors a solver keeps per block
+struct PersistNeeds {
+    bool q, gather_r, own, local_x, scale;
+};
+template <int SOLVER> static PersistNeeds needs_of()
+{
+    using Tr = PersistTraits<SOLVER>;
+    return {Tr::kQ, Tr::kGatherR, Tr::kOwnG, Tr::kLocalX, Tr::kScale};
+}
+static PersistNeeds persist_needs(int solver)
+{
+    switch (solver) {
+    case CF_CG: return needs_of<CF_CG>();
+    case CF_PCG: return needs_of<CF_PCG>();
+    case CF_JACOBI: return needs_of<CF_JACOBI>();
+    case CF_RICHARDSON: return needs_of<CF_RICHARDSON>();
+    case CF_MR: return needs_of<CF_MR>();
+    case CF_JMR: return needs_of<CF_JMR>();
+    default: return needs_of<CF_MRJACOBI>();   // (MRS too)
+    }
+}
+
 static const void *persist_kernel(int solver, int scope, int format)
 {
     switch (solver) {
@@ -789,12 +810,7 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
     P.l1 = l1;
     P.power_steps = A.power_steps;
 
-    const bool q = solver != CF_JACOBI && solver != CF_RICHARDSON;
-    const bool gather_r = solver == CF_MR || solver == CF_JMR || solver == CF_JACOBI;
-    const bool local_x = solver != CF_RICHARDSON;
-    const bool scale = solver == CF_PCG || solver == CF_JACOBI || solver == CF_MRJACOBI || solver == CF_MRS ||
-                       solver == CF_JMR;
-    const bool own = solver == CF_CG || solver == CF_PCG || solver == CF_MRJACOBI || solver == CF_MRS;
+    const PersistNeeds need = persist_needs(solver);
     const int ns = A.n_slices;
     // everything a block of `slices` slices keeps in shared memory, in doubles
     auto plan_all = [&](int slices, bool cluster) {
@@ -806,12 +822,12 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
             return o;
         };
         p.off = take(slices / 2 + 2);
-        p.q = q ? take(32 * slices) : -1;
+        p.q = need.q ? take(32 * slices) : -1;
         p.r = take(32 * slices);
-        p.x = local_x || cluster ? take(32 * slices) : -1;
-        p.scale = scale ? take(32 * slices) : -1;
+        p.x = need.local_x || cluster ? take(32 * slices) : -1;
+        p.scale = need.scale ? take(32 * slices) : -1;
         const bool power = cluster && solver == CF_RICHARDSON;
-        p.g = own || power ? take(32 * slices) : -1;
+        p.g = need.own || power ? take(32 * slices) : -1;
         p.g2 = power || (cluster && solver == CF_JACOBI) ? take(32 * slices) : -1;
         p.val = take(32 * slices * max_len);
         p.col = take(16 * slices * max_len);
@@ -853,9 +869,9 @@ void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, co
             };
             P.plan.val = P.plan.col = P.plan.scale = P.plan.g = P.plan.g2 = -1;
             P.plan.off = take(most <= 4096, most / 2 + 2);
-            P.plan.q = take(most <= 4096 && q, 32 * most);
-            P.plan.r = take(most <= 4096 && !gather_r, 32 * most);
-            P.plan.x = take(most <= 4096 && local_x, 32 * most);
+            P.plan.q = take(most <= 4096 && need.q, 32 * most);
+            P.plan.r = take(most <= 4096 && !need.gather_r, 32 * most);
+            P.plan.x = take(most <= 4096 && need.local_x, 32 * most);
             smem = sizeof(double) * (size_t)at;
         }
     }
