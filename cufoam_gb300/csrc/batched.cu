@@ -1223,7 +1223,7 @@ static bool solve_groups(Context *ctx, Batch *B, BatchArgs &a, int nrhs, bool mi
     const int S = (int)B->mats.size();
     const void *kernel = group_kernel_for(nrhs, mixed, false), *resumed = group_kernel_for(nrhs, mixed, true);
     int per_sm = 0;
-    if (!persist_usable(ctx, CF_CG, kSell, false)) return false;
+    if (!persist_possible(ctx)) return false;
     for (const void *k : {kernel, resumed}) {
         int n = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kGroupThreads, 0) != cudaSuccess || n < 1) {

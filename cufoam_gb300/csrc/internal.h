@@ -349,7 +349,8 @@ SmallSolveResult solve_small_single_cluster(Matrix *m, int solver, const cf_cont
 bool small_cg_ok(Context *ctx);
 
 // a whole FP64 solve in the fast order as one launch (persist.cu)
-bool persist_usable(Context *ctx, int solver, int format, bool mixed);
+bool persist_possible(Context *ctx);
+bool persist_usable(Context *ctx, int solver, int format, bool mixed, const Matrix *m);
 void launch_persist(Context *ctx, int solver, int format, const SolveArgs &A, const DevState &S, int l1, Matrix *m,
                     DevState *out);
 // ... and a whole mixed-precision solve (persist_mixed.cu); the total of FP32

@@ -15,6 +15,8 @@
 //     for the whole solve while they fit (about 250k rows of a 7-point
 //     system): only the gathered vector is exchanged, through L2;
 //   * the grid with the matrix streamed from L2 or HBM.
+// Large systems, whose vectors outgrow L2, stay with the multi-kernel loop
+// (persist_usable).
 // Measured on GB300, us per step and for normFactor + residual + first step
 // (7-point systems; multi-kernel loop, or the single-cluster kernels at 4k
 // rows -> here):
@@ -652,14 +654,10 @@ static const void *persist_kernel(int solver, int scope, int format)
     }
 }
 
-// Whether a solve over the SELL-32 copy runs here (faster than the
-// multi-kernel loop at every size, see the top of the file); CSR matrices
-// (their staging buffers), BiCG's fast order and devices without cooperative
-// launches or with more SMs than the partial sums are sized for run the loop.
-bool persist_usable(Context *ctx, int solver, int format, bool mixed)
+// Cooperative launches, and no more SMs than the partial sums are sized for.
+bool persist_possible(Context *ctx)
 {
-    if (format == kCsr || ctx->sm_count > kPMaxGrid) return false;
-    if (!mixed && !persist_kernel(solver, kScopeGrid, format)) return false;
+    if (ctx->sm_count > kPMaxGrid) return false;
     if (ctx->coop_ok < 0) {
         int coop = 0;
         if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) != cudaSuccess) {
@@ -669,6 +667,42 @@ bool persist_usable(Context *ctx, int solver, int format, bool mixed)
         ctx->coop_ok = coop;
     }
     return ctx->coop_ok == 1;
+}
+
+// Whether a solve over the SELL-32 copy runs here.  CSR matrices (their staging
+// buffers), BiCG's fast order and devices where it is not possible run the
+// multi-kernel loop, and so do large systems:
+//
+// * FP64.  A block's rows are contiguous, so at any time 152 windows of the
+//   gathered vector are in use, each twice the largest column offset; the loop
+//   deals slices round robin and has one.  Once the windows (at most the whole
+//   vector) outgrow their part of L2 the loop is faster.  us per step, here /
+//   loop: CG 176^3 153 / 159, 208^3 254 / 254, 224^3 323 / 311, 256^3 473 / 450;
+//   MR 208^3 212 / 213, 256^3 400 / 379; PCG 208^3 293 / 293, 256^3 540 / 524;
+//   Jacobi 192^3 151 / 155, 208^3 200 / 195; MRJacobi, which gathers z beside r,
+//   176^3 169 / 170, 192^3 218 / 214, 256^3 515 / 479.  Narrow windows stay here:
+//   4096^2 CG 397 / 419, MRJacobi 436 / 449; 64 x 64 x 4096 CG 436 / 450.
+// * Richardson, one product per step: 176^3 128 / 129, 192^3 168 / 164, 256^3 411
+//   / 369; 4096^2 351 / 340.
+// * FP32 sweeps: past L2 their products are bound by loads in flight, 32 warps
+//   per SM here and 48 in the loop.  MR 160^3 46 / 49, 176^3 61 / 61, 256^3 225 /
+//   199; MRJacobi, JMR 176^3 71 / 75, 192^3 99 / 97, 256^3 254 / 231; BiCGStab 208^3
+//   312 / 317, 224^3 388 / 387, 256^3 598 / 558; CG is faster here at every size
+//   (288^3 399 / 445).
+//
+// The limits are shares of L2 (135.5 MB) that 8 bytes per row, or the windows,
+// take: 0.53 is 9M rows.
+bool persist_usable(Context *ctx, int solver, int format, bool mixed, const Matrix *m)
+{
+    if (format == kCsr || !persist_possible(ctx)) return false;
+    if (!mixed && !persist_kernel(solver, kScopeGrid, format)) return false;
+    const double l2 = (double)ctx->l2_bytes;
+    const double vector = 8.0 * m->n, windows = std::min(vector, 16.0 * m->max_offset * ctx->sm_count);
+    const bool diag = solver == CF_MRJACOBI || solver == CF_MRS;
+    if (mixed)
+        return solver == CF_CG || vector <= (solver == CF_BICG ? 0.65 : diag || solver == CF_JMR ? 0.385 : 0.32) * l2;
+    if (solver == CF_RICHARDSON) return vector <= 0.355 * l2;
+    return windows <= (diag ? 0.325 : solver == CF_JACOBI ? 0.47 : 0.53) * l2;
 }
 
 // Asked for the kernel to be launched, with its own registers and the most

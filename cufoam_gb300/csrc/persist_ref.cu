@@ -377,7 +377,7 @@ out:
 // the reference's grid within what the sequential sums take.
 bool persist_ref_usable(Context *ctx, int solver, bool sell)
 {
-    return solver == CF_BICG && sell && ctx->ref_grid <= kSeqMax && persist_usable(ctx, CF_CG, kSell, false);
+    return solver == CF_BICG && sell && ctx->ref_grid <= kSeqMax && persist_possible(ctx);
 }
 
 void launch_persist_ref(Context *ctx, const SolveArgs &A, const DevState &S, int l1, DevState *out)

@@ -772,7 +772,7 @@ void solve(Matrix *m, int solver, const cf_controls &c, const double *b_in, doub
     SolveArgs *d_args = ctx->args.as<SolveArgs>();
     // the fast order over the SELL-32 copy: one launch
     const bool persist =
-        use_graph && (ref ? persist_ref_usable(ctx, solver, sell) : persist_usable(ctx, solver, fmt, mixed));
+        use_graph && (ref ? persist_ref_usable(ctx, solver, sell) : persist_usable(ctx, solver, fmt, mixed, m));
     if (use_graph && !mixed && !persist) {
         try {
             ge = loop_graph(ctx, kk, solver, CF_PREC_FP64, cap, ref, d_args, fmt);
