@@ -21,10 +21,10 @@
 // (7-point systems; multi-kernel loop, or the single-cluster kernels at 4k
 // rows -> here):
 //                4k          22k         219k        893k        2.1M rows
-//   CG step      7.0->5.4   16.6->7.9   28.8->12.8  43.9->27.0  72.1->55.7
-//   Jacobi step  4.7->2.3    8.3->3.4   15.3->7.4   28.8->20.6  53.5->43.9
+//   CG step      7.0->5.0   16.6->7.9   28.8->12.8  43.9->27.0  72.1->55.7
+//   Jacobi step  4.7->2.2    8.3->3.4   15.3->7.4   28.8->20.6  53.5->43.9
 //   MRJacobi     8.2->5.1   16.0->7.2   24.0->12.3  38.8->25.8  70.4->53.9
-//   CG set-up     27->28     102->30     160->48     267->94     422->170
+//   CG set-up     27->24     102->30     160->48     267->94     422->170
 // At 2.1M rows the FP64 unit bounds a CG step: 12 operations per row, 64
 // cycles per warp and sub-partition each, are 83,000 of its 115,000 cycles.
 // The arithmetic of a row and of an element
