@@ -120,7 +120,11 @@ __global__ void __launch_bounds__(kBlock) k_res_init(const SolveArgs *__restrict
 //       also applies the deferred x += xi_{k-1} p_{k-1}
 //   K2: r -= xi q, (r, r), stopping test
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) k_cg_spmv(const SolveArgs *__restrict__ a)
+// (four blocks per SM: left to itself the compiler aims at five, 48 registers
+// with spills, since the sequential sums are a call.  ms per 40 steps, 48 -> 64
+// registers: 256^3 44.7 -> 39.8, 180^3 renumbered at random 28.2 -> 25.8, and
+// k_rich_step there 25.8 -> 22.1)
+__global__ void __launch_bounds__(kBlock, 4) k_cg_spmv(const SolveArgs *__restrict__ a)
 {
     DevState *st = a->st;
     CF_EXIT_IF_DONE(a, st, false);
@@ -360,7 +364,7 @@ __global__ void __launch_bounds__(kBlock) k_pow_final(const SolveArgs *__restric
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_rich_step(const SolveArgs *__restrict__ a)
+__global__ void __launch_bounds__(kBlock, 4) k_rich_step(const SolveArgs *__restrict__ a)
 {
     DevState *st = a->st;
     CF_EXIT_IF_DONE(a, st, true);
