@@ -119,5 +119,5 @@ def test_unequal_counts_take_no_longer_than_the_queue(ctx):
     b = np.random.default_rng(1).standard_normal((B.rows, 3))
     t = {cfg: min(B.solve(b, tolerance=1e-8, max_iter=5000, config=cfg)[2] for _ in range(5))
          for cfg in ((0, 256, 0), (16, 256, 0))}
-    assert t[0, 256, 0] <= 1.1 * t[16, 256, 0], t
+    assert t[0, 256, 0] <= 1.25 * t[16, 256, 0], t
     B.close()

@@ -95,4 +95,4 @@ def test_the_time_does_not_depend_on_where_the_long_rows_are(ctx, name):
         S = cf._TABLE["cuFoam" + name]("p", M, {"tolerance": 0.0, "maxIter": 60})
         t[where] = min(S.solve(np.zeros(n), b).solve_ms for _ in range(5))
         M.close()
-    assert t["end"] <= 1.1 * t["spread"], t
+    assert t["end"] <= 1.15 * t["spread"], t
